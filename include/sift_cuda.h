@@ -92,8 +92,9 @@ typedef enum {
 typedef struct {
     int32_t device;          /* CUDA device ordinal */
     int32_t storage;         /* SiftCudaStorage (default SIFT_CUDA_STORAGE_U8) */
-    int32_t level_tile_rows; /* rows of the fused level kernel's tiles: 0 (default: 64), 64 or 32;
-                                the output is the same (the batched form always uses 64) */
+    int32_t level_tile_rows; /* rows of the fused level kernel's tiles: 0 (default) or 64: 64-row tiles on planes
+                                that fill the device with them and 32-row tiles on smaller ones; 32: 32-row
+                                tiles on every plane; the output is the same (the batched form uses 64) */
     uint32_t reserved[5];
 } SiftCudaOptions;
 

@@ -34,8 +34,8 @@ size_t batch_lz_bytes();
 void batch_lz_fill(void* out, int vtab, int vw, int htab, int hw, const LanczosUniform& uni);
 int launch_blur_level_flat(const BatchPyr& bp, uint8_t* tmp, int o, int s, int r, int n_img,
                            const uint32_t* fused_pref, uint32_t n_fused, const uint32_t* rows_pref, uint32_t n_rows,
-                           int max_w, const uint32_t* cols_pref, uint32_t n_cols, const float* wts,
-                           const float* lut255, cudaStream_t st, int* launches, int fused_max_radius);
+                           int max_w, const uint32_t* cols_pref, uint32_t n_cols, const float* wts, const TcBlur& b,
+                           const void* frags, const float* lut255, cudaStream_t st, int* launches);
 int launch_lanczos_flat(const BatchPyr& bp, int o, int n_img, const uint32_t* pref, uint32_t n_tiles,
                         const void* lz, const int* itab, const float* ftab, cudaStream_t st);
 
@@ -212,12 +212,11 @@ struct BatchEngine {
         BlurPlan bp = blur_plan(p);
         std::vector<float> wts;
         auto add_blur = [&](float sigma) {
-            LevelBlur b{sigma, 0, wts.size()};
+            LevelBlur b{sigma, 0, wts.size(), {}, 0};
             if (sigma > 0.0f) {
                 auto k = gaussian_kernel(sigma);
                 b.radius = (int)(k.size() / 2);
-                wts.insert(wts.end(), k.begin(), k.end());
-                while (wts.size() % 4) wts.push_back(0.0f);
+                append_taps(k, &b, &wts);
             }
             return b;
         };
@@ -410,8 +409,8 @@ struct BatchEngine {
                 return 0;
             }
             return bump(launch_blur_level_flat(bp, tmp, o, s, b.radius, N, pref(pf.fused), pf.n_fused, pref(pf.rows),
-                                               pf.n_rows, max_w, pref(pf.cols), pf.n_cols, wts + b.woff, lut, q,
-                                               &nl, 8),
+                                               pf.n_rows, max_w, pref(pf.cols), pf.n_cols, wts + b.woff, b.tc, wts + b.foff,
+                                               lut, q, &nl),
                         "batch blur");
         };
         // pyramid

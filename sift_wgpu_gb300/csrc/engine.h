@@ -40,8 +40,9 @@ namespace sift {
 // launchers (pyramid.cu, detect.cu, describe.cu)
 template <typename TG>
 int launch_blur_level(const uint8_t* in, int in_pitch, uint8_t* tmp, TG* out, uint8_t* out_u8, int pitch, int W,
-                      int H, int r, const float* wts, const float* lut255, cudaStream_t st, int* launches,
-                      int fused_max_radius, const ImgRef* ref = nullptr, int tile_rows = 64);
+                      int H, int r, const float* wts, const TcBlur& b, const void* frags, const float* lut255,
+                      cudaStream_t st, int* launches, int fused_max_radius, const ImgRef* ref = nullptr,
+                      int tile_rows = 64);
 template <typename TG>
 int launch_copy_level(const TG* prev, const uint8_t* prev_u8, TG* out, uint8_t* out_u8, int pitch, int W,
                       int H, cudaStream_t st);
@@ -154,7 +155,26 @@ struct LevelBlur {
     float sigma;   // 0 = copy
     int radius;
     size_t woff;   // offset in the weight table
+    TcBlur tc;     // the tensor-core form of the taps
+    size_t foff;   // element offset of its fragments in the weight table
 };
+
+// Appends a blur's taps and then its tensor-core fragments to the weight
+// table (each part from a 16-byte boundary).
+inline void append_taps(const std::vector<float>& k, LevelBlur* b, std::vector<float>* wts) {
+    auto pad = [&] {
+        while (wts->size() % 4) wts->push_back(0.0f);
+    };
+    b->woff = wts->size();
+    wts->insert(wts->end(), k.begin(), k.end());
+    pad();
+    b->tc = tc_blur(k);
+    b->foff = wts->size();
+    wts->resize(b->foff + b->tc.frags.size());
+    if (!b->tc.frags.empty()) std::memcpy(wts->data() + b->foff, b->tc.frags.data(), b->tc.frags.size() * 4);
+    b->tc.frags.clear();
+    pad();
+}
 
 struct Engine {
     SiftCudaParams p{};
@@ -246,9 +266,10 @@ struct Engine {
 
     // Launch-shape knobs (set by the batch autotuner; the defaults are the
     // tuned values for single 1080p..4096 images): the largest blur radius
-    // that runs as one fused kernel, the persistent grids of the
-    // orientation and descriptor kernels in CTAs per SM, and the height of
-    // the fused level kernel's tiles (64 or 32 rows).
+    // that runs as one fused kernel (8: every radius it takes), the
+    // persistent grids of the orientation and descriptor kernels in CTAs per
+    // SM, and the height of the fused level kernel's tiles (64: by the
+    // plane's size; 32: always 32 rows).
     struct Tuning {
         int fused_max_radius = 8;
         int ori_ctas_per_sm = 4;
@@ -434,12 +455,11 @@ struct Engine {
         BlurPlan bp = blur_plan(p);
         std::vector<float> wts;
         auto add_blur = [&](float sigma) {
-            LevelBlur b{sigma, 0, wts.size()};
+            LevelBlur b{sigma, 0, wts.size(), {}, 0};
             if (sigma > 0.0f) {
                 auto k = gaussian_kernel(sigma);
                 b.radius = (int)(k.size() / 2);
-                wts.insert(wts.end(), k.begin(), k.end());
-                while (wts.size() % 4) wts.push_back(0.0f);
+                append_taps(k, &b, &wts);
             }
             return b;
         };
@@ -611,7 +631,7 @@ struct Engine {
             }
             int nl = 0;
             if (launch_blur_level<TG>(prev_u8, od.pitch, tmp, out, out_u8, od.pitch, od.W, od.H, b.radius,
-                                      wts + b.woff, lut, q, &nl, tune.fused_max_radius, nullptr,
+                                      wts + b.woff, b.tc, wts + b.foff, lut, q, &nl, tune.fused_max_radius, nullptr,
                                       tune.level_tile_rows))
                 return cuda_fail(cudaGetLastError(), "blur level");
             launches += nl;
@@ -702,8 +722,9 @@ struct Engine {
             if (base.sigma > 0.0f) {
                 int nl = 0;
                 if (launch_blur_level<TG>(img, (int)stride, d_tmp.as<uint8_t>(), G + o0.g_off, U + o0.u_off,
-                                          o0.pitch, o0.W, o0.H, base.radius, wts + base.woff, lut, st,
-                                          &nl, tune.fused_max_radius, d_ref.as<ImgRef>(), tune.level_tile_rows))
+                                          o0.pitch, o0.W, o0.H, base.radius, wts + base.woff, base.tc,
+                                          wts + base.foff, lut, st, &nl, tune.fused_max_radius, d_ref.as<ImgRef>(),
+                                          tune.level_tile_rows))
                     return cuda_fail(cudaGetLastError(), "blur (base)");
                 launches += nl;
             } else {

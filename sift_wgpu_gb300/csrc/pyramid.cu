@@ -17,10 +17,8 @@
 // 4-byte plane.
 //
 // Kernels
-//   k_blur_level   both separable passes of a level for r <= 8 (the first two
-//                  octaves at the default sigma): a 64 x 64 tile stages its
-//                  u8 window with 16-byte loads, the horizontal pass goes to
-//                  shared memory, the vertical pass writes level and u8.
+//   k_blur_level   both separable passes of a level for r <= 28 on the tensor
+//                  cores (level_tc.cuh), bit for bit the sequential sums.
 //   k_blur_rows    horizontal pass for larger radii, one row per CTA. u8 out.
 //   k_blur_cols    vertical pass for larger radii on a 32 x 64 tile.
 //   k_lanczos_fused  the 2x Lanczos3 resize between octaves, both passes.
@@ -29,7 +27,9 @@
 #include <cstring>
 #include <type_traits>
 
+#include "level_tc.cuh"
 #include "sift_internal.cuh"
+#include "tables.h"
 
 namespace sift {
 namespace {
@@ -179,6 +179,21 @@ __host__ __device__ constexpr int taps8(int r) { return ((2 * r + 1) + 7) & ~7; 
 
 template <typename TG>
 __device__ __forceinline__ void store_level4(TG* p, const int v[4], const float* lut);
+template <>
+__device__ __forceinline__ void store_level4<float>(float* p, const int v[4], const float* lut) {
+    *reinterpret_cast<float4*>(p) = make_float4(lut[v[0]], lut[v[1]], lut[v[2]], lut[v[3]]);
+}
+template <>
+__device__ __forceinline__ void store_level4<uint8_t>(uint8_t*, const int*, const float*) {}
+template <>
+__device__ __forceinline__ void store_level4<__half>(__half* p, const int v[4], const float*) {
+    const __half2 a = __halves2half2(__int2half_rn(v[0]), __int2half_rn(v[1]));
+    const __half2 b = __halves2half2(__int2half_rn(v[2]), __int2half_rn(v[3]));
+    uint2 u;
+    u.x = *reinterpret_cast<const unsigned*>(&a);
+    u.y = *reinterpret_cast<const unsigned*>(&b);
+    *reinterpret_cast<uint2*>(p) = u;
+}
 
 template <typename TG>
 __device__ __forceinline__ void blur_cols_tile(const uint8_t* __restrict__ tmp, int tmp_pitch, TG* __restrict__ out,
@@ -273,273 +288,21 @@ __global__ void __launch_bounds__(kColThreads) k_blur_cols(const uint8_t* __rest
                        blockIdx.y * kColRows, sm);
 }
 
-// ---------------------------------------------------------------------------
-// Packed pairs of f32: mul.rn.f32x2 rounds each of the two products like a
-// scalar multiply. The products are added to scalar accumulators: a packed
-// multiply followed by a packed add was measured to come out fused (one
-// rounding: a third of the sums differed from the reference's), a packed
-// multiply followed by scalar adds matched the scalar sequence on 2^20 sums.
-typedef unsigned long long f32x2;
-__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
-    f32x2 d;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-    return d;
-}
-__device__ __forceinline__ f32x2 pack2(float lo, float hi) {
-    return ((f32x2)__float_as_uint(hi) << 32) | __float_as_uint(lo);
-}
-__device__ __forceinline__ float lo2(f32x2 v) { return __uint_as_float((unsigned)v); }
-__device__ __forceinline__ float hi2(f32x2 v) { return __uint_as_float((unsigned)(v >> 32)); }
-// tap sum step for two accumulators: a + v * k, rounded after the products
-// and after the sums
-__device__ __forceinline__ void tap2(float& a_lo, float& a_hi, f32x2 v, f32x2 k) {
-    const f32x2 p = mul2(v, k);
-    a_lo = __fadd_rn(a_lo, lo2(p));
-    a_hi = __fadd_rn(a_hi, hi2(p));
-}
-
-// ---------------------------------------------------------------------------
-// Fused level kernel: both separable passes of one level in one launch, for
-// radii up to 8. The CTA stages the (64 + 2r)-row clamp-to-edge neighbourhood
-// of its 64 x 64 output tile from the previous level's u8 plane, runs the
-// horizontal pass for all 64 + 2r rows into shared memory (u8-truncated like
-// imageproc's intermediate image), then the vertical pass, and writes the
-// level and its u8 plane; each scale is read once, as bytes.
-//
-// Staged row layout: shared column c holds global x = x0 - 16 - sh + c with
-// sh = r mod 4, so an interior row is the 96 bytes [x0 - 16, x0 + 80) written
-// without conditions, and the horizontal pass's first input (x0 - r, column
-// 16 + sh - r) is 16-byte aligned for its float4 window. Each vertical-pass
-// thread owns 4 columns x 4 rows: one float4 shared load per tap, two packed
-// multiplies per row and tap, and vector stores of level and u8 copy.
-constexpr int kFTX = 64, kFTY = 64, kFThreads = 256;
-constexpr int kFMaxR = 8;
-constexpr int kFSW = 100;  // staged row stride (floats): sh + 96 <= 99
-
-size_t blur_fused_smem(int r, int ty = kFTY) {
-    const int taps = 2 * r + 1;
-    const size_t rows = (size_t)ty + 2 * r;
-    return sizeof(float) * ((size_t)3 * ((taps + 3) & ~3) + 256 + rows * kFSW + rows * kFTX);
-}
-
-template <typename TG>
-__device__ __forceinline__ void store_level4(TG* p, const int v[4], const float* lut);
-template <>
-__device__ __forceinline__ void store_level4<float>(float* p, const int v[4], const float* lut) {
-    *reinterpret_cast<float4*>(p) = make_float4(lut[v[0]], lut[v[1]], lut[v[2]], lut[v[3]]);
-}
-template <>
-__device__ __forceinline__ void store_level4<uint8_t>(uint8_t*, const int*, const float*) {}
-template <>
-__device__ __forceinline__ void store_level4<__half>(__half* p, const int v[4], const float*) {
-    const __half2 a = __halves2half2(__int2half_rn(v[0]), __int2half_rn(v[1]));
-    const __half2 b = __halves2half2(__int2half_rn(v[2]), __int2half_rn(v[3]));
-    uint2 u;
-    u.x = *reinterpret_cast<const unsigned*>(&a);
-    u.y = *reinterpret_cast<const unsigned*>(&b);
-    *reinterpret_cast<uint2*>(p) = u;
-}
-
-// Shared layout of the fused level kernel (floats): kw2[wpad] (pairs),
-// kw[wpad], lut[256], src[RH][kFSW] (staged input as floats), hb[RH][kFTX].
-// A tile is 64 columns by TY rows (64, or 32 for more, smaller CTAs on small
-// planes), computed by 4 * TY threads: 16 per row in the horizontal pass,
-// 4 x 4 outputs each in the vertical pass.
-template <int R, int TY = kFTY>
-struct FusedLayout {
-    static_assert(TY == 32 || TY == 64, "fused tile height");
-    static constexpr int taps = 2 * R + 1;
-    static constexpr int wpad = (taps + 3) & ~3;
-    static constexpr int RH = TY + 2 * R;
-    static constexpr int sh = R & 3;
-    static constexpr int threads = 4 * TY;
-};
-
-// the tap weights (single and paired) and the v / 255 table into shared memory
-template <int R, int TY = kFTY>
-__device__ __forceinline__ void blur_level_weights(const float* __restrict__ wts, const float* __restrict__ lut255,
-                                                   float* sm) {
-    using Lx = FusedLayout<R, TY>;
-    f32x2* kw2 = reinterpret_cast<f32x2*>(sm);
-    float* kw = sm + 2 * Lx::wpad;
-    float* lut = kw + Lx::wpad;
-    for (int i = threadIdx.x; i < Lx::wpad; i += Lx::threads) {
-        const float k = i < Lx::taps ? wts[i] : 0.0f;
-        kw2[i] = pack2(k, k);
-        kw[i] = k;
-    }
-    for (int i = threadIdx.x; i < 256; i += Lx::threads) lut[i] = lut255[i];
-}
-
-template <int R, int TY = kFTY>
-__device__ __forceinline__ bool blur_level_interior(int x0, int y0, int W, int H) {
-    return x0 >= 16 && x0 + 80 <= W && y0 >= R && y0 + TY + R <= H;
-}
-
-// Stages the tile's (TY + 2R)-row neighbourhood from the previous level's u8
-// plane (global memory) as floats: interior tiles with 16-byte loads of
-// [x0 - 16, x0 + 80), border tiles clamp-to-edge.
-template <int R, int TY = kFTY>
-__device__ __forceinline__ void blur_level_stage_global(const uint8_t* __restrict__ in, int in_pitch, int W, int H,
-                                                        int x0, int y0, float* sm) {
-    using Lx = FusedLayout<R, TY>;
-    float* src = sm + 3 * Lx::wpad + 256;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    if (blur_level_interior<R, TY>(x0, y0, W, H) && (in_pitch & 15) == 0) {
-        constexpr int Q = 6;
-        const uint8_t* org = in + (long long)(y0 - R) * in_pitch + (x0 - 16);
-#pragma unroll 2
-        for (int q = tid; q < Lx::RH * Q; q += Lx::threads) {
-            const int yy = q / Q, k = q - yy * Q;
-            float v[16];
-            unpack16(*reinterpret_cast<const uint4*>(org + (long long)yy * in_pitch + 16 * k), v);
-            float* d = src + (size_t)yy * kFSW + Lx::sh + 16 * k;
-#pragma unroll
-            for (int e = 0; e < 16; ++e) d[e] = v[e];
-        }
-    } else {
-        // clamp-to-edge, only the columns the passes read: 16 + sh - R .. sh + 80 + R
-        for (int yy = warp; yy < Lx::RH; yy += Lx::threads / 32) {
-            const uint8_t* row = in + (long long)clampi(y0 - R + yy, 0, H - 1) * in_pitch;
-            float* d = src + (size_t)yy * kFSW;
-            for (int c = 16 + Lx::sh - R + lane; c <= Lx::sh + 80 + R; c += 32)
-                d[c] = float_of_u8(row[clampi(x0 - 16 - Lx::sh + c, 0, W - 1)]);
-        }
-    }
-}
-
-// Both passes from the staged floats (the caller synchronises the CTA
-// between staging and this): horizontal pass into hb, then the vertical pass,
-// writing the level and its u8 plane.
-template <typename TG, int R, int TY = kFTY>
-__device__ __forceinline__ void blur_level_compute(TG* __restrict__ out, uint8_t* __restrict__ out_u8, int pitch,
-                                                   int W, int H, int x0, int y0, float* sm) {
-    using Lx = FusedLayout<R, TY>;
-    constexpr int taps = Lx::taps;
-    constexpr int RH = Lx::RH;
-    constexpr int sh = Lx::sh;
-    const f32x2* kw2 = reinterpret_cast<const f32x2*>(sm);
-    const float* kw = sm + 2 * Lx::wpad;
-    const float* lut = kw + Lx::wpad;
-    const float* src = lut + 256;
-    float* hb = const_cast<float*>(src) + (size_t)RH * kFSW;
-    const int tid = threadIdx.x;
-    // horizontal pass: 16 threads per row, 4 outputs each (float4 sliding window)
-    {
-        const int xq = (tid & 15) * 4;
-        for (int yy = tid >> 4; yy < RH; yy += Lx::threads / 16) {
-            const float* base = src + (size_t)yy * kFSW + (16 + sh - R) + xq;
-            float a0 = 0.0f, a1 = 0.0f, a2 = 0.0f, a3 = 0.0f;
-            float4 A = *reinterpret_cast<const float4*>(base);
-            int i = 0;
-#pragma unroll
-            for (; i + 4 <= taps; i += 4) {
-                const float4 B = *reinterpret_cast<const float4*>(base + i + 4);
-                const float4 K = *reinterpret_cast<const float4*>(kw + i);
-                a0 = __fadd_rn(a0, __fmul_rn(A.x, K.x));
-                a1 = __fadd_rn(a1, __fmul_rn(A.y, K.x));
-                a2 = __fadd_rn(a2, __fmul_rn(A.z, K.x));
-                a3 = __fadd_rn(a3, __fmul_rn(A.w, K.x));
-                a0 = __fadd_rn(a0, __fmul_rn(A.y, K.y));
-                a1 = __fadd_rn(a1, __fmul_rn(A.z, K.y));
-                a2 = __fadd_rn(a2, __fmul_rn(A.w, K.y));
-                a3 = __fadd_rn(a3, __fmul_rn(B.x, K.y));
-                a0 = __fadd_rn(a0, __fmul_rn(A.z, K.z));
-                a1 = __fadd_rn(a1, __fmul_rn(A.w, K.z));
-                a2 = __fadd_rn(a2, __fmul_rn(B.x, K.z));
-                a3 = __fadd_rn(a3, __fmul_rn(B.y, K.z));
-                a0 = __fadd_rn(a0, __fmul_rn(A.w, K.w));
-                a1 = __fadd_rn(a1, __fmul_rn(B.x, K.w));
-                a2 = __fadd_rn(a2, __fmul_rn(B.y, K.w));
-                a3 = __fadd_rn(a3, __fmul_rn(B.z, K.w));
-                A = B;
-            }
-#pragma unroll
-            for (; i < taps; ++i) {
-                const float k = kw[i];
-                a0 = __fadd_rn(a0, __fmul_rn(base[i + 0], k));
-                a1 = __fadd_rn(a1, __fmul_rn(base[i + 1], k));
-                a2 = __fadd_rn(a2, __fmul_rn(base[i + 2], k));
-                a3 = __fadd_rn(a3, __fmul_rn(base[i + 3], k));
-            }
-            const float4 o4 = make_float4(clamp_u8f(a0), clamp_u8f(a1), clamp_u8f(a2), clamp_u8f(a3));
-            *reinterpret_cast<float4*>(hb + (size_t)yy * kFTX + xq) = o4;
-        }
-    }
-    __syncthreads();
-    // vertical pass: thread = 4 columns x 4 rows, a 4-row float4 window
-    // sliding down the taps
-    const int cg = tid & 15, rg = tid >> 4;
-    const ulonglong2* hb2 = reinterpret_cast<const ulonglong2*>(hb) + cg;  // row stride kFTX / 4
-    float4 acc[4];
-#pragma unroll
-    for (int j = 0; j < 4; ++j) acc[j] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    ulonglong2 w0 = hb2[(4 * rg + 0) * (kFTX / 4)], w1 = hb2[(4 * rg + 1) * (kFTX / 4)],
-               w2 = hb2[(4 * rg + 2) * (kFTX / 4)];
-#pragma unroll
-    for (int i = 0; i < taps; ++i) {
-        const ulonglong2 w3 = hb2[(4 * rg + i + 3) * (kFTX / 4)];
-        const f32x2 k = kw2[i];
-        const ulonglong2 w[4] = {w0, w1, w2, w3};
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            tap2(acc[j].x, acc[j].y, w[j].x, k);
-            tap2(acc[j].z, acc[j].w, w[j].y, k);
-        }
-        w0 = w1;
-        w1 = w2;
-        w2 = w3;
-    }
-    const int xc = x0 + 4 * cg;
-    if (xc >= W) return;
-    const bool full = xc + 3 < W;
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-        const int y = y0 + 4 * rg + j;
-        if (y >= H) break;
-        const int v[4] = {to_u8(acc[j].x), to_u8(acc[j].y), to_u8(acc[j].z), to_u8(acc[j].w)};
-        const long long o = (long long)y * pitch + xc;
-        if (full) {
-            store_level4(out + o, v, lut);
-            *reinterpret_cast<unsigned*>(out_u8 + o) =
-                (unsigned)v[0] | ((unsigned)v[1] << 8) | ((unsigned)v[2] << 16) | ((unsigned)v[3] << 24);
-        } else {
-            for (int c = 0; c < 4 && xc + c < W; ++c) {
-                store_level(out + o + c, v[c], lut[v[c]]);
-                out_u8[o + c] = (uint8_t)v[c];
-            }
-        }
-    }
-}
-
-
-template <typename TG, int R, int TY = kFTY>
-__device__ __forceinline__ void blur_level_tile(const uint8_t* __restrict__ in, int in_pitch, TG* __restrict__ out,
-                                                uint8_t* __restrict__ out_u8, int pitch, int W, int H,
-                                                const float* __restrict__ wts, const float* __restrict__ lut255,
-                                                int x0, int y0, float* sm) {
-    static_assert(R >= 1 && R <= kFMaxR, "fused radius");
-    blur_level_weights<R, TY>(wts, lut255, sm);
-    blur_level_stage_global<R, TY>(in, in_pitch, W, H, x0, y0, sm);
-    __syncthreads();
-    blur_level_compute<TG, R, TY>(out, out_u8, pitch, W, H, x0, y0, sm);
-}
-
-template <typename TG, int R, int TY>
-__global__ void __launch_bounds__(4 * TY) k_blur_level(const uint8_t* __restrict__ in, int in_pitch,
-                                                          TG* __restrict__ out, uint8_t* __restrict__ out_u8,
-                                                          int pitch, int W, int H,
-                                                          const float* __restrict__ wts,
-                                                          const float* __restrict__ lut255,
-                                                          const ImgRef* __restrict__ ref) {
+// Fused level kernel: both passes of one level on the tensor cores
+// (level_tc.cuh), a 64 x TY tile per CTA.
+template <typename TG, int P, int PV, int TY, bool CLAMP>
+__global__ void __launch_bounds__(tc::kThreads) k_blur_level(const uint8_t* __restrict__ in, int in_pitch,
+                                                             TG* __restrict__ out, uint8_t* __restrict__ out_u8,
+                                                             int pitch, int W, int H, TcParams tp,
+                                                             const ImgRef* __restrict__ ref) {
     chain_wait();
     if (ref) {  // a host call's base level: the image is wherever the cell says
         in = ref->ptr;
         in_pitch = (int)ref->pitch;
     }
-    extern __shared__ __align__(16) float sm[];
-    blur_level_tile<TG, R, TY>(in, in_pitch, out, out_u8, pitch, W, H, wts, lut255, blockIdx.x * kFTX,
-                               blockIdx.y * TY, sm);
+    extern __shared__ __align__(16) uint16_t smh[];
+    tc::level_tile<TG, P, PV, TY, CLAMP>(in, in_pitch, out, out_u8, pitch, W, H, tp, blockIdx.x * tc::kTX,
+                                         blockIdx.y * TY, smh);
 }
 
 // A level whose blur increment is below 1e-4 is a copy of the previous one
@@ -749,6 +512,7 @@ __global__ void k_lanczos_h(const float* __restrict__ src, int src_pitch, TG* __
 // serves the image k with pref[k] <= b < pref[k + 1], where pref is the
 // launch's prefix over the images' tile (or row) counts, and tile b - pref[k]
 // of that image; the tile bodies are the single-image kernels' own.
+constexpr int kBatchTY = 64;
 __device__ __forceinline__ int find_image(const uint32_t* __restrict__ pref, int n, uint32_t b) {
     int lo = 0, hi = n;
     while (hi - lo > 1) {
@@ -769,21 +533,19 @@ __device__ __forceinline__ const uint8_t* level_src(const BatchPyr& bp, const Oc
     return bp.U + od.u_off + (long long)(s - 1) * od.plane;
 }
 
-template <int R>
-__global__ void __launch_bounds__(kFThreads) kb_blur_level(BatchPyr bp, int o, int s, int n_img,
-                                                           const uint32_t* __restrict__ pref,
-                                                           const float* __restrict__ wts,
-                                                           const float* __restrict__ lut255) {
+template <int P, int PV, bool CLAMP>
+__global__ void __launch_bounds__(tc::kThreads) kb_blur_level(BatchPyr bp, int o, int s, int n_img,
+                                                              const uint32_t* __restrict__ pref, TcParams tp) {
     chain_wait();
-    extern __shared__ __align__(16) float sm[];
+    extern __shared__ __align__(16) uint16_t smh[];
     const int k = find_image(pref, n_img, blockIdx.x);
     const OctaveDev od = bp.ents[k * bp.O + o];
-    const int t = (int)(blockIdx.x - pref[k]), tx = (od.W + kFTX - 1) / kFTX;
+    const int t = (int)(blockIdx.x - pref[k]), tx = (od.W + tc::kTX - 1) / tc::kTX;
     int in_pitch = 0;
     const uint8_t* in = level_src(bp, od, k, s, &in_pitch);
     uint8_t* out = bp.U + od.u_off + (long long)s * od.plane;
-    blur_level_tile<uint8_t, R>(in, in_pitch, out, out, od.pitch, od.W, od.H, wts, lut255, (t % tx) * kFTX,
-                                (t / tx) * kFTY, sm);
+    tc::level_tile<uint8_t, P, PV, kBatchTY, CLAMP>(in, in_pitch, out, out, od.pitch, od.W, od.H, tp, (t % tx) * tc::kTX,
+                                                    (t / tx) * kBatchTY, smh);
 }
 
 __global__ void __launch_bounds__(kRowThreads) kb_blur_rows(BatchPyr bp, uint8_t* __restrict__ tmp, int o, int s,
@@ -847,55 +609,66 @@ size_t blur_cols_smem(int r) {
     return sizeof(float) * ((size_t)taps8(r) + 256 + (size_t)(kColRows + taps8(r) - 1) * kColTX);
 }
 
+// 64-row tiles from this many on (two per multiprocessor): fewer leave
+// multiprocessors idle or with one CTA, and 32-row tiles, which recompute
+// more halo (48 against 80 rows per 64), still finish sooner.
+constexpr long long kTallTiles = 2 * 152;
+
 static int set_smem(const void* k, size_t smem) {
     if (smem <= 48 * 1024) return 0;
     return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) == cudaSuccess ? 0 : -1;
 }
 
-// One level from the previous level's u8 plane: fused when r <= 8 and r <=
-// fused_max_radius (the horizontal pass recomputes a 2r-row halo per tile,
-// which stops paying beyond r = 8), on tiles of tile_rows (64 or 32) rows,
-// else the two separable passes.
-template <typename TG, int TY>
-using BlurLevelKernel = void (*)(const uint8_t*, int, TG*, uint8_t*, int, int, int, const float*, const float*,
-                                 const ImgRef*);
-template <typename TG, int TY>
-BlurLevelKernel<TG, TY> blur_level_kernel(int r) {
-    switch (r) {
-        case 1: return k_blur_level<TG, 1, TY>;
-        case 2: return k_blur_level<TG, 2, TY>;
-        case 3: return k_blur_level<TG, 3, TY>;
-        case 4: return k_blur_level<TG, 4, TY>;
-        case 5: return k_blur_level<TG, 5, TY>;
-        case 6: return k_blur_level<TG, 6, TY>;
-        case 7: return k_blur_level<TG, 7, TY>;
-        default: return k_blur_level<TG, 8, TY>;
-    }
+// The level kernel's shape for a radius: f(P, PV) with the smallest window
+// and rows that hold it (tables.cpp: tc_blur lays the fragments out for them).
+template <class F>
+static int for_tc_shape(int r, F f) {
+    if (r <= 4) return f(std::integral_constant<int, 4>{}, std::integral_constant<int, 8>{});
+    if (r <= 8) return f(std::integral_constant<int, 12>{}, std::integral_constant<int, 8>{});
+    if (r <= 12) return f(std::integral_constant<int, 12>{}, std::integral_constant<int, 16>{});
+    if (r <= 16) return f(std::integral_constant<int, 20>{}, std::integral_constant<int, 16>{});
+    if (r <= 20) return f(std::integral_constant<int, 20>{}, std::integral_constant<int, 24>{});
+    if (r <= 24) return f(std::integral_constant<int, 28>{}, std::integral_constant<int, 24>{});
+    return f(std::integral_constant<int, 28>{}, std::integral_constant<int, 32>{});
 }
 
-template <typename TG, int TY>
-int launch_blur_level_fused(const uint8_t* in, int in_pitch, TG* out, uint8_t* out_u8, int pitch, int W, int H,
-                            int r, const float* wts, const float* lut255, cudaStream_t st, const ImgRef* ref) {
-    const BlurLevelKernel<TG, TY> kern = blur_level_kernel<TG, TY>(r);
-    const size_t smem = blur_fused_smem(r, TY);
+template <typename TG, int P, int PV, int TY, bool CLAMP>
+int launch_blur_level_tc(const uint8_t* in, int in_pitch, TG* out, uint8_t* out_u8, int pitch, int W, int H,
+                         const TcParams& tp, cudaStream_t st, const ImgRef* ref) {
+    constexpr size_t smem = tc::Shape<P, PV, TY>::smem;
+    const auto kern = k_blur_level<TG, P, PV, TY, CLAMP>;
     if (set_smem((const void*)kern, smem)) return -1;
-    dim3 grid((W + kFTX - 1) / kFTX, (H + TY - 1) / TY);
-    if (launch_chained(kern, grid, 4 * TY, smem, st, in, in_pitch, out, out_u8, pitch, W, H, wts, lut255, ref) !=
+    dim3 grid((W + tc::kTX - 1) / tc::kTX, (H + TY - 1) / TY);
+    if (launch_chained(kern, grid, tc::kThreads, smem, st, in, in_pitch, out, out_u8, pitch, W, H, tp, ref) !=
         cudaSuccess)
         return -1;
     return cudaPeekAtLastError() == cudaSuccess ? 0 : -1;
 }
 
+// One level from the previous level's u8 plane: one launch on the tensor
+// cores for the radii it takes (up to 28) unless the autotuner's radius limit
+// (below 8) excludes them, else the two separable passes.
+static bool level_fused(const TcBlur& b, int r, int fused_max_radius) {
+    return b.ok && (fused_max_radius >= 8 || r <= fused_max_radius);
+}
+
 template <typename TG>
 int launch_blur_level(const uint8_t* in, int in_pitch, uint8_t* tmp, TG* out, uint8_t* out_u8, int pitch, int W,
-                      int H, int r, const float* wts, const float* lut255, cudaStream_t st, int* launches,
-                      int fused_max_radius, const ImgRef* ref, int tile_rows) {
-    if (r <= kFMaxR && r <= fused_max_radius) {
-        const int rc = tile_rows == 32
-                           ? launch_blur_level_fused<TG, 32>(in, in_pitch, out, out_u8, pitch, W, H, r, wts, lut255,
-                                                             st, ref)
-                           : launch_blur_level_fused<TG, 64>(in, in_pitch, out, out_u8, pitch, W, H, r, wts, lut255,
-                                                             st, ref);
+                      int H, int r, const float* wts, const TcBlur& b, const void* frags, const float* lut255,
+                      cudaStream_t st, int* launches, int fused_max_radius, const ImgRef* ref, int tile_rows) {
+    if (level_fused(b, r, fused_max_radius)) {
+        const TcParams tp{static_cast<const uint4*>(frags), wts, r, b.init_a, b.init_b, b.scale_b, b.whole, b.near};
+        // planes whose 64-row tiles would leave multiprocessors idle take 32-row tiles
+        const bool tall = tile_rows != 32 && (long long)((W + 63) / 64) * ((H + 63) / 64) >= kTallTiles;
+        const int rc = for_tc_shape(r, [&](auto p, auto pv) {
+            constexpr int P = decltype(p)::value, PV = decltype(pv)::value;
+            if constexpr (P == 4) {  // only narrow kernels sum to 256
+                if (b.clamp)
+                    return launch_blur_level_tc<TG, P, PV, 32, true>(in, in_pitch, out, out_u8, pitch, W, H, tp, st, ref);
+            }
+            return tall ? launch_blur_level_tc<TG, P, PV, 64, false>(in, in_pitch, out, out_u8, pitch, W, H, tp, st, ref)
+                        : launch_blur_level_tc<TG, P, PV, 32, false>(in, in_pitch, out, out_u8, pitch, W, H, tp, st, ref);
+        });
         if (rc) return rc;
         *launches += 1;
         return 0;
@@ -961,7 +734,7 @@ int lanczos_fused_span() { return kLzSpan; }
 
 // ---- flattened batch launchers ------------------------------------------------
 
-int blur_level_tiles(int W, int H) { return W > 0 && H > 0 ? ((W + kFTX - 1) / kFTX) * ((H + kFTY - 1) / kFTY) : 0; }
+int blur_level_tiles(int W, int H) { return W > 0 && H > 0 ? ((W + tc::kTX - 1) / tc::kTX) * ((H + kBatchTY - 1) / kBatchTY) : 0; }
 int blur_col_tiles(int W, int H) {
     return W > 0 && H > 0 ? ((W + kColTX - 1) / kColTX) * ((H + kColRows - 1) / kColRows) : 0;
 }
@@ -972,32 +745,30 @@ void batch_lz_fill(void* out, int vtab, int vw, int htab, int hw, const LanczosU
     std::memcpy(out, &z, sizeof z);
 }
 
-// Level s of octave o of every image of a batch: the fused kernel (r <= 8,
-// tiles prefixed by fused_pref) or the two passes (rows prefixed by
+// Level s of octave o of every image of a batch: the fused kernel (tiles
+// prefixed by fused_pref) or the two passes (rows prefixed by
 // rows_pref, column tiles by cols_pref; tmp holds each entry's
 // horizontal-pass plane at its t_off).
 int launch_blur_level_flat(const BatchPyr& bp, uint8_t* tmp, int o, int s, int r, int n_img,
                            const uint32_t* fused_pref, uint32_t n_fused, const uint32_t* rows_pref, uint32_t n_rows,
-                           int max_w, const uint32_t* cols_pref, uint32_t n_cols, const float* wts,
-                           const float* lut255, cudaStream_t st, int* launches, int fused_max_radius) {
-    if (r <= kFMaxR && r <= fused_max_radius) {
+                           int max_w, const uint32_t* cols_pref, uint32_t n_cols, const float* wts, const TcBlur& b,
+                           const void* frags, const float* lut255, cudaStream_t st, int* launches) {
+    if (level_fused(b, r, 8)) {
         if (n_fused == 0) return 0;
-        void (*kern)(BatchPyr, int, int, int, const uint32_t*, const float*, const float*);
-        switch (r) {
-            case 1: kern = kb_blur_level<1>; break;
-            case 2: kern = kb_blur_level<2>; break;
-            case 3: kern = kb_blur_level<3>; break;
-            case 4: kern = kb_blur_level<4>; break;
-            case 5: kern = kb_blur_level<5>; break;
-            case 6: kern = kb_blur_level<6>; break;
-            case 7: kern = kb_blur_level<7>; break;
-            default: kern = kb_blur_level<8>; break;
-        }
-        const size_t smem = blur_fused_smem(r);
-        if (set_smem((const void*)kern, smem)) return -1;
-        if (launch_chained(kern, n_fused, kFThreads, smem, st, bp, o, s, n_img, fused_pref, wts, lut255) !=
-            cudaSuccess)
-            return -1;
+        const TcParams tp{static_cast<const uint4*>(frags), wts, r, b.init_a, b.init_b, b.scale_b, b.whole, b.near};
+        auto go = [&](auto kern, size_t smem) -> int {
+            if (set_smem((const void*)kern, smem)) return -1;
+            return launch_chained(kern, n_fused, tc::kThreads, smem, st, bp, o, s, n_img, fused_pref, tp) == cudaSuccess ? 0 : -1;
+        };
+        const int rc = for_tc_shape(r, [&](auto p, auto pv) {
+            constexpr int P = decltype(p)::value, PV = decltype(pv)::value;
+            constexpr size_t smem = tc::Shape<P, PV, kBatchTY>::smem;
+            if constexpr (P == 4) {
+                if (b.clamp) return go(kb_blur_level<P, PV, true>, smem);
+            }
+            return go(kb_blur_level<P, PV, false>, smem);
+        });
+        if (rc) return rc;
         *launches += 1;
         return cudaPeekAtLastError() == cudaSuccess ? 0 : -1;
     }
@@ -1028,7 +799,8 @@ int lanczos_fused_tile() { return kLzT; }
 
 #define SIFT_INST(TG)                                                                                              \
     template int launch_blur_level<TG>(const uint8_t*, int, uint8_t*, TG*, uint8_t*, int, int, int, int,           \
-                                       const float*, const float*, cudaStream_t, int*, int, const ImgRef*, int);   \
+                                       const float*, const TcBlur&, const void*, const float*, cudaStream_t, int*, \
+                                       int, const ImgRef*, int);                                                   \
     template int launch_copy_level<TG>(const TG*, const uint8_t*, TG*, uint8_t*, int, int, int,                    \
                                        cudaStream_t);                                                              \
     template int launch_u8_to_level<TG>(const uint8_t*, long long, TG*, uint8_t*, int, int, int, cudaStream_t,     \

@@ -66,6 +66,115 @@ std::vector<float> gaussian_kernel(float sigma) {
     return k;
 }
 
+namespace {
+// The f16 bits of a whole number of at most 11 significant bits.
+uint32_t half_of_int(int v) {
+    const uint32_t s = v < 0 ? 0x8000u : 0u;
+    uint32_t m = (uint32_t)(v < 0 ? -v : v);
+    if (m == 0) return 0;
+    int e = 0;
+    while (m >> (e + 1)) ++e;
+    m = e <= 10 ? m << (10 - e) : m >> (e - 10);
+    return s | (uint32_t)(e + 15) << 10 | (m & 0x3ffu);
+}
+}  // namespace
+
+// Weights W = round(w 2^q) as a 2^shift + b with whole limbs that f16 holds
+// (a <= 2048) and whose sums over 255-valued pixels stay below 2^24, so the
+// tensor core's f32 accumulators hold both sums exactly whatever its order of
+// addition. The level value s = sum(W p) / 2^q is then known to within
+//   quantisation   255 max(sum of the positive, sum of the negative w - W/2^q)
+//   the reference's rounding: one per product, one per partial sum of the
+//                  sequential f32 sum, each at most 2^-24 of its value, the
+//                  partial sum after tap k being at most 255 (w_0 + .. + w_k)
+//   the kernel's   2^-16 (2^-15 with 9 whole bits), rounding the two limbs'
+//                  sum to 15 (14) fraction bits
+// The kernel adds that bound e to s and takes floor(s + e) where its fraction
+// is at least 2 e (there the reference truncates to the same integer); the
+// other pixels, a few in 10^4, are summed again in the reference's order.
+TcBlur tc_blur(const std::vector<float>& w) {
+    TcBlur t;
+    const int n = (int)w.size(), r = n / 2;
+    if (n < 1 || r > 28) return t;
+    double wmax = 0.0, wsum = 0.0;
+    for (float v : w) {
+        if (!(v >= 0.0f)) return t;
+        wmax = std::max(wmax, (double)v);
+        wsum += v;
+    }
+    if (!(wmax > 0.0)) return t;
+    // a = w 2^qa <= 2047, sums of a below 2^24 / 2 with the start value
+    int qa = 15;
+    while (qa > 4 && wmax * std::ldexp(1.0, qa) > 2040.0) --qa;
+    std::vector<long long> a(n), b(n);
+    int shift = 12;
+    double quant = 0.0;
+    for (;; --shift) {
+        if (shift < 4) return t;
+        long long sb = 0;
+        double up = 0.0, down = 0.0;
+        for (int i = 0; i < n; ++i) {
+            const long long W = std::llrint(std::ldexp((double)w[i], qa + shift));
+            a[i] = (W + (1ll << (shift - 1))) >> shift;
+            b[i] = W - a[i] * (1ll << shift);
+            sb += b[i] < 0 ? -b[i] : b[i];
+            const double d = (double)w[i] - std::ldexp((double)W, -(qa + shift));
+            (d > 0 ? up : down) += std::fabs(d);
+        }
+        quant = 255.0 * std::max(up, down);
+        if (sb * 255 < (1ll << 23)) break;
+    }
+    for (int i = 0; i < n; ++i)
+        if (a[i] > 2047) return t;
+    const double u = std::ldexp(1.0, -24);
+    double cum = 0.0, steps = 0.0;
+    for (int i = 0; i < n; ++i) {
+        cum += w[i];
+        steps += cum;
+    }
+    const double ref = 255.0 * u * (steps + wsum) * (1.0 + 4.0 * n * u);
+    t.clamp = 255.0 * wsum + 1.0 >= 256.0;
+    const int frac = t.clamp ? 14 : 15;
+    if (255.0 * wsum + 1.0 >= std::ldexp(1.0, 23 - frac) || qa + 24 - frac > 24) return t;
+    const double e = quant + ref + std::ldexp(1.0, -frac);
+    // s in units of 1 is 2^(qa - 24) in the accumulators (pixels enter as
+    // f16 subnormals, v 2^-24); the start value puts s in the mantissa with
+    // `frac` fraction bits
+    t.init_a = (float)std::ldexp(1.0, qa + (23 - frac) - 24);
+    const double be = std::ceil(std::ldexp(e, qa + shift));  // whole b units
+    if (be * 2 >= std::ldexp(1.0, 24)) return t;
+    t.init_b = (float)std::ldexp(be, -24);
+    t.scale_b = (float)std::ldexp(1.0, -shift);
+    t.whole = (float)(std::ldexp(1.0, qa - 24 + 23) - t.init_a);
+    const uint32_t thr = (uint32_t)std::ceil(2.0 * std::ldexp(be, frac - qa - shift)) + 1u;
+    uint32_t p2 = 1;
+    while (p2 < thr) p2 <<= 1;
+    if (p2 >> (frac - 2)) return t;
+    t.near = ((1u << frac) - 1u) & ~(p2 - 1u);
+    // fragments (m16n8k16): lane = 4 g + t holds k = 2t, 2t+1 (+8)
+    const int P = r <= 4 ? 4 : (r + 3) / 8 * 8 + 4, PV = (r + 7) / 8 * 8;
+    t.kh = (8 + 2 * P) / 16;
+    t.kv = (16 + 2 * PV) / 16;
+    auto pair = [&](const std::vector<long long>& v, int i) -> uint32_t {  // taps i, i + 1
+        auto at = [&](int j) { return j >= 0 && j < n ? half_of_int((int)v[(size_t)j]) : 0u; };
+        return at(i) | at(i + 1) << 16;
+    };
+    for (int ks = 0; ks < t.kh; ++ks)
+        for (int lane = 0; lane < 32; ++lane) {
+            const int g = lane >> 2, k = 16 * ks + 2 * (lane & 3), i = k - g - (P - r);  // column n = g
+            for (const auto* v : {&a, &b})
+                for (int d : {0, 8}) t.frags.push_back(pair(*v, i + d));
+        }
+    for (int ks = 0; ks < t.kv; ++ks)
+        for (int lane = 0; lane < 32; ++lane) {
+            const int g = lane >> 2, k = 16 * ks + 2 * (lane & 3), i = k - g - (PV - r);  // row m = g, g + 8
+            for (const auto* v : {&a, &b})
+                for (int d : {0, -8, 8, 0}) t.frags.push_back(pair(*v, i + d));
+        }
+    t.ok = true;
+    return t;
+}
+
 AxisTaps lanczos_axis(uint32_t src, uint32_t dst) {
     AxisTaps t;
     float ratio = (float)src / (float)dst;
