@@ -96,7 +96,7 @@ struct BatchEngine {
     std::vector<std::vector<LevelBlur>> lv;
     size_t lut_off = 0;
 
-    DevMem d_img, d_U, d_tmp, d_tmp2, d_ents, d_pref, d_imgaddr, d_imgpitch, d_wts, d_ltab, d_lw, d_lz;
+    DevMem d_cell, d_img, d_U, d_tmp, d_tmp2, d_ents, d_pref, d_imgaddr, d_imgpitch, d_wts, d_ltab, d_lw, d_lz;
     // the device reads pageable host memory coherently (Grace's address
     // translation): the base level then reads the caller's images in place
     bool host_reads = false;
@@ -372,6 +372,12 @@ struct BatchEngine {
         hx_dranges = reinterpret_cast<uint32_t*>(dptr + hx_ranges_off());
         hx_dkps = reinterpret_cast<Keypoint*>(dptr + hx_kps_off());
         hx_ddesc = reinterpret_cast<float*>(dptr + hx_desc_off());
+        RunCell c{};  // what the descriptor stage reads of it
+        c.desc = hx_ddesc;
+        c.cap = cap_x;
+        CK(d_cell.ensure(sizeof c), "cudaMalloc(run cell)");
+        CK(cudaMemcpyAsync(d_cell.p, &c, sizeof c, cudaMemcpyHostToDevice, st), "H2D run cell");
+        CK(cudaStreamSynchronize(st), "run cell");
         return 0;
     }
 
@@ -466,7 +472,7 @@ struct BatchEngine {
             return rc;
         const int dgrid = (int)std::max<uint32_t>(cap_cand / 16, 64);
         if (int rc = bump(launch_descriptor<uint8_t>(U, tb, d_oriented.as<Keypoint>(), oc, d_desc.as<float>(),
-                                                     cap_ori, hx_ddesc, cap_x, dgrid, 152 * 8, st),
+                                                     cap_ori, d_cell.as<RunCell>(), dgrid, 152 * 8, st),
                           "batch descriptor"))
             return rc;
         if (launch_chained(k_batch_export, 152 * 4, 256, 0, st, d_ents.as<OctaveDev>(), O, N, total_words,

@@ -441,7 +441,7 @@ constexpr int kDescGridSide = 2 * kDescRadGrid + 3;   // offsets -(rad+1) .. rad
 
 // The descriptor of one oriented keypoint (src/sift.rs:917-1060 and
 // normalize_and_clip_descriptor, src/sift.rs:889-913), computed by the whole
-// CTA (kDescThreads threads; it synchronises the CTA) into dst[0 .. 128):
+// CTA (kDescThreads threads; it synchronises the CTA) into dst()[0 .. 128):
 //  1. The bilinear samples the gradients need, bilinear(xo + i, yo + j) for
 //     integer offsets i, j in [-(rad+1), rad+1], go to a shared grid once
 //     (the reference re-evaluates four bilinears per window sample).
@@ -454,10 +454,10 @@ constexpr int kDescGridSide = 2 * kDescRadGrid + 3;   // offsets -(rad+1) .. rad
 //  3. The four warps normalise, clip at 0.2, renormalise.
 // Radii above the grid (not reachable with the default sigma) fall back to
 // per-sample bilinears from the level itself.
-template <typename TG>
+template <typename TG, class Dst>
 __device__ __forceinline__ void describe_one(const TG* __restrict__ arena, const EntryTable& tab, const Keypoint& kp,
                                              float* grid, unsigned int* hist, float* red_lo, float* red_hi,
-                                             float* __restrict__ dst) {
+                                             const Dst& dst) {
     const int tid = threadIdx.x;
     const float sqrt2 = __fsqrt_rn(2.0f);
     const int e = kp.octave;  // entry
@@ -827,7 +827,7 @@ __device__ __forceinline__ void describe_one(const TG* __restrict__ arena, const
                 __fsqrt_rn(__fadd_rn(__fadd_rn(red_hi[0], red_hi[1]), __fadd_rn(red_hi[2], red_hi[3])));
             if (!(n2 < 1e-8f)) d = __fmul_rn(d, __fdiv_rn(1.0f, n2));
         }
-            dst[bin] = d;
+        dst()[bin] = d;
     }
 }
 
@@ -845,7 +845,7 @@ __global__ void __launch_bounds__(kDescThreads, 8) k_descriptor(const TG* __rest
                                                               const Keypoint* __restrict__ oriented,
                                                               OctCounters* __restrict__ oc,
                                                               float* __restrict__ desc, uint32_t cap,
-                                                              float* __restrict__ hdesc, uint32_t hcap,
+                                                              const RunCell* __restrict__ cell,
                                                               int persist_from) {
     chain_wait();
     __shared__ __align__(16) float grid[kDescGridSide * (kDescGridSide + 1)];
@@ -860,8 +860,15 @@ __global__ void __launch_bounds__(kDescThreads, 8) k_descriptor(const TG* __rest
     // claims the next item while the CTA works on the current one (slot
     // next[p ^ 1]), unless the CTA retires after the current one.
     __shared__ uint32_t next[2];
+    // a host call's mapped result buffer, by the run's cell
+    __shared__ float* hdesc;
+    __shared__ uint32_t hcap;
     const bool persist = (int)blockIdx.x >= persist_from;
-    if (tid == 0) next[0] = atomicAdd(&oc->next_desc, 1u);
+    if (tid == 0) {
+        next[0] = atomicAdd(&oc->next_desc, 1u);
+        hdesc = cell ? cell->desc : nullptr;
+        hcap = cell ? cell->cap : 0u;
+    }
     for (int taken = 0, p = 0;; ++taken, p ^= 1) {
         __syncthreads();  // next[p] is visible, the grid and histogram are free
         const uint32_t cur = next[p];
@@ -875,7 +882,8 @@ __global__ void __launch_bounds__(kDescThreads, 8) k_descriptor(const TG* __rest
         const uint32_t i = base + (n - 1 - cur);
         const Keypoint kp = oriented[i];
         // keypoints below hcap straight into the host call's mapped buffer
-        describe_one<TG>(arena, tab, kp, grid, hist, red_lo, red_hi, (i < hcap ? hdesc : desc) + (size_t)i * kDescLen);
+        describe_one<TG>(arena, tab, kp, grid, hist, red_lo, red_hi,
+                         [&] { return (i < hcap ? hdesc : desc) + (size_t)i * kDescLen; });
         if (tid == 0) next[p ^ 1] = claim;
     }
 }
@@ -904,11 +912,10 @@ int launch_orient_emit(const Keypoint* refined_at, uint32_t ncap, int o, Counter
 
 template <typename TG>
 int launch_descriptor(const TG* arena, const EntryTable& tab, const Keypoint* oriented,
-                      OctCounters* oc, float* desc, uint32_t cap, float* hdesc, uint32_t hcap, int grid,
-                      int persist_ctas, cudaStream_t st) {
-    if (!hdesc) hcap = 0;
-    if (launch_chained(k_descriptor<TG>, grid, kDescThreads, 0, st, arena, tab, oriented, oc, desc, cap, hdesc,
-                       hcap, std::max(grid - persist_ctas, 0)) != cudaSuccess)
+                      OctCounters* oc, float* desc, uint32_t cap, const RunCell* cell, int grid, int persist_ctas,
+                      cudaStream_t st) {
+    if (launch_chained(k_descriptor<TG>, grid, kDescThreads, 0, st, arena, tab, oriented, oc, desc, cap, cell,
+                       std::max(grid - persist_ctas, 0)) != cudaSuccess)
         return -1;
     return cudaPeekAtLastError() == cudaSuccess ? 0 : -1;
 }
@@ -918,7 +925,7 @@ int launch_descriptor(const TG* arena, const EntryTable& tab, const Keypoint* or
                                         const uint32_t*,                                                           \
                                         uint32_t, OctCounters*, float*, uint32_t*, int, int, cudaStream_t);        \
     template int launch_descriptor<TG>(const TG*, const EntryTable&, const Keypoint*, OctCounters*,                \
-                                       float*, uint32_t, float*, uint32_t, int, int, cudaStream_t);
+                                       float*, uint32_t, const RunCell*, int, int, cudaStream_t);
 SIFT_INST(float)
 SIFT_INST(__half)
 SIFT_INST(uint8_t)

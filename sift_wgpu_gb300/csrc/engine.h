@@ -56,8 +56,10 @@ int launch_lanczos(const uint8_t* src, int src_pitch, int W, int H, float* tmp, 
 int lanczos_fused_span();
 int lanczos_fused_tile();
 int pixel_channels(int format);
-int launch_export(const Counters* ctr, const Keypoint* kps, Counters* hctr, Keypoint* hkps, uint32_t cap,
-                  cudaStream_t st);
+int launch_begin(const RunCell* hcell, RunCell* cell, Counters* ctr, unsigned long long* scan, size_t n_scan,
+                 cudaStream_t st);
+int launch_fetch(const uint8_t* src, long long stride, uint8_t* img, long long pitch, int W, int H, cudaStream_t st);
+int launch_export(const Counters* ctr, const Keypoint* kps, const RunCell* cell, cudaStream_t st);
 int launch_draw_keypoints(const uint8_t* d_gray, int stride, const Keypoint* d_kps, uint32_t n, uint8_t* d_rgb,
                           int pitch, int W, int H, uint8_t r, uint8_t g, uint8_t b, cudaStream_t st);
 size_t match_scratch_bytes(uint32_t nq, uint32_t nt);
@@ -89,8 +91,8 @@ int launch_orient_emit(const Keypoint* refined_at, uint32_t ncap, int o, Counter
                        cudaStream_t st);
 template <typename TG>
 int launch_descriptor(const TG* arena, const EntryTable& tab, const Keypoint* oriented,
-                      OctCounters* oc, float* desc, uint32_t cap, float* hdesc, uint32_t hcap, int grid,
-                      int persist_ctas, cudaStream_t st);
+                      OctCounters* oc, float* desc, uint32_t cap, const RunCell* cell, int grid, int persist_ctas,
+                      cudaStream_t st);
 // Error reporting (engine.cu): the calling thread's sift_cuda_last_error.
 extern thread_local std::string g_last_error;
 int fail(int code, const std::string& msg);
@@ -252,15 +254,15 @@ struct Engine {
         return (float*)(hx.as<char>() + align_up(sizeof(Counters), 256) + align_up((size_t)cap_x * sizeof(Keypoint), 256));
     }
     size_t img_pitch = 0;
-    // The image cell the base level reads (ImgRef): set by every upload.
-    // Pageable caller images are read where they are when the device reads
-    // pageable host memory coherently (a GB300's Grace host), saving the
-    // staged copy; pinned and device images are copied to d_img (a DMA copy
-    // is faster than the base level's staging reads over the host link).
-    DevMem d_ref;
-    HostPinned h_ref;
+    // The next run's cell (upload and run fill it in), its mapped copy, which
+    // the run's first kernel reads, and its device copy.
+    RunCell cell{};
+    HostPinned h_cell;
+    RunCell* h_cell_dev = nullptr;  // the mapped copy's device address
+    DevMem d_cell;
+    bool unsynced = false;  // a run that may still read the mapped copy has not been waited for
     int pageable_reads = -1;  // device attribute, read once
-    bool image_in_place = false, ref_valid = false;
+    bool image_in_place = false;
     uint32_t launches = 0;
     bool last_desc = true;
 
@@ -288,13 +290,14 @@ struct Engine {
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t gexec = nullptr;
     struct GraphKey {
-        uint32_t W = 0, H = 0, cap_ori = 0, cap_x = 0;  // cap_x 0: no export node
+        uint32_t W = 0, H = 0, cap_ori = 0;
+        bool exp = false;  // ends with the export
         std::vector<uint32_t> cap_c;
         bool with_desc = false;
         Tuning tune{};
         bool operator==(const GraphKey& o) const {
             return W == o.W && H == o.H && cap_ori == o.cap_ori && cap_c == o.cap_c && with_desc == o.with_desc &&
-                   tune == o.tune && cap_x == o.cap_x;
+                   tune == o.tune && exp == o.exp;
         }
     } gkey{};
     uint32_t graph_launches = 0;
@@ -412,6 +415,21 @@ struct Engine {
         }
         CK(h_ctr.ensure(sizeof(Counters)), "cudaHostAlloc(counters)");
         CK(d_ctr.ensure(sizeof(Counters)), "cudaMalloc(counters)");
+        CK(d_cell.ensure(sizeof(RunCell)), "cudaMalloc(run cell)");
+        CK(h_cell.ensure(sizeof(RunCell)), "cudaHostAlloc(run cell)");
+        std::memset(h_cell.p, 0, sizeof(RunCell));
+        CK(cudaHostGetDevicePointer((void**)&h_cell_dev, h_cell.p, 0), "cudaHostGetDevicePointer");
+        return 0;
+    }
+
+    // Publishes the next run's cell. A run in flight may still read the old
+    // one (device-resident runs are asynchronous): it is waited for first.
+    int write_cell() {
+        if (std::memcmp(&cell, h_cell.p, sizeof cell) != 0) {
+            if (unsynced) CK(cudaStreamSynchronize(st), "previous run");
+            std::memcpy(h_cell.p, &cell, sizeof cell);
+        }
+        unsynced = true;
         return 0;
     }
 
@@ -612,8 +630,9 @@ struct Engine {
         };
         std::vector<cudaEvent_t> run_ev;
         mark(&run_ev);
-        CK(cudaMemsetAsync(d_ctr.p, 0, sizeof(Counters), st), "memset counters");
-        CK(cudaMemsetAsync(d_scan.p, 0, scan_words * sizeof(unsigned long long), st), "memset scan state");
+        const RunCell* rc = d_cell.as<RunCell>();
+        if (ok(launch_begin(h_cell_dev, d_cell.as<RunCell>(), ctr, d_scan.as<unsigned long long>(), scan_words, st)))
+            return cuda_fail(cudaGetLastError(), "run start");
         int O_used = 0;
         for (int o = 0; o < O && pyr.oct[o].W > 0 && pyr.oct[o].H > 0; ++o) O_used = o + 1;
 
@@ -710,8 +729,7 @@ struct Engine {
             // host calls: descriptors below cap_x go straight into the mapped
             // export buffer while the stage runs, the rest to d_desc
             if (ok(launch_descriptor<TG>(G, tab(), d_oriented.as<Keypoint>(), &ctr->oct[o], d_desc.as<float>(), cap_ori,
-                                         exp ? hx_ddesc : nullptr, exp ? cap_x : 0u, grid,
-                                         152 * tune.desc_ctas_per_sm, q)))
+                                         exp ? rc : nullptr, grid, 152 * tune.desc_ctas_per_sm, q)))
                 return cuda_fail(cudaGetLastError(), "descriptor");
             return 0;
         };
@@ -723,13 +741,13 @@ struct Engine {
                 int nl = 0;
                 if (launch_blur_level<TG>(img, (int)stride, d_tmp.as<uint8_t>(), G + o0.g_off, U + o0.u_off,
                                           o0.pitch, o0.W, o0.H, base.radius, wts + base.woff, base.tc,
-                                          wts + base.foff, lut, st, &nl, tune.fused_max_radius, d_ref.as<ImgRef>(),
+                                          wts + base.foff, lut, st, &nl, tune.fused_max_radius, &rc->ref,
                                           tune.level_tile_rows))
                     return cuda_fail(cudaGetLastError(), "blur (base)");
                 launches += nl;
             } else {
                 if (ok(launch_u8_to_level<TG>(img, stride, G + o0.g_off, U + o0.u_off, o0.pitch, o0.W, o0.H, st,
-                                              d_ref.as<ImgRef>())))
+                                              &rc->ref)))
                     return cuda_fail(cudaGetLastError(), "base copy");
             }
         }
@@ -792,7 +810,7 @@ struct Engine {
         if (prof) ev_runs.push_back(std::move(run_ev));
         if (exp) {
             // counters and keypoints; the descriptors are there already
-            if (ok(launch_export(ctr, d_oriented.as<Keypoint>(), hx_dctr, hx_dkps, cap_x, st)))
+            if (ok(launch_export(ctr, d_oriented.as<Keypoint>(), rc, st)))
                 return cuda_fail(cudaGetLastError(), "export");
         }
         last_desc = with_desc;
@@ -858,6 +876,11 @@ struct Engine {
     int run(bool with_desc, bool exp = false) {
         const long long stride = (long long)img_pitch;
         desc_on_host = 0;
+        cell.ctr = exp ? hx_dctr : nullptr;
+        cell.kps = exp ? hx_dkps : nullptr;
+        cell.desc = exp ? hx_ddesc : nullptr;
+        cell.cap = exp ? cap_x : 0u;
+        if (int rc = write_cell()) return rc;
         if (prof) return enqueue(d_img.as<uint8_t>(), stride, with_desc, false, exp);
         GraphKey key;
         key.W = W;
@@ -866,7 +889,7 @@ struct Engine {
         key.cap_c = cap_c;
         key.with_desc = with_desc;
         key.tune = tune;
-        key.cap_x = exp ? cap_x : 0;
+        key.exp = exp;
         if (!gexec || !(key == gkey)) {
             drop_graph();
             CK(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal), "begin capture");
@@ -917,42 +940,58 @@ struct Engine {
         return 0;
     }
 
-    int upload(const uint8_t* img, uint32_t w, uint32_t h, uint32_t stride, cudaMemcpyKind kind) {
-        const size_t pitch = align_up(std::max<uint32_t>(w, 1), 128);
-        if (pitch != img_pitch || !d_img.p || d_img.bytes < pitch * std::max<uint32_t>(h, 1)) drop_graph();
-        img_pitch = pitch;
-        CK(d_img.ensure(img_pitch * std::max<uint32_t>(h, 1)), "cudaMalloc(image)");
-        if (!d_ref.p) {
-            CK(d_ref.ensure(sizeof(ImgRef)), "cudaMalloc(image cell)");
-            CK(h_ref.ensure(sizeof(ImgRef)), "cudaHostAlloc(image cell)");
-        }
+    static constexpr size_t kFetchFrom = 1u << 20;
+
+    // The address by which kernels read host memory at p: pinned memory
+    // through its mapping, pageable memory itself on a device that reads it
+    // coherently (a GB300's Grace host); null elsewhere.
+    const uint8_t* device_reads(const uint8_t* p, bool* pageable) {
         if (pageable_reads < 0) {
             int v = 0;
             if (cudaDeviceGetAttribute(&v, cudaDevAttrPageableMemoryAccess, opt.device) != cudaSuccess) v = 0;
             pageable_reads = v == 1 ? 1 : 0;
         }
-        // in place: a pageable host image starting and striding on 16 bytes
-        // (the level kernel's staging loads), a blurred base level
-        bool in_place = false;
-        if (pageable_reads && kind == cudaMemcpyHostToDevice && img && w && h && base.sigma > 0.0f &&
-            ((uintptr_t)img & 15) == 0 && (stride & 15) == 0 && stride <= (1u << 30)) {
-            cudaPointerAttributes a{};
-            if (cudaPointerGetAttributes(&a, img) == cudaSuccess) in_place = a.type == cudaMemoryTypeUnregistered;
-            else cudaGetLastError();
+        cudaPointerAttributes a{};
+        if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+            cudaGetLastError();
+            return nullptr;
         }
-        image_in_place = in_place;
-        const ImgRef cell = in_place ? ImgRef{img, (long long)stride} : ImgRef{d_img.as<uint8_t>(), (long long)img_pitch};
-        if (!in_place && w && h && img)
+        const bool plain = a.type == cudaMemoryTypeUnregistered && pageable_reads == 1;
+        if (pageable) *pageable = plain;
+        if (plain) return p;
+        return a.type == cudaMemoryTypeHost ? static_cast<const uint8_t*>(a.devicePointer) : nullptr;
+    }
+
+    int upload(const uint8_t* img, uint32_t w, uint32_t h, uint32_t stride, cudaMemcpyKind kind) {
+        const size_t pitch = align_up(std::max<uint32_t>(w, 1), 128);
+        if (pitch != img_pitch || !d_img.p || d_img.bytes < pitch * std::max<uint32_t>(h, 1)) drop_graph();
+        img_pitch = pitch;
+        CK(d_img.ensure(img_pitch * std::max<uint32_t>(h, 1)), "cudaMalloc(image)");
+        // How a host image comes in:
+        //  - pageable memory, on a device that reads it coherently: small
+        //    images that start and stride on 16 bytes are read where they are
+        //    by the base level; larger ones, and others, are brought into
+        //    d_img by k_fetch. The base level reads 1.9 bytes over the link
+        //    per pixel (tile halos), k_fetch one, ahead of it: kFetchFrom
+        //    pixels is where they meet;
+        //  - anything else: copied to d_img.
+        const uint8_t* src = nullptr;
+        bool direct = false;
+        image_in_place = false;
+        if (kind == cudaMemcpyHostToDevice && img && w && h && stride <= (1u << 30)) {
+            bool pageable = false;
+            const uint8_t* p = device_reads(img, &pageable);
+            if (pageable) src = p;
+            image_in_place = pageable && ((uintptr_t)img & 15) == 0 && (stride & 15) == 0;
+            direct = image_in_place && base.sigma > 0.0f && (size_t)w * h < kFetchFrom;
+        }
+        if (src && !direct) {
+            if (launch_fetch(src, (long long)stride, d_img.as<uint8_t>(), (long long)img_pitch, (int)w, (int)h, st))
+                return cuda_fail(cudaGetLastError(), "fetch image");
+        } else if (!src && w && h && img) {
             CK(cudaMemcpy2DAsync(d_img.p, img_pitch, img, stride, w, h, kind, st), "copy image");
-        // The cell is rewritten only when it changes: a run that reads it is
-        // ordered after the copy on the stream, and a changed cell comes from
-        // a host call, which has waited for the previous run to end.
-        ImgRef* r = h_ref.as<ImgRef>();
-        if (!ref_valid || r->ptr != cell.ptr || r->pitch != cell.pitch) {
-            *r = cell;
-            CK(cudaMemcpyAsync(d_ref.p, h_ref.p, sizeof(ImgRef), cudaMemcpyHostToDevice, st), "H2D image cell");
-            ref_valid = true;
         }
+        cell.ref = direct ? ImgRef{img, (long long)stride} : ImgRef{d_img.as<uint8_t>(), (long long)img_pitch};
         return 0;
     }
 
@@ -963,14 +1002,22 @@ struct Engine {
         if (format == SIFT_CUDA_PIXELS_GRAY8) {
             if (int rc = upload(img, w, h, stride, cudaMemcpyHostToDevice)) return rc;
         } else {
-            // colour bytes to the device, luma into the image plane
+            // luma into the image plane: of 4-channel pixels straight from
+            // the caller's rows where the device reads them (16-byte loads),
+            // else of a device copy
             const size_t ch = (size_t)pixel_channels(format), row = (size_t)w * ch;
-            const size_t pitch = align_up(std::max<size_t>(row, 1), 128);
-            CK(d_px.ensure(pitch * std::max<uint32_t>(h, 1)), "cudaMalloc(colour image)");
             if (int rc = upload(nullptr, w, h, 0, cudaMemcpyHostToDevice)) return rc;
             if (w && h) {
-                CK(cudaMemcpy2DAsync(d_px.p, pitch, img, stride, row, h, cudaMemcpyHostToDevice, st), "copy pixels");
-                if (launch_to_luma(format, d_px.as<uint8_t>(), (long long)pitch, (int)w, (int)h, d_img.as<uint8_t>(),
+                const uint8_t* px = nullptr;
+                size_t pitch = stride;
+                if (ch == 4 && ((uintptr_t)img & 15) == 0 && (stride & 15) == 0) px = device_reads(img, nullptr);
+                if (!px) {
+                    pitch = align_up(row, 128);
+                    CK(d_px.ensure(pitch * h), "cudaMalloc(colour image)");
+                    CK(cudaMemcpy2DAsync(d_px.p, pitch, img, stride, row, h, cudaMemcpyHostToDevice, st), "copy pixels");
+                    px = d_px.as<uint8_t>();
+                }
+                if (launch_to_luma(format, px, (long long)pitch, (int)w, (int)h, d_img.as<uint8_t>(),
                                    (long long)img_pitch, st))
                     return cuda_fail(cudaGetLastError(), "luma conversion");
             }
@@ -979,6 +1026,7 @@ struct Engine {
         for (int attempt = 0; attempt < 8; ++attempt) {
             if (int rc = run(with_desc, true)) return rc;
             CK(cudaStreamSynchronize(st), "run");
+            unsynced = false;
             const Counters c = *hx_ctr();
             *h_ctr.as<Counters>() = c;
             bool retry = false;

@@ -313,6 +313,7 @@ struct Server {
     // Returns 0 or a status; on 0 the slot is either running again or done.
     int complete(Slot* s) {
         Request* r = s->req;
+        s->eng->unsynced = false;  // its event completed
         const Counters c = *s->eng->hx_ctr();
         bool retry = false;
         if (int rc = s->eng->grow_from(c, &retry)) return rc;

@@ -60,17 +60,30 @@ struct OctaveDev {
     long long t_off;          // byte offset of the entry's horizontal-pass plane (batch runs)
 };
 
-// A batch's pyramid in device memory (u8 storage): the entries of the batch
-// (image-major), the u8 level arena, the horizontal-pass planes, and the
-// input images packed at per-image offsets.
-// Where a host call's image is read from, set before each run: the
-// engine's device copy, or the caller's pageable buffer on a device that
-// reads pageable host memory coherently (the captured graph reads the cell).
+// Where the base level reads its image: the engine's device copy, or the
+// caller's pageable buffer on a device that reads pageable host memory
+// coherently.
 struct ImgRef {
     const uint8_t* ptr;
     long long pitch;
 };
 
+// What changes from run to run of one captured graph: where the image is and
+// where the results go. The host writes it into mapped memory before a run;
+// the run's first kernel (k_begin) copies it to device memory, from where the
+// later kernels read it.
+struct RunCell {
+    ImgRef ref;
+    Counters* ctr;       // mapped result buffer: counters, keypoints, descriptors
+    Keypoint* kps;
+    float* desc;
+    uint32_t cap;        // keypoints that the buffer holds (0: no buffer)
+    uint32_t pad;
+};
+
+// A batch's pyramid in device memory (u8 storage): the entries of the batch
+// (image-major), the u8 level arena, the horizontal-pass planes, and the
+// input images packed at per-image offsets.
 struct BatchPyr {
     uint8_t* U;
     const OctaveDev* ents;
