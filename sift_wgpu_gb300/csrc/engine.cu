@@ -1,4 +1,7 @@
-// engine.cu — error state and the C ABI of the per-image engine (engine.h).
+// engine.cu — error state, lent result buffers and the C ABI of the per-image
+// engine (engine.h).
+#include <unordered_map>
+
 #include "engine.h"
 
 namespace sift {
@@ -23,6 +26,53 @@ int cuda_fail(cudaError_t e, const char* what) {
 // translation unit of the library; returns code.
 int report_error(int code, const char* msg) { return fail(code, msg ? std::string(msg) : std::string()); }
 
+namespace {
+// Lent result buffers by the address of their keypoints, for
+// sift_cuda_result_free. Never destroyed: results may be freed while the
+// process ends.
+struct Lent {
+    std::shared_ptr<ExportBuf> buf;
+    std::shared_ptr<ExportPool> pool;
+};
+struct LentTable {
+    std::mutex mu;
+    std::unordered_map<const void*, Lent> by_kps;
+};
+LentTable& lent_table() {
+    static LentTable* t = new LentTable;
+    return *t;
+}
+}  // namespace
+
+bool lend_result(const std::shared_ptr<ExportBuf>& buf, const std::shared_ptr<ExportPool>& pool) {
+    try {
+        LentTable& t = lent_table();
+        std::lock_guard<std::mutex> g(t.mu);
+        t.by_kps.emplace(buf->kps(), Lent{buf, pool});
+    } catch (const std::bad_alloc&) {
+        return false;
+    }
+    std::lock_guard<std::mutex> g(pool->mu);
+    ++pool->lent;
+    return true;
+}
+
+// Takes a lent buffer back; false if kps is not one's.
+static bool return_result(const void* kps) {
+    Lent l;
+    {
+        LentTable& t = lent_table();
+        std::lock_guard<std::mutex> g(t.mu);
+        auto it = t.by_kps.find(kps);
+        if (it == t.by_kps.end()) return false;
+        l = std::move(it->second);
+        t.by_kps.erase(it);
+    }
+    std::lock_guard<std::mutex> g(l.pool->mu);
+    --l.pool->lent;
+    if (!l.pool->closed && l.pool->idle.size() < ExportPool::kIdle) l.pool->idle.push_back(l.buf);
+    return true;
+}
 
 }  // namespace sift
 
@@ -187,8 +237,10 @@ int sift_cuda_to_luma(const uint8_t* d_pixels, uint32_t width, uint32_t height, 
 
 void sift_cuda_result_free(SiftCudaResult* r) {
     if (!r) return;
-    std::free(r->kps);
-    std::free(r->desc);
+    if (!r->kps || !sift::return_result(r->kps)) {
+        std::free(r->kps);
+        std::free(r->desc);
+    }
     r->kps = nullptr;
     r->desc = nullptr;
     r->n = 0;
@@ -448,7 +500,7 @@ int sift_cuda_debug_stage(SiftCudaEngine* engine, int stage, void* out, uint64_t
             // after a host call the first descriptors are in the export buffer only
             const uint64_t m = std::min<uint64_t>(nd, capacity);
             const uint64_t on_host = std::min<uint64_t>((uint64_t)e.desc_on_host * sift::kDescLen, m);
-            if (on_host) std::memcpy(out, e.hx_desc(), on_host * sizeof(float));
+            if (on_host) std::memcpy(out, e.last->desc(), on_host * sizeof(float));
             if (m > on_host && cudaMemcpy((float*)out + on_host, e.d_desc.as<float>() + on_host,
                                           (m - on_host) * sizeof(float), cudaMemcpyDeviceToHost) != cudaSuccess)
                 return sift::cuda_fail(cudaGetLastError(), "D2H stage");

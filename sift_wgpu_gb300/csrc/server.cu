@@ -314,7 +314,7 @@ struct Server {
     int complete(Slot* s) {
         Request* r = s->req;
         s->eng->unsynced = false;  // its event completed
-        const Counters c = *s->eng->hx_ctr();
+        const Counters c = *s->eng->hx->ctr();
         bool retry = false;
         if (int rc = s->eng->grow_from(c, &retry)) return rc;
         if (retry) {
@@ -613,9 +613,9 @@ int sift_cuda_server_poll(SiftCudaServer* server, SiftCudaServed* out, int64_t t
     out->done_s = r->t_done;
     if (r->status == 0 && r->slot) {
         const sift::Engine& e = *r->slot->eng;
-        out->n = e.hx_ctr()->n_oriented;
-        out->kps = (const SiftCudaKeypoint*)e.hx_kps();
-        out->desc = e.hx_desc();
+        out->n = e.hx->ctr()->n_oriented;
+        out->kps = (const SiftCudaKeypoint*)e.hx->kps();
+        out->desc = e.hx->desc();
     }
     return 1;
 }

@@ -213,9 +213,9 @@ class Engine:
         a = np.asarray(img)
         if a.ndim == 3 and a.dtype == np.uint8 and a.shape[2] in (3, 4):
             return self.detect_and_compute_pixels(a, _capi.PIXELS_RGB8 if a.shape[2] == 3 else _capi.PIXELS_RGBA8)
-        # the drop-in entry: the library copies the results out of the
-        # buffers the GPU wrote (over a few host threads) into arrays that
-        # are returned without another copy
+        # the drop-in entry: the library lends the buffer the GPU wrote (or
+        # copies out of it, while results are held), returned as arrays
+        # without another copy
         return self._call(_capi.lib().sift_cuda_detect_and_compute, img, True)
 
     def detect_and_compute_pixels(self, img, fmt: int) -> tuple[np.ndarray, np.ndarray]:
@@ -233,16 +233,10 @@ class Engine:
         L = _capi.lib()
         _capi.check(L.sift_cuda_detect_and_compute_pixels(self.handle, a.ctypes.data if a.size else None, w, h,
                                                           a.strides[0], fmt, C.byref(res)))
-        try:
-            n = res.n
-            kps = np.empty(n, dtype=KEYPOINT_DTYPE)
-            desc = np.empty((n, DESC_LEN), dtype=np.float32)
-            if n:
-                C.memmove(kps.ctypes.data, res.kps, n * KEYPOINT_DTYPE.itemsize)
-                C.memmove(desc.ctypes.data, res.desc, n * DESC_LEN * 4)
-        finally:
-            L.sift_cuda_result_free(C.byref(res))
-        return kps, desc
+        if res.n:
+            return _owned_result(res, True)
+        L.sift_cuda_result_free(C.byref(res))
+        return np.empty(0, dtype=KEYPOINT_DTYPE), np.empty((0, DESC_LEN), dtype=np.float32)
 
     def detect(self, img) -> np.ndarray:
         return self._call(_capi.lib().sift_cuda_detect, img, False)[0]
