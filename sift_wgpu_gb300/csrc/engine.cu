@@ -293,24 +293,34 @@ int sift_cuda_match(SiftCudaEngine* engine, const float* query, uint32_t n_query
     Engine& e = engine->e;
     if (int rc = e.set_device()) return rc;
     const size_t qb = (size_t)n_query * sift::kDescLen * sizeof(float), tb = (size_t)n_train * sift::kDescLen * sizeof(float);
+    const size_t ob = (size_t)n_query * sizeof(SiftCudaMatch);
     if (e.d_mq.ensure(qb) != cudaSuccess || e.d_mt.ensure(std::max<size_t>(tb, 16)) != cudaSuccess ||
-        e.d_mo.ensure((size_t)n_query * sizeof(SiftCudaMatch)) != cudaSuccess ||
-        e.d_ms.ensure(sift::match_scratch_bytes(n_query, n_train)) != cudaSuccess)
+        e.d_ms.ensure(sift::match_scratch_bytes(n_query, n_train)) != cudaSuccess ||
+        e.h_mo.ensure(ob + 256) != cudaSuccess)
         return sift::cuda_fail(cudaGetLastError(), "cudaMalloc(match)");
     cudaStream_t st = e.st;
-    if (cudaMemcpyAsync(e.d_mq.p, query, qb, cudaMemcpyHostToDevice, st) != cudaSuccess ||
-        (tb && cudaMemcpyAsync(e.d_mt.p, train, tb, cudaMemcpyHostToDevice, st) != cudaSuccess))
+    // Rows that start on 16 bytes in memory the device reads come in with
+    // the norm kernel, others through the copy engine; the results (and the
+    // error word) go to a mapped buffer, so one wait ends the call.
+    auto rows = [&](const float* p) -> const float* {
+        if (!p || ((uintptr_t)p & 15) != 0) return nullptr;
+        bool pageable = false;
+        const uint8_t* d = e.device_reads((const uint8_t*)p, &pageable);
+        return pageable ? (const float*)d : nullptr;
+    };
+    const float *hq = rows(query), *ht = n_train ? rows(train) : nullptr;
+    if ((!hq && cudaMemcpyAsync(e.d_mq.p, query, qb, cudaMemcpyHostToDevice, st) != cudaSuccess) ||
+        (tb && !ht && cudaMemcpyAsync(e.d_mt.p, train, tb, cudaMemcpyHostToDevice, st) != cudaSuccess))
         return sift::cuda_fail(cudaGetLastError(), "H2D descriptors");
-    if (sift::launch_match(e.d_mq.as<float>(), n_query, e.d_mt.as<float>(), n_train, e.d_mo.as<SiftCudaMatch>(),
-                           e.d_ms.p, st))
+    char* mo = nullptr;
+    if (cudaHostGetDevicePointer((void**)&mo, e.h_mo.p, 0) != cudaSuccess)
+        return sift::cuda_fail(cudaGetLastError(), "cudaHostGetDevicePointer");
+    if (sift::launch_match(e.d_mq.as<float>(), n_query, e.d_mt.as<float>(), n_train, (SiftCudaMatch*)(mo + 256), e.d_ms.p,
+                           st, hq, ht, (uint32_t*)mo))
         return sift::cuda_fail(cudaGetLastError(), "match");
-    uint32_t err = 0;
-    if (cudaMemcpyAsync(out, e.d_mo.p, (size_t)n_query * sizeof(SiftCudaMatch), cudaMemcpyDeviceToHost, st) !=
-            cudaSuccess ||
-        cudaMemcpyAsync(&err, sift::match_error_word(e.d_ms.p, n_query, n_train), sizeof(err), cudaMemcpyDeviceToHost,
-                        st) != cudaSuccess ||
-        cudaStreamSynchronize(st) != cudaSuccess)
-        return sift::cuda_fail(cudaGetLastError(), "match results");
+    if (cudaStreamSynchronize(st) != cudaSuccess) return sift::cuda_fail(cudaGetLastError(), "match results");
+    const uint32_t err = *e.h_mo.as<uint32_t>();
+    if (!err) std::memcpy(out, e.h_mo.as<char>() + 256, ob);
     if (err) return sift::fail(SIFT_CUDA_ERR_CUDA, "matching: a tensor-core pipeline wait ran out (no results)");
     return 0;
 }

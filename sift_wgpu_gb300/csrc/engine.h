@@ -64,9 +64,8 @@ int launch_export(const Counters* ctr, const Keypoint* kps, const RunCell* cell,
 int launch_draw_keypoints(const uint8_t* d_gray, int stride, const Keypoint* d_kps, uint32_t n, uint8_t* d_rgb,
                           int pitch, int W, int H, uint8_t r, uint8_t g, uint8_t b, cudaStream_t st);
 size_t match_scratch_bytes(uint32_t nq, uint32_t nt);
-const uint32_t* match_error_word(const void* scratch, uint32_t nq, uint32_t nt);
 int launch_match(const float* d_q, uint32_t nq, const float* d_t, uint32_t nt, SiftCudaMatch* d_out, void* scratch,
-                 cudaStream_t st);
+                 cudaStream_t st, const float* h_q = nullptr, const float* h_t = nullptr, uint32_t* err_out = nullptr);
 int launch_to_luma(int format, const uint8_t* px, long long stride, int W, int H, uint8_t* out, long long out_pitch,
                    cudaStream_t st);
 int launch_extrema_mask(const uint8_t* u8arena, const float* lut255, const EntryTable& tab, const OctaveDev& od,
@@ -279,7 +278,8 @@ struct Engine {
     uint32_t cap_cand = 0, cap_ori = 0;
 
     DevMem d_px;  // colour input before its luma conversion
-    DevMem d_mq, d_mt, d_mo, d_ms;  // descriptor matching: query, train, result, scratch
+    DevMem d_mq, d_mt, d_ms;  // descriptor matching: query, train, scratch
+    HostPinned h_mo;          // its results: error word, matches from byte 256 on
     DevMem d_dg, d_dk, d_drgb;       // drawing: grey input, keypoints, RGB output
     DevMem d_img, d_G, d_U, d_tmp, d_tmpo, d_ltmp, d_wts, d_ltab, d_lw;
     DevMem d_words, d_cand_off, d_keep, d_scan;
