@@ -96,7 +96,7 @@ struct BatchEngine {
     std::vector<std::vector<LevelBlur>> lv;
     size_t lut_off = 0;
 
-    DevMem d_cell, d_img, d_U, d_tmp, d_tmp2, d_ents, d_pref, d_imgaddr, d_imgpitch, d_wts, d_ltab, d_lw, d_lz;
+    DevMem d_bins, d_cell, d_img, d_U, d_tmp, d_tmp2, d_ents, d_pref, d_imgaddr, d_imgpitch, d_wts, d_ltab, d_lw, d_lz;
     // the device reads pageable host memory coherently (Grace's address
     // translation): the base level then reads the caller's images in place
     bool host_reads = false;
@@ -161,6 +161,8 @@ struct BatchEngine {
         CK(cudaEventCreate(&ev_t0), "cudaEventCreate");
         CK(cudaEventCreate(&ev_t1), "cudaEventCreate");
         CK(d_ctr.ensure(sizeof(Counters)), "cudaMalloc(counters)");
+        CK(d_bins.ensure(ori_bins_bytes()), "cudaMalloc(orientation bins)");
+        if (launch_ori_bins(d_bins.as<uint8_t>(), st)) return cuda_fail(cudaGetLastError(), "orientation bins");
         CK(h_ctr.ensure(sizeof(Counters)), "cudaHostAlloc(counters)");
         int pageable = 0;
         if (cudaDeviceGetAttribute(&pageable, cudaDevAttrPageableMemoryAccess, opt.device) != cudaSuccess) pageable = 0;
@@ -457,7 +459,7 @@ struct BatchEngine {
                           "batch refine"))
             return rc;
         const int ogrid = (int)std::max<uint32_t>(cap_cand / 64, 32);
-        if (int rc = bump(launch_orientation<uint8_t>(U, tb, lut, d_refined.as<Keypoint>(), d_keep.as<uint32_t>(),
+        if (int rc = bump(launch_orientation(U, tb, lut, d_bins.as<uint8_t>(), d_refined.as<Keypoint>(), d_keep.as<uint32_t>(),
                                                       cap_cand, oc, d_ori_angle.as<float>(), d_ori_count.as<uint32_t>(),
                                                       ogrid, 152 * 4, st),
                           "batch orientation"))

@@ -6,7 +6,7 @@
 //
 //   k_orientation   one warp per refined keypoint (orient_one): the (2r+1)^2
 //                   window is split over the lanes, each lane takes its samples
-//                   two at a time and adds them into its own column of a
+//                   four at a time and adds them into its own column of a
 //                   bin-major shared histogram (conflict-free, no atomics),
 //                   columns are summed in a fixed order, then the two [1,1,1]/3
 //                   smoothing passes and the peak test run one bin per lane;
@@ -28,8 +28,8 @@
 //
 // The orientation histogram follows the reference's f32 operation order
 // without FMA, except the Gaussian weight (hardware exponential of a
-// reciprocal product) and the angle (polynomial atan2 away from bin edges,
-// atan2f and the IEEE division next to them, so every bin index is exact);
+// reciprocal product); every bin index is exact (a table over the byte
+// differences);
 // its column sums are in a fixed order. The descriptor loop trades exactness
 // for speed within the descriptor tolerance (see describe_one). Orientations
 // and descriptors therefore agree with the reference within rounding, not bit
@@ -95,23 +95,12 @@ template <typename TG>
 struct GaussPlane {
     const TG* base;
     int pitch, W, H;
-    // u8 levels: v / 255 from this table (shared memory) when given, else
-    // by div255; both are the IEEE quotient
-    const float* lut;
-    __device__ __forceinline__ float at(const TG* p) const {
-        if constexpr (std::is_same<TG, uint8_t>::value) {
-            if (lut) return lut[*p];
-        }
-        return gnorm(p);
-    }
     // get_gauss_pixel_value (src/sift.rs:218-223)
     __device__ __forceinline__ float px(int x, int y) const {
         x = clampi(x, 0, W - 1);
         y = clampi(y, 0, H - 1);
-        return at(base + (long long)y * pitch + x);
+        return gnorm(base + (long long)y * pitch + x);
     }
-    // the same for coordinates already inside the level
-    __device__ __forceinline__ float px_in(int x, int y) const { return at(base + y * pitch + x); }
     // get_gauss_pixel_value in v units (graw)
     __device__ __forceinline__ float px_raw(int x, int y) const {
         x = clampi(x, 0, W - 1);
@@ -135,168 +124,216 @@ struct GaussPlane {
 };
 
 template <typename TG>
-__device__ __forceinline__ GaussPlane<TG> plane_for(const TG* arena, const OctaveDev& od, int S, int layer,
-                                                    const float* lut = nullptr) {
+__device__ __forceinline__ GaussPlane<TG> plane_for(const TG* arena, const OctaveDev& od, int S, int layer) {
     const int li = clampi(layer, 0, S + 2);
-    return GaussPlane<TG>{arena + od.g_off + (long long)li * od.plane, od.pitch, od.W, od.H, lut};
+    return GaussPlane<TG>{arena + od.g_off + (long long)li * od.plane, od.pitch, od.W, od.H};
 }
 
 
-// The exact orientation bin position of a gradient angle (src/sift.rs:652-656):
-// atan2 in (-pi, pi] to [0, 2 pi), times 36, divided by 2 pi.
-__device__ __forceinline__ float exact_bin_pos(float ang) {
-    const float two_pi = 2.0f * kPi;
-    const float an = ang < 0.0f ? __fadd_rn(ang, two_pi) : ang;
-    return __fdiv_rn(__fmul_rn(an, (float)kOriBins), two_pi);  // in [0, 36]
+// ---------------------------------------------------------------------------
+// Orientation. Every storage mode keeps the levels as u8 planes, which this
+// stage reads: a gradient is a pair of differences of bytes, and its bin of
+// the 36 (src/sift.rs:652-656) depends on that pair alone. kBinSide^2 bins,
+// one for each pair, are made once (k_ori_bins): off the axes every
+// difference pair's angle is at least 6.4e-5 bins from a bin edge, above the
+// f32 rounding of the reference's sequence (the differences of the two
+// v / 255, atan2f, the wrap and the division: below 2e-5 bins), so the f64
+// angle decides; on the axes the f32 sequence gives the bins 0, 9, 18 and 26
+// (3/2 pi times 36 over 2 pi rounds below 27). A lookup replaces the
+// arctangent polynomial, the edge test and its exact path; with it, the
+// window's integer addressing, four samples in flight per lane, the row
+// prefetch and the smoothing in registers took the octave-0 launch from 50 to
+// 40 us at 1080p (43 -> 24 M warp instructions) and from 380 to 256 us at
+// 4096 x 4096, where it issues 2.4 instructions a cycle and SM, bound by
+// issue and the latency of the byte loads together.
+constexpr int kBinSide = 512;  // differences -256 .. 255
+constexpr int kBinZero = (kBinSide / 2) * kBinSide + kBinSide / 2;
+
+__global__ void __launch_bounds__(kBinSide) k_ori_bins(uint8_t* __restrict__ bins) {
+    chain_wait();
+    const int dx = (int)threadIdx.x - kBinSide / 2, dy = (int)blockIdx.x - kBinSide / 2;
+    int b;
+    if (dy == 0) {
+        b = dx < 0 ? 18 : 0;
+    } else if (dx == 0) {
+        b = dy > 0 ? 9 : 26;
+    } else {
+        const double two_pi = 6.283185307179586476925;
+        const double a = atan2((double)dy, (double)dx);
+        b = (int)((a < 0.0 ? a + two_pi : a) * (double)kOriBins / two_pi);
+    }
+    bins[blockIdx.x * kBinSide + threadIdx.x] = (uint8_t)b;
 }
 
-// Bin positions of the four axis directions. The levels are quantised, so
-// many gradients have gx or gy exactly 0; their angles (0, pi/2, pi, -pi/2)
-// fall exactly on bin edges, where only the exact sequence decides the bin.
-// They are computed once with that sequence instead of per sample.
-struct AxisBins {
-    float right, up, left, down;  // angle 0, pi/2, pi, -pi/2
+// The tables of the orientation stage: v / 255 (shared memory) and the bins.
+struct OriTables {
+    const float* lut;
+    const uint8_t* bins;
 };
-__device__ __forceinline__ AxisBins axis_bins() {
-    return AxisBins{exact_bin_pos(atan2f(0.0f, 1.0f)), exact_bin_pos(atan2f(1.0f, 0.0f)),
-                    exact_bin_pos(atan2f(0.0f, -1.0f)), exact_bin_pos(atan2f(-1.0f, 0.0f))};
-}
 
-// One orientation sample (src/sift.rs:640-662) into the lane's column of the
-// bin-major histogram hist[bin][32]: the gradient (gx, gy) at window offset
-// (fdx, fdy), added as +0.0 when the sample lies outside the level (`in`
-// false), which leaves a bin bit-identical.
-// bf: the polynomial bin position of the gradient (ori_bin_pos2).
-__device__ __forceinline__ void ori_add(float gx, float gy, float fdx, float fdy, float inv_wd, bool in,
-                                        float* hist, int lane, const AxisBins& ab, float bf) {
+// The four neighbours of a sample's pixel, as bytes.
+struct OriBytes {
+    uint32_t right, left, below, above;
+};
+
+// One sample (src/sift.rs:640-662): its bin and its share, the magnitude
+// times the Gaussian weight at window offset (fdx, fdy).
+struct OriSample {
+    uint32_t bin;
+    float v;
+};
+__device__ __forceinline__ OriSample ori_sample(const OriBytes& p, float fdx, float fdy, float inv_wd,
+                                                const OriTables& tb) {
+    OriSample s;
+    s.bin = tb.bins[(p.below - p.above) * (uint32_t)kBinSide + (p.right - p.left) + (uint32_t)kBinZero];
+    const float gx = __fsub_rn(tb.lut[p.right], tb.lut[p.left]), gy = __fsub_rn(tb.lut[p.below], tb.lut[p.above]);
     // the hardware square root (within an ulp; the bins are sums whose
     // order differs from the reference's anyway)
     const float mag = sqrt_approx(__fadd_rn(__fmul_rn(gx, gx), __fmul_rn(gy, gy)));
     // exp(-(dx^2 + dy^2) / wd) with the quotient as a product by 1 / wd and
     // the hardware exponential: a few ulp from expf of the IEEE quotient,
     // the same order as expf's own distance from the host libm
-    const float wgt = __expf(__fmul_rn(-__fadd_rn(__fmul_rn(fdx, fdx), __fmul_rn(fdy, fdy)), inv_wd));
-    // Bin index: from the polynomial atan2 and a multiply by 36 / (2 pi)
-    // (a few ulp from the exact value); axis directions take their exact
-    // position from the table; any other angle within 1e-4 of a bin edge
-    // takes atan2f and the IEEE division, the exact sequence (rare: the
-    // branch no longer splits warps on every flat patch). Away from the
-    // edges all three floor to the same bin.
-    const bool axis = gx == 0.0f || gy == 0.0f;  // (0, 0): atan2 0, angle 0
-    const float bax = gy == 0.0f ? (gx < 0.0f ? ab.left : ab.right) : (gy > 0.0f ? ab.up : ab.down);
-    bf = axis ? bax : bf;
-    if (!axis && fabsf(__fsub_rn(bf, rintf(bf))) < 1e-4f) bf = exact_bin_pos(atan2f(gy, gx));
-    const int fl = floor_i(bf);
-    const int bin = fl >= kOriBins ? fl - kOriBins : fl;
-    const float v = __fmul_rn(mag, wgt);
-    float* h = hist + bin * 32 + lane;
-    *h = __fadd_rn(*h, in ? v : 0.0f);
+    const float ex = __fmul_rn(-__fadd_rn(__fmul_rn(fdx, fdx), __fmul_rn(fdy, fdy)), inv_wd);
+    const float wgt = ex2_approx(__fmul_rn(ex, 1.4426950408889634f));  // in [e^-10, 1]
+    s.v = __fmul_rn(mag, wgt);
+    return s;
 }
 
-// The polynomial bin positions of two gradients: atan2_poly to [0, 2 pi),
-// times 36 / (2 pi) (src/sift.rs:652-656), on f32x2 pairs.
-__device__ __forceinline__ float2 ori_bin_pos2(float2 gy, float2 gx) {
-    const float two_pi = 2.0f * kPi;
-    const float2 pa = atan2_poly2(gy, gx);
-    const float2 pw = __fadd2_rn(pa, make_float2(two_pi, two_pi));
-    const float2 pn = make_float2(pa.x < 0.0f ? pw.x : pa.x, pa.y < 0.0f ? pw.y : pa.y);
-    const float k = (float)kOriBins / two_pi;
-    return __fmul2_rn(pn, make_float2(k, k));
+// Two samples, in this order, into the lane's column of the bin-major
+// histogram hist[bin][32]: both bins are read at once, the first sum is
+// forwarded where they are the same.
+__device__ __forceinline__ void ori_add2(const OriSample& a, const OriSample& b, float* hist_lane) {
+    float* ha = hist_lane + a.bin * 32;
+    float* hb = hist_lane + b.bin * 32;
+    const float va = *ha, vb = *hb;
+    const float na = __fadd_rn(va, a.v);
+    const float nb = __fadd_rn(a.bin == b.bin ? na : vb, b.v);
+    *ha = na;
+    *hb = nb;
 }
 
 // The orientation window of one keypoint (src/sift.rs:640-662), lane-strided:
-// sample k = lane + 32 j of the (2r+1)^2 window, read from the level (the
-// reads mostly hit L1). A lane takes its samples two at a time (k and
-// k + 32: their loads in flight together, the two arctangents on f32x2
-// pairs) and adds them to its histogram column in window order, as one at a
-// time would. Windows at the level's border take the CHECK form.
-template <typename TG, bool CHECK>
-__device__ __forceinline__ void ori_window(const GaussPlane<TG>& g, float xo, float yo, int r, float wd, float* hist,
-                                           int lane, const AxisBins& ab) {
+// sample k = lane + 32 j of the (2r+1)^2 window, row-major, read from the u8
+// level. A lane takes its samples kOriStep at a time (k, k + 32, ..: their
+// loads in flight together) and adds them to its histogram column in window
+// order, as one at a time would; samples past the window or outside the level
+// add +0.0, which leaves a bin bit-identical.
+// PLAIN: the window is inside the level and every position rounds to the
+// keypoint's rounded position plus its offset, so a sample is one offset into
+// the plane; else each position is rounded (f32::round of the f32 sum) and
+// clamped by itself.
+constexpr int kOriStep = 4;
+template <bool PLAIN>
+__device__ __forceinline__ void ori_window(const uint8_t* __restrict__ u8arena, long long level, int pitch, int W, int H,
+                                           float xo, float yo, int r, float wd, float* hist_lane, int lane,
+                                           const OriTables& tb) {
     const float inv_wd = __frcp_rn(wd);
     const int side = 2 * r + 1;
     const float side_f = (float)side, r_f = (float)r;
-    // Sample k = lane + 32 j of the window (row-major) is (fdx, fdy) =
-    // (k % side - r, k / side - r): exact small integers in f32 that advance
-    // by fixed amounts per step, with one row wrap (as selects) at most.
-    const int q0 = lane / side, dq = 32 / side;
-    const float dr_f = (float)(32 - dq * side), dq_f = (float)dq;
-    auto wrap = [&](float& x, float& y) {
-        const bool w = x > r_f;
-        x = w ? x - side_f : x;
-        y = w ? y + 1.0f : y;
-    };
-    // the gradient at a window offset (src/sift.rs:640-651)
-    auto grad = [&](float fdx, float fdy, float& gx, float& gy, bool& in) {
-        int xi = round_away_i(__fadd_rn(xo, fdx));
-        int yi = round_away_i(__fadd_rn(yo, fdy));
-        in = true;
-        if (CHECK) {
-            in = !(xi < 1 || xi >= g.W - 1 || yi < 1 || yi >= g.H - 1);
-            xi = clampi(xi, 1, g.W - 2);
-            yi = clampi(yi, 1, g.H - 2);
+    // Sample k = lane + 32 j is (x, y) = (k % side - r, k / side - r): exact
+    // small integers in f32 that advance by fixed amounts per step, with one
+    // row wrap (as selects) at most; `off` is its byte offset.
+    const float inv_side = rcp_approx(side_f);
+    const int q0 = floor_i(((float)lane + 0.5f) * inv_side), dq = floor_i(32.5f * inv_side), dr = 32 - dq * side;
+    const float dr_f = (float)dr, dq_f = (float)dq;
+    const int doff = dq * pitch + dr, woff = pitch - side;
+    float x = (float)(lane - q0 * side) - r_f, y = (float)q0 - r_f;
+    // (32-bit offsets from the arena, which PLAIN levels lie within)
+    const uint32_t org = (uint32_t)level + (uint32_t)((round_away_i(yo) - r) * pitch + (round_away_i(xo) - r));
+    uint32_t off = org + (uint32_t)(q0 * pitch + lane - q0 * side);
+    while (y <= r_f) {
+        float sx[kOriStep], sy[kOriStep];
+        bool in[kOriStep];
+        OriBytes p[kOriStep];
+#pragma unroll
+        for (int u = 0; u < kOriStep; ++u) {
+            sx[u] = x;
+            sy[u] = y;
+            in[u] = y <= r_f;
+            if (PLAIN) {
+                const uint32_t at = in[u] ? off : org, below = at + (uint32_t)pitch, above = at - (uint32_t)pitch;
+                p[u] = OriBytes{(u8arena + 1)[at], (u8arena - 1)[at], u8arena[below], u8arena[above]};
+            } else {
+                int xi = round_away_i(__fadd_rn(xo, x)), yi = round_away_i(__fadd_rn(yo, y));
+                in[u] = in[u] && !(xi < 1 || xi >= W - 1 || yi < 1 || yi >= H - 1);
+                xi = clampi(xi, 1, W - 2);
+                yi = clampi(yi, 1, H - 2);
+                const uint8_t* at = u8arena + level + (long long)yi * pitch + xi;
+                p[u] = OriBytes{at[1], at[-1], at[pitch], at[-pitch]};
+            }
+            // the next sample
+            x += dr_f;
+            y += dq_f;
+            off += (uint32_t)doff;
+            const bool w = x > r_f;
+            x = w ? x - side_f : x;
+            y = w ? y + 1.0f : y;
+            off = w ? off + (uint32_t)woff : off;
         }
-        gx = __fsub_rn(g.px_in(xi + 1, yi), g.px_in(xi - 1, yi));
-        gy = __fsub_rn(g.px_in(xi, yi + 1), g.px_in(xi, yi - 1));
-    };
-    float fdx = (float)(lane - q0 * side) - r_f, fdy = (float)q0 - r_f;
-    for (;;) {
-        wrap(fdx, fdy);
-        if (fdy > r_f) break;
-        float fdx1 = fdx + dr_f, fdy1 = fdy + dq_f;
-        wrap(fdx1, fdy1);
-        const bool has1 = fdy1 <= r_f;  // else the second reads the first's offset and is not added
-        float gx0, gy0, gx1, gy1;
-        bool in0, in1;
-        grad(fdx, fdy, gx0, gy0, in0);
-        grad(has1 ? fdx1 : fdx, has1 ? fdy1 : fdy, gx1, gy1, in1);
-        const float2 bf = ori_bin_pos2(make_float2(gy0, gy1), make_float2(gx0, gx1));
-        ori_add(gx0, gy0, fdx, fdy, inv_wd, in0, hist, lane, ab, bf.x);
-        if (has1) ori_add(gx1, gy1, fdx1, fdy1, inv_wd, in1, hist, lane, ab, bf.y);
-        fdx = fdx1 + dr_f;
-        fdy = fdy1 + dq_f;
+        OriSample s[kOriStep];
+#pragma unroll
+        for (int u = 0; u < kOriStep; ++u) {
+            s[u] = ori_sample(p[u], sx[u], sy[u], inv_wd, tb);
+            s[u].v = in[u] ? s[u].v : 0.0f;
+        }
+#pragma unroll
+        for (int u = 0; u < kOriStep; u += 2) ori_add2(s[u], s[u + 1], hist_lane);
     }
 }
 
 // The orientation peaks of one refined keypoint (src/sift.rs:605-726),
 // computed by one warp: the window into the warp's bin-major histogram
-// hist[36][32], the column sums and the two smoothing passes in hs[36], the
+// hist[36][32], the column sums and the two smoothing passes in registers, the
 // peaks in bin order written to angles[0 .. count). Returns the count (the
 // same in every lane).
-template <typename TG>
-__device__ __forceinline__ uint32_t orient_one(const TG* __restrict__ arena, const EntryTable& tab, const Keypoint& kp,
-                                               float* hist, float* hs, int lane, const AxisBins& ab,
-                                               float* __restrict__ angles, const float* lut) {
+__device__ __forceinline__ uint32_t orient_one(const uint8_t* __restrict__ u8arena, const EntryTable& tab,
+                                               const Keypoint& kp, float* hist, int lane,
+                                               float* __restrict__ angles, const OriTables& tb) {
     const float two_pi = 2.0f * kPi;
     const float bin_w = 2.0f * kPi / (float)kOriBins;
     const int e = kp.octave;  // entry
     if (!(e >= 0 && e < tab.n)) return 0;
     const OctaveDev od = tab.ents[e];
     const int o = od.octave;
-    const GaussPlane<TG> g = plane_for(arena, od, tab.S, kp.layer, lut);
-    const float scale = __int_as_float((127 + o) << 23);
-    const float xo = __fdiv_rn(kp.x, scale), yo = __fdiv_rn(kp.y, scale);
-    const float so = __fdiv_rn(kp.size, scale);
+    const long long level = od.u_off + (long long)clampi(kp.layer, 0, tab.S + 2) * od.plane;
+    // division by 2^o is the multiplication by 2^-o, exactly
+    const float inv_scale = __int_as_float((127 - o) << 23);
+    const float xo = __fmul_rn(kp.x, inv_scale), yo = __fmul_rn(kp.y, inv_scale);
+    const float so = __fmul_rn(kp.size, inv_scale);
     if (!(so > 0.0f)) return 0;
     const int r = rust_as_i32(roundf(__fmul_rn(4.5f, so)));
     const float ws = __fmul_rn(1.5f, so);
     const float wd = __fmul_rn(__fmul_rn(2.0f, ws), ws);
 #pragma unroll
-    for (int b = 0; b < kOriBins; ++b) hist[b * 32 + lane] = 0.0f;
+    for (int b = 0; b < kOriBins / 4; ++b)
+        reinterpret_cast<float4*>(hist)[b * 32 + lane] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    __syncwarp();
 
     // Windows entirely inside the level (most keypoints) take the loop
     // without bounds checks; the others add +0.0 for samples outside, which
-    // leaves a bin bit-identical.
-    const bool interior = xo - (float)r >= 2.5f && xo + (float)r <= (float)(g.W - 3) - 0.5f &&
-                          yo - (float)r >= 2.5f && yo + (float)r <= (float)(g.H - 3) - 0.5f;
-    if (interior)
-        ori_window<TG, false>(g, xo, yo, r, wd, hist, lane, ab);
+    // leaves a bin bit-identical. The plain loop also wants positions well
+    // off the rounding edge: an f32 sum xo + dx below 2^16 is within 2^-9 of
+    // the exact one, so it rounds to round(xo) + dx.
+    const bool interior = xo - (float)r >= 2.5f && xo + (float)r <= (float)(od.W - 3) - 0.5f &&
+                          yo - (float)r >= 2.5f && yo + (float)r <= (float)(od.H - 3) - 0.5f;
+    const bool plain = interior && level + od.plane < (1ll << 32) && fabsf(xo - floorf(xo) - 0.5f) > 0.0078125f && fabsf(yo - floorf(yo) - 0.5f) > 0.0078125f;
+    if (plain) {
+        // every row's first and last sector on the way before the first is needed
+        const uint8_t* row = u8arena + level + (long long)(round_away_i(yo) - r - 1 + lane) * od.pitch + (round_away_i(xo) - r - 1);
+        for (int q = lane; q < 2 * r + 3; q += 32, row += 32ll * od.pitch) {
+            asm volatile("prefetch.global.L1 [%0];" ::"l"(row));
+            asm volatile("prefetch.global.L1 [%0];" ::"l"(row + 2 * r + 2));
+        }
+    }
+    if (plain)
+        ori_window<true>(u8arena, level, od.pitch, od.W, od.H, xo, yo, r, wd, hist + lane, lane, tb);
     else
-        ori_window<TG, true>(g, xo, yo, r, wd, hist, lane, ab);
+        ori_window<false>(u8arena, level, od.pitch, od.W, od.H, xo, yo, r, wd, hist + lane, lane, tb);
     __syncwarp();
     // Column sums: bin `lane` in four interleaved partial sums (the column
     // index rotated by the bin keeps the 32 lanes in 32 banks), bins 32..35
     // by eight lanes each and a shuffle tree.
+    float h0, h1;
     {
         const float* hb = hist + lane * 32;
         float s0 = 0.0f, s1 = 0.0f, s2 = 0.0f, s3 = 0.0f;
@@ -307,7 +344,7 @@ __device__ __forceinline__ uint32_t orient_one(const TG* __restrict__ arena, con
             s2 = __fadd_rn(s2, hb[(l + 2 + lane) & 31]);
             s3 = __fadd_rn(s3, hb[(l + 3 + lane) & 31]);
         }
-        hs[lane] = __fadd_rn(__fadd_rn(s0, s1), __fadd_rn(s2, s3));
+        h0 = __fadd_rn(__fadd_rn(s0, s1), __fadd_rn(s2, s3));
         const int bb = 32 + (lane >> 3), c0 = (lane & 7) * 4;
         const float* ht = hist + bb * 32;
         float t = __fadd_rn(__fadd_rn(ht[(c0 + bb) & 31], ht[(c0 + 1 + bb) & 31]),
@@ -315,39 +352,48 @@ __device__ __forceinline__ uint32_t orient_one(const TG* __restrict__ arena, con
         t = __fadd_rn(t, __shfl_xor_sync(0xffffffffu, t, 1));
         t = __fadd_rn(t, __shfl_xor_sync(0xffffffffu, t, 2));
         t = __fadd_rn(t, __shfl_xor_sync(0xffffffffu, t, 4));
-        if ((lane & 7) == 0) hs[bb] = t;
+        h1 = __shfl_sync(0xffffffffu, t, 8 * (lane & 3));
     }
-    __syncwarp();
-    for (int it = 0; it < 2; ++it) {
-        float nv0 = 0.0f, nv1 = 0.0f;
-        for (int b = lane, q = 0; b < kOriBins; b += 32, ++q) {
-            const float v = __fdiv_rn(
-                __fadd_rn(__fadd_rn(hs[(b + kOriBins - 1) % kOriBins], hs[b]), hs[(b + 1) % kOriBins]), 3.0f);
-            if (q == 0) nv0 = v; else nv1 = v;
-        }
-        __syncwarp();
-        for (int b = lane, q = 0; b < kOriBins; b += 32, ++q) hs[b] = q == 0 ? nv0 : nv1;
-        __syncwarp();
-    }
-    float mx = fmaxf(hs[lane], lane + 32 < kOriBins ? hs[lane + 32] : 0.0f);
+    // Bin `lane` is h0, bin 32 + lane of lanes 0..3 is h1; the neighbours on
+    // the circle of 36 come by shuffles.
+    float p0, n0, p1, n1;
+    auto neighbours = [&]() {
+        p0 = __shfl_up_sync(0xffffffffu, h0, 1);
+        n0 = __shfl_down_sync(0xffffffffu, h0, 1);
+        p1 = __shfl_up_sync(0xffffffffu, h1, 1);
+        n1 = __shfl_down_sync(0xffffffffu, h1, 1);
+        const float last = __shfl_sync(0xffffffffu, h1, kOriBins - 33), mid = __shfl_sync(0xffffffffu, h1, 0);
+        const float b31 = __shfl_sync(0xffffffffu, h0, 31), b0 = __shfl_sync(0xffffffffu, h0, 0);
+        p0 = lane == 0 ? last : p0;
+        n0 = lane == 31 ? mid : n0;
+        p1 = lane == 0 ? b31 : p1;
+        n1 = lane == kOriBins - 33 ? b0 : n1;
+    };
 #pragma unroll
-    for (int m = 16; m > 0; m >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, m));
+    for (int it = 0; it < 2; ++it) {
+        neighbours();
+        h0 = div3(__fadd_rn(__fadd_rn(p0, h0), n0));
+        h1 = div3(__fadd_rn(__fadd_rn(p1, h1), n1));
+    }
+    neighbours();
+    const bool tail = lane < kOriBins - 32;
+    // the sums are not negative, so their bits order them
+    const float mx = __uint_as_float(
+        __reduce_max_sync(0xffffffffu, max(__float_as_uint(h0), tail ? __float_as_uint(h1) : 0u)));
     const float thr = __fmul_rn(mx, 0.8f);
     bool pk[2] = {false, false};
     float pa[2] = {0.0f, 0.0f};
-    for (int b = lane, q = 0; b < kOriBins; b += 32, ++q) {
-        const float cv = hs[b];
-        if (!(cv >= thr)) continue;
-        const float pv = hs[(b + kOriBins - 1) % kOriBins];
-        const float nv = hs[(b + 1) % kOriBins];
-        if (cv > pv && cv > nv) {
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+        const float cv = q ? h1 : h0, pv = q ? p1 : p0, nv = q ? n1 : n0;
+        pk[q] = (q == 0 || tail) && cv >= thr && cv > pv && cv > nv;
+        if (pk[q]) {
             const float den = __fadd_rn(__fsub_rn(pv, __fmul_rn(2.0f, cv)), nv);
             const float off = fabsf(den) > 1e-5f ? __fdiv_rn(__fmul_rn(0.5f, __fsub_rn(pv, nv)), den) : 0.0f;
-            const float center = __fmul_rn(__fadd_rn((float)b, 0.5f), bin_w);
+            const float center = __fmul_rn(__fadd_rn((float)(lane + 32 * q), 0.5f), bin_w);
             const float a = __fadd_rn(center, __fmul_rn(off, bin_w));
             float fa = rem_euclid_2b(a, two_pi);  // a in (0, 2 pi + pi/36)
             if (fa > kPi) fa = __fsub_rn(fa, two_pi);
-            pk[q] = true;
             pa[q] = fa;
         }
     }
@@ -360,9 +406,9 @@ __device__ __forceinline__ uint32_t orient_one(const TG* __restrict__ arena, con
     return (uint32_t)(__popc(m0) + __popc(m1));
 }
 
-template <typename TG>
-__global__ void __launch_bounds__(32 * kOriWarps, 5) k_orientation(const TG* __restrict__ arena, EntryTable tab,
+__global__ void __launch_bounds__(32 * kOriWarps, 5) k_orientation(const uint8_t* __restrict__ u8arena, EntryTable tab,
                                                                 const float* __restrict__ lut255,
+                                                                const uint8_t* __restrict__ bins,
                                                                 const Keypoint* __restrict__ refined_at,
                                                                 const uint32_t* __restrict__ keep, uint32_t ncap,
                                                                 OctCounters* __restrict__ oc,
@@ -370,31 +416,35 @@ __global__ void __launch_bounds__(32 * kOriWarps, 5) k_orientation(const TG* __r
                                                                 uint32_t* __restrict__ ori_count,
                                                                 int persist_from) {
     chain_wait();
-    __shared__ float hist[kOriWarps][kOriBins][32];
-    __shared__ float hs[kOriWarps][kOriBins];
-    // u8 levels: v / 255 from a shared copy of the table (one load per
-    // pixel instead of a conversion and the three-instruction quotient)
+    __shared__ __align__(16) float hist[kOriWarps][kOriBins][32];
     __shared__ float slut[256];
     const int lane = threadIdx.x, wid = threadIdx.y;
-    constexpr bool kU8 = std::is_same<TG, uint8_t>::value;
-    if (kU8) {
-        for (int v = wid * 32 + lane; v < 256; v += 32 * kOriWarps) slut[v] = lut255[v];
-        __syncthreads();
-    }
+    for (int v = wid * 32 + lane; v < 256; v += 32 * kOriWarps) slut[v] = lut255[v];
+    __syncthreads();
+    const OriTables tb{slut, bins};
     const uint32_t n = min(oc->n_cand, ncap);  // candidate slots; rejected ones get 0 peaks
-    const AxisBins ab = axis_bins();
     const bool persist = (int)blockIdx.x >= persist_from;
-    for (int taken = 0; persist || taken < kOriBudget; ++taken) {
-        uint32_t i = 0;
-        if (lane == 0) i = atomicAdd(&oc->next_ori, 1u);
-        i = __shfl_sync(0xffffffffu, i, 0);
-        if (i >= n) break;
-        i = n - 1 - i;  // from the last slot: the largest windows first
-        uint32_t cnt = 0;
-        if (keep[i])
-            cnt = orient_one<TG>(arena, tab, refined_at[i], &hist[wid][0][0], &hs[wid][0], lane, ab,
-                                 ori_angle + (size_t)i * kOriMaxPeaks, kU8 ? slut : nullptr);
-        if (lane == 0) ori_count[i] = cnt;
+    // A warp claims several slots at once where the list gives every resident
+    // warp at least four such claims (fewer leave warps idle at the end: 1080p
+    // 3 slots a claim 58 us, 1 slot 41 us); it skips the rejected ones (two
+    // in five) without a claim each.
+    const uint32_t claim = min(max(n / (4u * 152u * 5u * kOriWarps), 1u), (uint32_t)kOriBudget);
+    for (uint32_t taken = 0; persist || taken < (uint32_t)kOriBudget; taken += claim) {
+        uint32_t i0 = 0;
+        if (lane == 0) i0 = atomicAdd(&oc->next_ori, claim);
+        i0 = __shfl_sync(0xffffffffu, i0, 0);
+        if (i0 >= n) break;
+        // from the last slot: the largest windows first
+        const uint32_t mine = n - 1 - min(i0 + lane, n - 1);
+        const bool valid = lane < (int)claim && i0 + lane < n;
+        const bool kept = valid && keep[mine] != 0u;
+        if (valid && !kept) ori_count[mine] = 0u;
+        for (uint32_t m = __ballot_sync(0xffffffffu, kept); m; m &= m - 1u) {
+            const uint32_t i = n - 1 - (i0 + (uint32_t)__ffs(m) - 1u);
+            const uint32_t cnt = orient_one(u8arena, tab, refined_at[i], &hist[wid][0][0], lane,
+                                            ori_angle + (size_t)i * kOriMaxPeaks, tb);
+            if (lane == 0) ori_count[i] = cnt;
+        }
     }
 }
 
@@ -891,12 +941,17 @@ __global__ void __launch_bounds__(kDescThreads, 8) k_descriptor(const TG* __rest
 
 }  // namespace
 
-template <typename TG>
-int launch_orientation(const TG* arena, const EntryTable& tab, const float* lut255, const Keypoint* refined_at,
-                       const uint32_t* keep, uint32_t ncap, OctCounters* oc, float* ori_angle, uint32_t* ori_count,
-                       int grid, int persist_ctas, cudaStream_t st) {
-    if (launch_chained(k_orientation<TG>, grid, dim3(32, kOriWarps), 0, st, arena, tab, lut255, refined_at, keep, ncap,
-                       oc, ori_angle, ori_count, std::max(grid - persist_ctas, 0)) != cudaSuccess)
+size_t ori_bins_bytes() { return (size_t)kBinSide * kBinSide; }
+int launch_ori_bins(uint8_t* bins, cudaStream_t st) {
+    if (launch_chained(k_ori_bins, kBinSide, kBinSide, 0, st, bins) != cudaSuccess) return -1;
+    return cudaPeekAtLastError() == cudaSuccess ? 0 : -1;
+}
+
+int launch_orientation(const uint8_t* u8arena, const EntryTable& tab, const float* lut255, const uint8_t* bins,
+                       const Keypoint* refined_at, const uint32_t* keep, uint32_t ncap, OctCounters* oc,
+                       float* ori_angle, uint32_t* ori_count, int grid, int persist_ctas, cudaStream_t st) {
+    if (launch_chained(k_orientation, grid, dim3(32, kOriWarps), 0, st, u8arena, tab, lut255, bins, refined_at, keep,
+                       ncap, oc, ori_angle, ori_count, std::max(grid - persist_ctas, 0)) != cudaSuccess)
         return -1;
     return cudaPeekAtLastError() == cudaSuccess ? 0 : -1;
 }
@@ -921,9 +976,6 @@ int launch_descriptor(const TG* arena, const EntryTable& tab, const Keypoint* or
 }
 
 #define SIFT_INST(TG)                                                                                              \
-    template int launch_orientation<TG>(const TG*, const EntryTable&, const float*, const Keypoint*,               \
-                                        const uint32_t*,                                                           \
-                                        uint32_t, OctCounters*, float*, uint32_t*, int, int, cudaStream_t);        \
     template int launch_descriptor<TG>(const TG*, const EntryTable&, const Keypoint*, OctCounters*,                \
                                        float*, uint32_t, const RunCell*, int, int, cudaStream_t);
 SIFT_INST(float)

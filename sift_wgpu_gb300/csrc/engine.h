@@ -82,10 +82,11 @@ int launch_emit(const uint8_t* u8arena, const float* lut255, const EntryTable& t
 int launch_refine(const uint8_t* u8arena, const float* lut255, const EntryTable& tab, float sigma, float contrast,
                   float edge, const Keypoint* cands, Keypoint* refined_at, uint32_t* keep, uint32_t cap,
                   OctCounters* oc, cudaStream_t st);
-template <typename TG>
-int launch_orientation(const TG* arena, const EntryTable& tab, const float* lut255, const Keypoint* refined_at,
-                       const uint32_t* keep, uint32_t ncap, OctCounters* oc, float* ori_angle, uint32_t* ori_count,
-                       int grid, int persist_ctas, cudaStream_t st);
+size_t ori_bins_bytes();
+int launch_ori_bins(uint8_t* bins, cudaStream_t st);
+int launch_orientation(const uint8_t* u8arena, const EntryTable& tab, const float* lut255, const uint8_t* bins,
+                       const Keypoint* refined_at, const uint32_t* keep, uint32_t ncap, OctCounters* oc,
+                       float* ori_angle, uint32_t* ori_count, int grid, int persist_ctas, cudaStream_t st);
 int launch_orient_emit(const Keypoint* refined_at, uint32_t ncap, int o, Counters* ctr, const float* ori_angle,
                        const uint32_t* ori_count, const uint32_t* ori_off, Keypoint* oriented, uint32_t cap,
                        cudaStream_t st);
@@ -277,6 +278,7 @@ struct Engine {
     size_t scan_words = 0;       // scan state of the run, zeroed at its start
     uint32_t cap_cand = 0, cap_ori = 0;
 
+    DevMem d_bins;  // orientation bins of byte difference pairs
     DevMem d_px;  // colour input before its luma conversion
     DevMem d_mq, d_mt, d_ms;  // descriptor matching: query, train, scratch
     HostPinned h_mo;          // its results: error word, matches from byte 256 on
@@ -465,6 +467,8 @@ struct Engine {
         }
         CK(h_ctr.ensure(sizeof(Counters)), "cudaHostAlloc(counters)");
         CK(d_ctr.ensure(sizeof(Counters)), "cudaMalloc(counters)");
+        CK(d_bins.ensure(ori_bins_bytes()), "cudaMalloc(orientation bins)");
+        if (launch_ori_bins(d_bins.as<uint8_t>(), st)) return cuda_fail(cudaGetLastError(), "orientation bins");
         CK(d_cell.ensure(sizeof(RunCell)), "cudaMalloc(run cell)");
         CK(h_cell.ensure(sizeof(RunCell)), "cudaHostAlloc(run cell)");
         std::memset(h_cell.p, 0, sizeof(RunCell));
@@ -750,7 +754,7 @@ struct Engine {
             // one warp-item per 8 candidate slots, 4 per warp; the last
             // 152 x ori_ctas_per_sm CTAs drain whatever is left
             const int grid = (int)std::max<uint32_t>(cap_c[o] / 64, 32);
-            if (ok(launch_orientation<TG>(G, tab(), lut, d_refined_at.as<Keypoint>() + cb[o], d_keep.as<uint32_t>() + cb[o],
+            if (ok(launch_orientation(U, tab(), lut, d_bins.as<uint8_t>(), d_refined_at.as<Keypoint>() + cb[o], d_keep.as<uint32_t>() + cb[o],
                                           cap_c[o], oc, d_ori_angle.as<float>() + (size_t)cb[o] * kOriMaxPeaks,
                                           d_ori_count.as<uint32_t>() + cb[o], grid, 152 * tune.ori_ctas_per_sm, q)))
                 return cuda_fail(cudaGetLastError(), "orientation");

@@ -166,6 +166,14 @@ __device__ __forceinline__ float div255(float v) {
     return __fmaf_rn(__fmaf_rn(-q, 255.0f, v), kInv255, q);
 }
 
+// v / 3 correctly rounded, by the same scheme (fl(1/3) is the correctly
+// rounded reciprocal), for v of 0 or far from the ends of the exponent range.
+__device__ __forceinline__ float div3(float v) {
+    constexpr float third = 0.3333333432674408f;  // fl(1/3)
+    const float q = __fmul_rn(v, third);
+    return __fmaf_rn(__fmaf_rn(-q, 3.0f, v), third, q);
+}
+
 // imageproc's Clamp<f32> for u8 on the truncation path, as a float:
 // min(max(trunc(a), 0), 255) (trunc of a negative a is <= 0).
 __device__ __forceinline__ float clamp_u8f(float a) { return fminf(fmaxf(trunc_pos(a), 0.0f), 255.0f); }
@@ -209,9 +217,9 @@ __device__ __forceinline__ float rem_euclid_2b(float a, float b) {
 // atan(a) = a * P(a^2) with P of degree 7, minimax in relative error on
 // [0, 1] (Lawson's reweighted least squares; tests/golden/fit_atan2.py makes
 // the coefficients; 2.5e-7 relative error evaluated in f32), then the octant
-// fix-ups: within 4 ulp of atan2f (tests/test_atan2_gpu.py). atan2(0, 0) = 0. Used where the
-// angle is interpolated linearly (descriptor bins), and by the orientation
-// histogram, whose bins are a hard floor, only away from the bin edges.
+// fix-ups: within 4 ulp of atan2f (tests/test_atan2_gpu.py). atan2(0, 0) = 0. No kernel of the run
+// uses it any more (the orientation's bins come from a table, the descriptor
+// wants atan2_bins); the accuracy tests measure it.
 __device__ __forceinline__ float atan2_poly(float y, float x) {
     const float ax = fabsf(x), ay = fabsf(y);
     const float mx = fmaxf(ax, ay), mn = fminf(ax, ay);
