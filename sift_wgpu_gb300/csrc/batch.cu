@@ -473,7 +473,7 @@ struct BatchEngine {
                           "batch orientation emit"))
             return rc;
         const int dgrid = (int)std::max<uint32_t>(cap_cand / 16, 64);
-        if (int rc = bump(launch_descriptor<uint8_t>(U, tb, d_oriented.as<Keypoint>(), oc, d_desc.as<float>(),
+        if (int rc = bump(launch_descriptor(U, tb, d_oriented.as<Keypoint>(), oc, d_desc.as<float>(),
                                                      cap_ori, d_cell.as<RunCell>(), dgrid, 152 * 8, st),
                           "batch descriptor"))
             return rc;

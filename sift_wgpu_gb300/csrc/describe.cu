@@ -53,60 +53,20 @@ constexpr int kOriWarps = 8;  // orientation: one keypoint per warp
 constexpr int kOriBudget = 4;   // keypoints per warp
 constexpr int kDescBudget = 2;  // keypoints per CTA
 
-// A Gaussian level pixel as v/255 (get_gauss_pixel_value, src/sift.rs:218-223):
-// f32 levels store it directly, f16 and u8 levels store v, divided here
-// (div255 is the IEEE quotient for every u8 value), so every storage mode
-// reads the same values.
-template <typename T>
-__device__ __forceinline__ float gnorm(const T* p);
-template <>
-__device__ __forceinline__ float gnorm<float>(const float* p) {
-    return *p;
-}
-template <>
-__device__ __forceinline__ float gnorm<__half>(const __half* p) {
-    return div255(__half2float(*p));
-}
-template <>
-__device__ __forceinline__ float gnorm<uint8_t>(const uint8_t* p) {
-    return div255(float_of_u8(*p));
-}
-
-// The same pixel as v itself (0..255): f32 levels give it back exactly as
-// fl(fl(v / 255) * 255) (true for every u8 value), f16 and u8 levels store it.
-// The descriptor works in these units: its histogram is L2-normalised, so the
-// factor 255 cancels, and the three storage modes give the same values.
-template <typename T>
-__device__ __forceinline__ float graw(const T* p);
-template <>
-__device__ __forceinline__ float graw<float>(const float* p) {
-    return __fmul_rn(*p, 255.0f);
-}
-template <>
-__device__ __forceinline__ float graw<__half>(const __half* p) {
-    return __half2float(*p);
-}
-template <>
-__device__ __forceinline__ float graw<uint8_t>(const uint8_t* p) {
-    return float_of_u8(*p);
-}
-
-template <typename TG>
+// One level of the u8 arena. Every storage mode keeps it, and both stages here
+// read it whatever else is stored: it is the smallest and the fastest to read,
+// and v / 255 (div255, the IEEE quotient) is the f32 mode's stored value.
 struct GaussPlane {
-    const TG* base;
+    const uint8_t* base;
     int pitch, W, H;
     // get_gauss_pixel_value (src/sift.rs:218-223)
-    __device__ __forceinline__ float px(int x, int y) const {
-        x = clampi(x, 0, W - 1);
-        y = clampi(y, 0, H - 1);
-        return gnorm(base + (long long)y * pitch + x);
+    __device__ __forceinline__ uint32_t at(int x, int y) const {
+        return base[(long long)clampi(y, 0, H - 1) * pitch + clampi(x, 0, W - 1)];
     }
-    // get_gauss_pixel_value in v units (graw)
-    __device__ __forceinline__ float px_raw(int x, int y) const {
-        x = clampi(x, 0, W - 1);
-        y = clampi(y, 0, H - 1);
-        return graw(base + (long long)y * pitch + x);
-    }
+    __device__ __forceinline__ float px(int x, int y) const { return div255((float)at(x, y)); }
+    // the same as v itself (0..255): the descriptor's histogram is
+    // L2-normalised, so the factor 255 cancels
+    __device__ __forceinline__ float px_raw(int x, int y) const { return (float)at(x, y); }
     // get_gauss_pixel_bilinear (src/sift.rs:238-266)
     __device__ __forceinline__ float bilinear(float x, float y) const {
         const float xf = floorf(x), yf = floorf(y);
@@ -123,12 +83,9 @@ struct GaussPlane {
     }
 };
 
-template <typename TG>
-__device__ __forceinline__ GaussPlane<TG> plane_for(const TG* arena, const OctaveDev& od, int S, int layer) {
-    const int li = clampi(layer, 0, S + 2);
-    return GaussPlane<TG>{arena + od.g_off + (long long)li * od.plane, od.pitch, od.W, od.H};
+__device__ __forceinline__ GaussPlane plane_for(const uint8_t* u8arena, const OctaveDev& od, int S, int layer) {
+    return GaussPlane{u8arena + od.u_off + (long long)clampi(layer, 0, S + 2) * od.plane, od.pitch, od.W, od.H};
 }
-
 
 // ---------------------------------------------------------------------------
 // Orientation. Every storage mode keeps the levels as u8 planes, which this
@@ -481,13 +438,101 @@ __global__ void k_orient_emit(const Keypoint* __restrict__ refined_at, uint32_t 
 
 constexpr int kDescThreads = 128;
 static_assert(kDescThreads == kDescLen && kDescThreads == 128, "one descriptor bin per thread, four warps");
-constexpr int kHistRow = 9;      // 8 angle bins + slot 8, the share of bin 0 that wrapped from bin 7
-constexpr int kHistSide = 6;     // cells -1..4 per axis: the 4 x 4 window and a border that takes the
-                                 // trilinear spill, so no sample needs a clamp or a validity test
-constexpr int kHistCopies = 8;   // lane & 7 picks the copy
-constexpr int kHistStride = 324; // 36 * kHistRow; 324 % 32 = 4 puts a bin's 8 copies in 8 banks
+// The histogram: 8 angle bins and a 9th (the share of bin 0 that wrapped from
+// bin 7) of cells -1..4 per axis (the 4 x 4 window and a border that takes the
+// trilinear spill, so no sample needs a clamp or a validity test), in 8 copies.
+// A row of cells is 5 apart from the next: cell 4 of one and cell -1 of the
+// next, whose sums nobody reads, are the same.
+// Word (bin, cell, copy) = bin * kHistBin + cell * 8 + copy: a bin's word lies
+// in a bank of its cell and copy alone, so that the lanes of a warp, most of
+// them in a few cells but in any bin, collide only by cell; the bank of a
+// layout with the bins innermost also depends on each lane's bin.
+constexpr int kHistSide = 5;
+constexpr int kHistCopies = 8;
+constexpr int kHistBin = 32 * kHistCopies;  // cells -1 .. 4 by -1 .. 4: 31, and one unused
+constexpr int kHistWords = 9 * kHistBin;
+static_assert(5 * kHistSide + 6 <= 32 && kHistBin % 32 == 0, "a word's bank is its cell's and copy's");
 constexpr int kDescRadGrid = 31;                      // largest radius served from the grid
 constexpr int kDescGridSide = 2 * kDescRadGrid + 3;   // offsets -(rad+1) .. rad+1
+
+// A row of the window and its sample pairs that can be inside the rotated
+// square, as a warp enumerates them: pair m of the warp, if it lies in this
+// row, is at window offset (px + 2 m, py), grid index c + 2 m; k holds the
+// parity of the grid row (times 2) and 16 times the histogram copy of m = 0.
+// The copy is (i + q) & 7 of pair i of row q: neighbours in a row and pairs
+// above each other, which mostly share cells, use different copies (2.35
+// wavefronts per atomic by a CPU model of the bank conflicts; by i & 7, 2.6;
+// with rows of cells 6 apart 2.5 and 2.8; a layout with the bins innermost
+// by lane & 7, 3.2).
+struct __align__(16) PairRow {
+    float px, py;
+    int c, k;
+};
+constexpr int kWarpRows = 16;                                  // a warp takes the rows q with q % 4 = warp
+constexpr int kWarpWords = kWarpRows * (kDescRadGrid + 1) / 32;  // a bit for each of its pairs
+struct WarpPairs {
+    PairRow row[kWarpRows];      // the rows that have pairs
+    uint32_t start[kWarpWords];  // the pairs that start a row
+};
+static_assert(kWarpRows * 4 >= 2 * kDescRadGrid + 1, "every row has a warp");
+
+// Fills in the warp's rows; returns the count of its pairs. (Row q, py = q -
+// rad, has pairs at px = 2 i - rad - p, i = 0 .. rad, p the parity of its grid
+// row q + 1.) The two strips |ca px + sa py| < lim and |ca py - sa px| < lim
+// cut an interval out of each row; near-zero ca, sa are widened to 1e-4, which
+// with the margins (0.01 on lim, a quarter pixel on x) only adds pairs. A
+// third of the window's pairs are outside; whether a sample is inside is
+// decided by itself.
+__device__ __forceinline__ int warp_pairs(WarpPairs* w, float ca, float sa, float lim, int rad, int gst, int warp,
+                                          int lane) {
+    const float ic = rcp_approx(copysignf(fmaxf(fabsf(ca), 1e-4f), ca)), is = rcp_approx(copysignf(fmaxf(fabsf(sa), 1e-4f), sa));
+    const float hx = (lim + 0.01f) * fabsf(ic), hy = (lim + 0.01f) * fabsf(is);
+    const float rad_f = (float)rad;
+    if (lane < kWarpWords) w->start[lane] = 0u;
+    // lane l: row 4 (l % 16) + warp (the lanes above 15 repeat them)
+    const int q = 4 * (lane & (kWarpRows - 1)) + warp, p = (q + 1) & 1;
+    const float py = (float)q - rad_f, shift = rad_f + (float)p, end = rad_f + 1.0f;
+    // both within [-rad - 1, rad + 1]
+    const float lo = fminf(fmaxf(fmaxf(-sa * ic * py - hx, ca * is * py - hy) - 0.25f, -end), end);
+    const float hi = fmaxf(fminf(fminf(-sa * ic * py + hx, ca * is * py + hy) + 0.25f, end), -end);
+    // px + 1 >= lo and px <= hi
+    const int first = max(-floor_i(-0.5f * (lo + shift - 1.0f)), 0);
+    const int last = min(floor_i(0.5f * (hi + shift)), rad);
+    const int count = q < 2 * rad + 1 ? max(last - first + 1, 0) : 0;
+    int at = count;
+#pragma unroll
+    for (int d = 1; d < kWarpRows; d <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, at, d, kWarpRows);
+        if ((lane & (kWarpRows - 1)) >= d) at += y;
+    }
+    const int total = __shfl_sync(0xffffffffu, at, kWarpRows - 1);
+    const bool some = count > 0 && lane < kWarpRows;
+    const uint32_t rows = __ballot_sync(0xffffffffu, some);
+    if (some) {
+        at -= count;  // the row's first pair
+        const int i0 = first - at;
+        w->row[__popc(rows & ((1u << lane) - 1u))] =
+            PairRow{(float)(2 * i0) - shift, py, (q + 1) * gst + 2 * i0 + 1, 16 * (i0 + q) + 2 * p};
+        atomicOr(&w->start[at >> 5], 1u << (at & 31));
+    }
+    __syncwarp();
+    return total;
+}
+
+// The eight shares of a sample, added to the histogram word by word: four
+// cells (the next in x, in y, in both; byte distances kX, kY), two bins (kA)
+// each.
+template <int kA, int kX, int kY>
+__device__ __forceinline__ void add_shares(uint32_t at, const uint32_t (&v)[8]) {
+    asm volatile(
+        "red.shared.add.u32 [%0], %1;\n red.shared.add.u32 [%0 + %15], %2;\n"
+        "red.shared.add.u32 [%0 + %9], %3;\n red.shared.add.u32 [%0 + %10], %4;\n"
+        "red.shared.add.u32 [%0 + %11], %5;\n red.shared.add.u32 [%0 + %12], %6;\n"
+        "red.shared.add.u32 [%0 + %13], %7;\n red.shared.add.u32 [%0 + %14], %8;" ::"r"(at),
+        "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "n"(kX), "n"(kX + kA),
+        "n"(kY), "n"(kY + kA), "n"(kX + kY), "n"(kX + kY + kA), "n"(kA)
+        : "memory");
+}
 
 // The descriptor of one oriented keypoint (src/sift.rs:917-1060 and
 // normalize_and_clip_descriptor, src/sift.rs:889-913), computed by the whole
@@ -496,22 +541,24 @@ constexpr int kDescGridSide = 2 * kDescRadGrid + 3;   // offsets -(rad+1) .. rad
 //     integer offsets i, j in [-(rad+1), rad+1], go to a shared grid once
 //     (the reference re-evaluates four bilinears per window sample).
 //  2. Each thread takes pairs of neighbouring window samples and evaluates
-//     both at once with Blackwell's packed f32x2 multiply/add/FMA (the kernel
-//     is bound by instruction issue); the eight trilinear contributions of
+//     both at once with Blackwell's packed f32x2 multiply/add/FMA; the eight
+//     trilinear contributions of
 //     each are added to 128 shared bins as u32 fixed point (2^-f units, f
 //     chosen so no bin can overflow): integer addition is associative, so the
 //     descriptor is the same on every run.
 //  3. The four warps normalise, clip at 0.2, renormalise.
 // Radii above the grid (not reachable with the default sigma) fall back to
 // per-sample bilinears from the level itself.
-template <typename TG, class Dst>
-__device__ __forceinline__ void describe_one(const TG* __restrict__ arena, const EntryTable& tab, const Keypoint& kp,
-                                             float* grid, unsigned int* hist, float* red_lo, float* red_hi,
+template <class Dst>
+__device__ __forceinline__ void describe_one(const uint8_t* __restrict__ u8arena, const EntryTable& tab,
+                                             const Keypoint& kp,
+                                             float* grid, unsigned int* hist, WarpPairs* pairs_of, float* red_lo,
+                                             float* red_hi,
                                              const Dst& dst) {
     const int tid = threadIdx.x;
     const float sqrt2 = __fsqrt_rn(2.0f);
     const int e = kp.octave;  // entry
-    for (int w = tid; w < kHistCopies * kHistStride / 4; w += kDescThreads)
+    for (int w = tid; w < kHistWords / 4; w += kDescThreads)
         reinterpret_cast<uint4*>(hist)[w] = make_uint4(0u, 0u, 0u, 0u);
     const bool valid_oct = e >= 0 && e < tab.n;
     OctaveDev od{};
@@ -523,7 +570,7 @@ __device__ __forceinline__ void describe_one(const TG* __restrict__ arena, const
     const bool valid = valid_oct && so > 0.0f;
     float inv_fix = 0.0f;
     if (valid) {
-        const GaussPlane<TG> g = plane_for(arena, od, tab.S, kp.layer);
+        const GaussPlane g = plane_for(u8arena, od, tab.S, kp.layer);
         const float xo = __fmul_rn(kp.x, inv_scale), yo = __fmul_rn(kp.y, inv_scale);
         const float ang = kp.angle;
         // the hardware sine and cosine (|ang| <= pi; absolute error ~4e-7,
@@ -546,13 +593,19 @@ __device__ __forceinline__ void describe_one(const TG* __restrict__ arena, const
         // phase (the pairs of odd rows start one sample to the left), all
         // four float pairs a pair of samples reads are 8-byte aligned.
         const int gst = gs + 1;
+        // |rx|, |ry| below lim keep xb, yb inside (-1, 4) after rounding, so
+        // every cell index lies in the padded grid (samples within 1e-6
+        // of the window edge, whose shares there are ~0, are left out)
+        const float lim = __fmul_rn(2.5f, bw) * 0.99999905f;
+        int n_pairs = 0;
         float lo = 3.0e38f, hi = 0.0f;
         if (use_grid) {
+            n_pairs = warp_pairs(pairs_of + (tid >> 5), ca, sa, lim, rad, gst, tid >> 5, tid & 31);
             // the spare slots, read only for the phantom element of a
             // row's end pair, hold 0
             if (tid < gs) grid[tid * gst + ((tid & 1) ? 0 : gs)] = 0.0f;
             // Bilinear samples at the window's integer offsets, in v units
-            // (graw), straight from the level (the patch stays in L1). All
+            // (px_raw), straight from the level (the patch stays in L1). All
             // of them share the
             // fraction of (xo, yo): the reference's sample positions xo + i
             // differ from it only by the rounding of that sum. Clamped
@@ -563,54 +616,70 @@ __device__ __forceinline__ void describe_one(const TG* __restrict__ arena, const
             const bool inner = px0 >= 0 && py0 >= 0 && px0 + gs < g.W && py0 + gs < g.H;
             const float inv_gs = 1.0f / (float)gs;
             if (inner) {
-                // A thread makes a strip of 4 x 2 grid points from 5 x 3
-                // pixels: each row's horizontal lerps serve the points
-                // above and below it, both columns at once on f32x2
-                // pairs (15 loads for 8 points); consecutive lanes take
-                // consecutive column pairs. The same two lerps per point
-                // as below, so the same values.
-                const int strips = (gs + 3) >> 2, cps = (gs + 1) >> 1;
-                const float inv_cps = 1.0f / (float)cps;
-                const TG* org = g.base + py0 * g.pitch + px0;
+                // A thread makes a block of 4 x 4 grid points from 5 rows of
+                // 5 pixels, two aligned words a row (the shift is the same
+                // for every block; the second word may end past the row, in
+                // its padding or the next, never past the arena): each
+                // row's horizontal lerps serve the points above and below
+                // it, two columns at once on f32x2 pairs. The same two
+                // lerps per point as below, so the same values.
+                const int blocks = (gs + 3) >> 2;
+                const float inv_blocks = 1.0f / (float)blocks;
+                const int pitch4 = g.pitch >> 2, shift = 8 * (px0 & 3);
+                const uint32_t* org = reinterpret_cast<const uint32_t*>(g.base + (long long)py0 * g.pitch + (px0 & ~3));
                 const float2 fdx2 = make_float2(fdx, fdx), fdy2 = make_float2(fdy, fdy);
                 const float2 neg1 = make_float2(-1.0f, -1.0f);
                 float tf = (float)tid;
-                for (int t = tid; t < strips * cps; t += kDescThreads, tf += (float)kDescThreads) {
-                    const int sy = floor_i((tf + 0.5f) * inv_cps);
-                    const int qx = 2 * (t - sy * cps), qy0 = 4 * sy;
-                    const int nr = min(4, gs - qy0);
-                    // an odd-width grid's last pair has a phantom second
-                    // column: its third pixel repeats the second (in
-                    // bounds) and nothing is stored for it
-                    const bool two = qx + 1 < gs;
-                    const int o2 = two ? 2 : 1;
-                    // all 15 loads first (rows past the strip's last
-                    // repeat it), then the lerps
-                    const TG* pp = org + qy0 * g.pitch + qx;
-                    float a[5][3];
+                for (int t = tid; t < blocks * blocks; t += kDescThreads, tf += (float)kDescThreads) {
+                    const int by = floor_i((tf + 0.5f) * inv_blocks), bx = t - by * blocks;
+                    const int nr = min(4, gs - 4 * by), nc = min(4, gs - 4 * bx);
+                    // all words first (rows past the block's last repeat it)
+                    const uint32_t* pp = org + 4 * by * pitch4 + bx;
+                    uint32_t w[5][2];
 #pragma unroll
                     for (int j = 0; j < 5; ++j) {
-                        const TG* pr = pp + min(j, nr) * g.pitch;
-                        a[j][0] = graw(pr);
-                        a[j][1] = graw(pr + 1);
-                        a[j][2] = graw(pr + o2);
+                        const uint32_t* pr = pp + min(j, nr) * pitch4;
+                        w[j][0] = pr[0];
+                        w[j][1] = pr[1];
                     }
-                    float2 A = make_float2(a[0][0], a[0][1]);
-                    float2 rp = __ffma2_rn(fdx2, __ffma2_rn(A, neg1, make_float2(a[0][1], a[0][2])), A);
-                    float* gp = grid + qy0 * gst + qx;  // qy0 even
+                    float* gp = grid + 4 * by * gst + 4 * bx;  // (gst is even: pairs of even rows are aligned)
+                    float2 up0, up1;
 #pragma unroll
-                    for (int j = 0; j < 4; ++j) {
-                        A = make_float2(a[j + 1][0], a[j + 1][1]);
-                        const float2 rn =
-                            __ffma2_rn(fdx2, __ffma2_rn(A, neg1, make_float2(a[j + 1][1], a[j + 1][2])), A);
-                        const float2 b = __ffma2_rn(fdy2, __ffma2_rn(rp, neg1, rn), rp);
-                        if (j < nr) {
-                            gp[j * gst + (j & 1)] = b.x;
-                            if (two) gp[j * gst + (j & 1) + 1] = b.y;
-                            lo = fminf(lo, fminf(b.x, b.y));
-                            hi = fmaxf(hi, fmaxf(b.x, b.y));
+                    for (int j = 0; j < 5; ++j) {
+                        const uint32_t b4 = __funnelshift_r(w[j][0], w[j][1], shift);
+                        const float a0 = float_of_byte<0>(b4), a1 = float_of_byte<1>(b4), a2 = float_of_byte<2>(b4),
+                                    a3 = float_of_byte<3>(b4), a4 = float_of_byte<0>(w[j][1] >> shift);
+                        const float2 l0 = make_float2(a0, a1), l1 = make_float2(a2, a3);
+                        const float2 r0 = __ffma2_rn(fdx2, __ffma2_rn(l0, neg1, make_float2(a1, a2)), l0);
+                        const float2 r1 = __ffma2_rn(fdx2, __ffma2_rn(l1, neg1, make_float2(a3, a4)), l1);
+                        if (j > 0 && j <= nr) {
+                            const float2 b0 = __ffma2_rn(fdy2, __ffma2_rn(up0, neg1, r0), up0);
+                            const float2 b1 = __ffma2_rn(fdy2, __ffma2_rn(up1, neg1, r1), up1);
+                            float* d = gp + (j - 1) * gst + ((j - 1) & 1);
+                            if (nc == 4) {
+                                if ((j - 1) & 1) {  // (odd rows sit one slot on: their middle pair is aligned)
+                                    d[0] = b0.x;
+                                    *reinterpret_cast<float2*>(d + 1) = make_float2(b0.y, b1.x);
+                                    d[3] = b1.y;
+                                } else {
+                                    *reinterpret_cast<float2*>(d) = b0;
+                                    *reinterpret_cast<float2*>(d + 2) = b1;
+                                }
+                                lo = fminf(lo, fminf(fminf(b0.x, b0.y), fminf(b1.x, b1.y)));
+                                hi = fmaxf(hi, fmaxf(fmaxf(b0.x, b0.y), fmaxf(b1.x, b1.y)));
+                            } else {
+                                const float v[3] = {b0.x, b0.y, b1.x};
+#pragma unroll
+                                for (int k = 0; k < 3; ++k)
+                                    if (k < nc) {
+                                        d[k] = v[k];
+                                        lo = fminf(lo, v[k]);
+                                        hi = fmaxf(hi, v[k]);
+                                    }
+                            }
                         }
-                        rp = rn;
+                        up0 = r0;
+                        up1 = r1;
                     }
                 }
             } else {
@@ -671,11 +740,7 @@ __device__ __forceinline__ void describe_one(const TG* __restrict__ arena, const
         const float inv_bw = 1.0f / bw;
         const float angb = ang * (4.0f / kPi);  // keypoint angle in 45-degree bins
         const float wexp = -1.4426950408889634f / wd;  // exp(-d2/wd) = exp2(d2 * wexp)
-        // |rx|, |ry| below lim keep xb, yb inside (-1, 4) after rounding, so
-        // every cell index lies in the padded grid (samples within 1e-6
-        // of the window edge, whose shares there are ~0, are left out)
-        const float lim = __fmul_rn(2.5f, bw) * 0.99999905f;
-        unsigned int* hcopy = hist + (tid & 7) * kHistStride;
+        const uint32_t hist_at = (uint32_t)__cvta_generic_to_shared(hist);
         const float rad_f = (float)rad;
         // windows that stay inside the level need no per-sample border test
         const bool edge = !(__fadd_rn(xo, -rad_f) >= 0.0f && __fadd_rn(xo, rad_f) < wm1 &&
@@ -689,16 +754,8 @@ __device__ __forceinline__ void describe_one(const TG* __restrict__ arena, const
             // window), from px = -rad - 1 in rows of odd grid index (the
             // first pair's first element is outside), so the float pairs
             // of the gradients' grid reads are 8-byte aligned (one 64-bit
-            // load each). Pair m = tid + 128 j: the base offset pxb (= px
-            // in even rows, px + 1 in odd ones), py (exact small integers
-            // in f32), the row parity p and the grid index c of element 0
-            // advance by fixed amounts with one row wrap per step.
-            const int hp = rad + 1;
-            const int q0 = tid / hp, dq = kDescThreads / hp;
-            const float dr_f = (float)(2 * (kDescThreads - dq * hp)), dq_f = (float)dq;
-            const int dc = dq * gst + 2 * (kDescThreads - dq * hp);
-            const int dqp = dq & 1;
-            const float wrap_f = (float)(2 * hp);
+            // load each). A warp enumerates the pairs of its rows that can be
+            // inside the rotated square (warp_pairs).
             // Fixed point on the subnormal grid: a float below 2^-125 is
             // k * 2^-149 and its bit pattern is k, so a contribution scaled
             // by 2^(fbits - 149) and rounded once to the nearest float (the
@@ -718,24 +775,21 @@ __device__ __forceinline__ void describe_one(const TG* __restrict__ arena, const
             constexpr float kAngScale = 7.888609052210118e-31f;  // 2^-100
             const float2 as2 = make_float2(kAngScale, kAngScale), nas2 = make_float2(-kAngScale, -kAngScale);
             const float2 angb2 = make_float2(angb, angb);
+            const WarpPairs* mine = pairs_of + (tid >> 5);
+            const uint32_t to_me = 0xffffffffu >> (31 - (tid & 31));
             auto pairs = [&](auto edge_tag) {
                 constexpr bool kEdge = decltype(edge_tag)::value;
-                float pxb = (float)(2 * (tid - q0 * hp)) - rad_f, py = (float)q0 - rad_f;
-                int c = (q0 + 1) * gst + 2 * (tid - q0 * hp) + 1;  // odd
-                int p = (q0 + 1) & 1;                               // parity of grid row q0 + 1
-                for (;; pxb += dr_f, py += dq_f, c += dc, p ^= dqp) {
-                    // the wrap to the next row as selects: a branch here
-                    // would split the warp for the rest of the step
-                    const bool wrap = pxb > rad_f;
-                    pxb = wrap ? pxb - wrap_f : pxb;
-                    py = wrap ? py + 1.0f : py;
-                    c = wrap ? c + 2 : c;
-                    p = wrap ? p ^ 1 : p;
-                    if (py > rad_f) break;
-                    const float px = p ? pxb - 1.0f : pxb;
+#pragma unroll 1
+                for (int m = tid & 31, before = -1; m < n_pairs; m += 32) {
+                    // the row: as many as have started up to this pair
+                    const uint32_t starts = mine->start[m >> 5];
+                    const PairRow row = mine->row[before + __popc(starts & to_me)];
+                    before += __popc(starts);
+                    const float px = fmaf(2.0f, (float)m, row.px), py = row.py;
                     const bool v0 = px >= -rad_f, v1 = px < rad_f;
+                    const int c = row.c + 2 * m;
                     // rows gr - 1 and gr + 1 sit one slot the other way
-                    const int cv = c + 1 - 2 * p;
+                    const int cv = c + 1 - (row.k & 2);
                     const float2 P = make_float2(px, px + 1.0f), Q = make_float2(py, py);
                     const float2 rx = __ffma2_rn(P, ca2, __fmul2_rn(Q, sa2));
                     const float2 ry = __ffma2_rn(P, nsa2, __fmul2_rn(Q, ca2));
@@ -747,9 +801,6 @@ __device__ __forceinline__ void describe_one(const TG* __restrict__ arena, const
                         in0 = in0 && rowin && !(xs0 < 0.0f || xs0 >= wm1);
                         in1 = in1 && rowin && !(xs1 < 0.0f || xs1 >= wm1);
                     }
-                    // warps whose 64 samples all fall outside skip the rest
-                    if (!__any_sync(__activemask(), in0 || in1)) continue;
-                    if (!(in0 || in1)) continue;
                     // (left, right) and (above, below) of both elements
                     const float2 gl = *reinterpret_cast<const float2*>(grid + c - 1);
                     const float2 gr = *reinterpret_cast<const float2*>(grid + c + 1);
@@ -759,12 +810,8 @@ __device__ __forceinline__ void describe_one(const TG* __restrict__ arena, const
                     const float2 gy = __ffma2_rn(gu, neg1, gd);
                     const float2 m2 = __ffma2_rn(gx, gx, __fmul2_rn(gy, gy));
                     const float2 ea = __ffma2_rn(__ffma2_rn(P, P, __fmul2_rn(Q, Q)), wexp2, fb2);
-                    float2 wm = __fmul2_rn(make_float2(sqrt_approx(m2.x), sqrt_approx(m2.y)),
+                    const float2 wm = __fmul2_rn(make_float2(sqrt_approx(m2.x), sqrt_approx(m2.y)),
                                            make_float2(ex2_approx(ea.x), ex2_approx(ea.y)));
-                    // an element outside the window adds zero shares to
-                    // cell (-1, -1) of its copy
-                    wm.x = in0 ? wm.x : 0.0f;
-                    wm.y = in1 ? wm.y : 0.0f;
                     const float2 ab = __fadd2_rn(atan2_bins2(gy, gx), make_float2(-angb, -angb));
                     const float2 xb = __ffma2_rn(rx, ib2, half3), yb = __ffma2_rn(ry, ib2, half3);
                     // floors by the 1.5 * 2^23 rounding-down add: the low
@@ -773,37 +820,34 @@ __device__ __forceinline__ void describe_one(const TG* __restrict__ arena, const
                     const float2 fx = __ffma2_rn(__fadd2_rn(tx, nm15), neg1, xb);
                     const float2 fy = __ffma2_rn(__fadd2_rn(ty, nm15), neg1, yb);
                     const float2 fa = __ffma2_rn(__fadd2_rn(ta, nm15), neg1, ab);
-                    // histogram word of cell (xbi, ybi), bin abi & 7:
-                    // ((ybi + 1) * 6 + xbi + 1) * 9 + (abi & 7), from the
-                    // float bits (the 0x4B400000 offsets cancel mod 2^32,
-                    // 0x4B400000 & 7 == 0)
-                    constexpr uint32_t kCellOff = 63u - 63u * 0x4B400000u;
-                    uint32_t at0 = __float_as_uint(ty.x) * (uint32_t)(kHistSide * kHistRow) +
-                                   __float_as_uint(tx.x) * (uint32_t)kHistRow + kCellOff +
-                                   (__float_as_uint(ta.x) & 7u);
-                    uint32_t at1 = __float_as_uint(ty.y) * (uint32_t)(kHistSide * kHistRow) +
-                                   __float_as_uint(tx.y) * (uint32_t)kHistRow + kCellOff +
-                                   (__float_as_uint(ta.y) & 7u);
-                    at0 = in0 ? at0 : 0u;
-                    at1 = in1 ? at1 : 0u;
+                    // histogram byte of cell (xbi, ybi), bin abi & 7 and the
+                    // pair's copy, from the float bits (the 0x4B400000
+                    // offsets cancel mod 2^32, 0x4B400000 & 7 == 0)
+                    constexpr uint32_t kA = 4 * kHistBin, kX = 4 * kHistCopies, kY = kX * kHistSide;
+                    constexpr uint32_t kCellOff = (kX + kY) - (kX + kY) * 0x4B400000u;
+                    const uint32_t at = hist_at + kCellOff + (uint32_t)((row.k >> 2) + 4 * m & 28);
+                    const uint32_t at0 = __float_as_uint(ty.x) * kY + __float_as_uint(tx.x) * kX +
+                                         (__float_as_uint(ta.x) & 7u) * kA + at;
+                    const uint32_t at1 = __float_as_uint(ty.y) * kY + __float_as_uint(tx.y) * kX +
+                                         (__float_as_uint(ta.y) & 7u) * kA + at;
                     const float2 wy0 = __fmul2_rn(wm, __ffma2_rn(fy, neg1, one2)), wy1 = __fmul2_rn(wm, fy);
                     const float2 wx0 = __ffma2_rn(fx, neg1, one2);
                     // (1 - fa) * 2^-100 and fa * 2^-100 (exact scalings)
                     const float2 wa0 = __ffma2_rn(fa, nas2, as2), wa1 = __fmul2_rn(fa, as2);
-                    unsigned int* h0 = hcopy + at0;
-                    unsigned int* h1 = hcopy + at1;
+                    uint32_t s0[8], s1[8];
 #pragma unroll
                     for (int cc = 0; cc < 4; ++cc) {
                         const float2 wxy = __fmul2_rn((cc & 1) ? fx : wx0, (cc & 2) ? wy1 : wy0);
-                        const int off = ((cc & 2) ? kHistSide * kHistRow : 0) + ((cc & 1) ? kHistRow : 0);
                         // the products, rounded to the nearest fixed-point
                         // integer on the subnormal grid, are their own bits
                         const float2 n0 = __fmul2_rn(wxy, wa0), n1 = __fmul2_rn(wxy, wa1);
-                        atomicAdd(h0 + off, __float_as_uint(n0.x));
-                        atomicAdd(h0 + off + 1, __float_as_uint(n1.x));
-                        atomicAdd(h1 + off, __float_as_uint(n0.y));
-                        atomicAdd(h1 + off + 1, __float_as_uint(n1.y));
+                        s0[2 * cc] = __float_as_uint(n0.x);
+                        s0[2 * cc + 1] = __float_as_uint(n1.x);
+                        s1[2 * cc] = __float_as_uint(n0.y);
+                        s1[2 * cc + 1] = __float_as_uint(n1.y);
                     }
+                    if (in0) add_shares<kA, kX, kY>(at0, s0);
+                    if (in1) add_shares<kA, kX, kY>(at1, s1);
                 }
             };
             if (edge)
@@ -835,13 +879,14 @@ __device__ __forceinline__ void describe_one(const TG* __restrict__ arena, const
                 const float wa1 = fa * to_fix, wa0 = to_fix - wa1;
                 const float wx0 = 1.0f - fx, wx1 = fx;
                 const float wy0 = wm * (1.0f - fy), wy1 = wm * fy;
-                unsigned int* h0 = hcopy + ((ybi + 1) * kHistSide + (xbi + 1)) * kHistRow + (abi & 7);
+                unsigned int* h0 =
+                    hist + (abi & 7) * kHistBin + ((ybi + 1) * kHistSide + (xbi + 1)) * kHistCopies + (tid & 7);
 #pragma unroll
                 for (int cc = 0; cc < 4; ++cc) {
                     const float wxy = ((cc & 1) ? wx1 : wx0) * ((cc & 2) ? wy1 : wy0);
-                    unsigned int* hc = h0 + ((cc & 2) ? kHistSide * kHistRow : 0) + ((cc & 1) ? kHistRow : 0);
+                    unsigned int* hc = h0 + ((cc & 2) ? kHistSide * kHistCopies : 0) + ((cc & 1) ? kHistCopies : 0);
                     atomicAdd(hc, __float_as_uint(__fmaf_rn(wxy, wa0, kMagic)) - 0x4B000000u);
-                    atomicAdd(hc + 1, __float_as_uint(__fmaf_rn(wxy, wa1, kMagic)) - 0x4B000000u);
+                    atomicAdd(hc + kHistBin, __float_as_uint(__fmaf_rn(wxy, wa1, kMagic)) - 0x4B000000u);
                 }
             }
         }
@@ -850,15 +895,26 @@ __device__ __forceinline__ void describe_one(const TG* __restrict__ arena, const
     // normalize_and_clip_descriptor (src/sift.rs:889-913), one bin per
     // thread; the sums of squares over the four warps in a fixed order
     {
+        // the copies' sums, lanes over the cells (two 16-byte reads a bin),
+        // then handed to the bins' own threads (through the grid's memory)
+        uint32_t* sums = reinterpret_cast<uint32_t*>(grid);
+        {
+            const int ia = tid >> 4, cell = tid & 15;
+            const unsigned int* h = hist + ia * kHistBin + (((cell >> 2) + 1) * kHistSide + (cell & 3) + 1) * kHistCopies;
+            // odd rows of cells read their halves in the other order: no bank conflicts
+            const int turn = cell & 4;
+            uint4 x = *reinterpret_cast<const uint4*>(h + turn), y = *reinterpret_cast<const uint4*>(h + (turn ^ 4));
+            unsigned v = x.x + x.y + x.z + x.w + y.x + y.y + y.z + y.w;
+            if (ia == 0) {
+                x = *reinterpret_cast<const uint4*>(h + 8 * kHistBin + turn);
+                y = *reinterpret_cast<const uint4*>(h + 8 * kHistBin + (turn ^ 4));
+                v += x.x + x.y + x.z + x.w + y.x + y.y + y.z + y.w;
+            }
+            sums[cell * 9 + ia] = v;
+        }
+        __syncthreads();
         const int bin = tid;  // (iy * 4 + ix) * 8 + ia
-        const int cell = bin >> 3, ia = bin & 7;
-        const int at = (((cell >> 2) + 1) * kHistSide + (cell & 3) + 1) * kHistRow + ia;
-        unsigned v = 0u;
-#pragma unroll
-        for (int c = 0; c < kHistCopies; ++c) v += hist[c * kHistStride + at];
-        if (ia == 0)
-#pragma unroll
-            for (int c = 0; c < kHistCopies; ++c) v += hist[c * kHistStride + at + 8];
+        const unsigned v = sums[(bin >> 3) * 9 + (bin & 7)];
         float d = __fmul_rn((float)v, inv_fix);
         float ss = __fmul_rn(d, d);
 #pragma unroll
@@ -882,16 +938,18 @@ __device__ __forceinline__ void describe_one(const TG* __restrict__ arena, const
 }
 
 // One CTA per oriented keypoint (persistent over the list), describe_one on
-// each. Neighbouring samples land in the same bins, so the lanes of a warp
-// add into kHistCopies copies of the histogram: adds to one address
-// serialise, adds to distinct copies do not. Lane l uses copy l & 7, so the
-// lanes sharing a copy hold samples 16 apart (mostly different cells) and
-// neighbouring lanes, which often hit the same bin, use copies 4 banks apart;
-// picking the copy by l >> 2 instead (4 neighbours per copy) costs 13 % more
-// time. The copies are summed in a fixed order; integer sums make the order
-// irrelevant.
-template <typename TG>
-__global__ void __launch_bounds__(kDescThreads, 8) k_descriptor(const TG* __restrict__ arena, EntryTable tab,
+// each. The shared-memory pipe bounds it: 80 % of its wavefronts at octave 0
+// of a 1080p frame (12 857 keypoints, 146 us; half of them the atomics, 2.46 a
+// warp instruction), with 69 % of the issue slots. What it was before, with a
+// histogram of bins innermost and pairs listed one by one in shared memory:
+// 167 us, the stage 223 us at 1080p and 1406 us at 4096 x 4096, now 199 and
+// 1261. Of that, the bank layout, the warps' own enumeration of their pairs
+// and the sums over copies gave 1406 -> 1298 us, the grid fill by words 1276,
+// rows of cells 5 apart 1261. Adding the shares of a pair's two samples at
+// once where they have the same cells and bin made 7 % more instructions and
+// no difference in time; 16 copies (2.1 wavefronts) leave room for 6 CTAs per
+// SM, and 6 took 2.5 % more than 7.
+__global__ void __launch_bounds__(kDescThreads, 7) k_descriptor(const uint8_t* __restrict__ u8arena, EntryTable tab,
                                                               const Keypoint* __restrict__ oriented,
                                                               OctCounters* __restrict__ oc,
                                                               float* __restrict__ desc, uint32_t cap,
@@ -899,7 +957,8 @@ __global__ void __launch_bounds__(kDescThreads, 8) k_descriptor(const TG* __rest
                                                               int persist_from) {
     chain_wait();
     __shared__ __align__(16) float grid[kDescGridSide * (kDescGridSide + 1)];
-    __shared__ __align__(16) unsigned int hist[kHistCopies * kHistStride];
+    __shared__ __align__(16) unsigned int hist[kHistWords];
+    __shared__ WarpPairs pairs_of[kDescThreads / 32];
     __shared__ float red_lo[kDescThreads / 32], red_hi[kDescThreads / 32];
     const int tid = threadIdx.x;
     const uint32_t base = oc->out_base;
@@ -932,12 +991,11 @@ __global__ void __launch_bounds__(kDescThreads, 8) k_descriptor(const TG* __rest
         const uint32_t i = base + (n - 1 - cur);
         const Keypoint kp = oriented[i];
         // keypoints below hcap straight into the host call's mapped buffer
-        describe_one<TG>(arena, tab, kp, grid, hist, red_lo, red_hi,
+        describe_one(u8arena, tab, kp, grid, hist, pairs_of, red_lo, red_hi,
                          [&] { return (i < hcap ? hdesc : desc) + (size_t)i * kDescLen; });
         if (tid == 0) next[p ^ 1] = claim;
     }
 }
-
 
 }  // namespace
 
@@ -965,22 +1023,12 @@ int launch_orient_emit(const Keypoint* refined_at, uint32_t ncap, int o, Counter
     return cudaPeekAtLastError() == cudaSuccess ? 0 : -1;
 }
 
-template <typename TG>
-int launch_descriptor(const TG* arena, const EntryTable& tab, const Keypoint* oriented,
-                      OctCounters* oc, float* desc, uint32_t cap, const RunCell* cell, int grid, int persist_ctas,
-                      cudaStream_t st) {
-    if (launch_chained(k_descriptor<TG>, grid, kDescThreads, 0, st, arena, tab, oriented, oc, desc, cap, cell,
+int launch_descriptor(const uint8_t* u8arena, const EntryTable& tab, const Keypoint* oriented, OctCounters* oc,
+                      float* desc, uint32_t cap, const RunCell* cell, int grid, int persist_ctas, cudaStream_t st) {
+    if (launch_chained(k_descriptor, grid, kDescThreads, 0, st, u8arena, tab, oriented, oc, desc, cap, cell,
                        std::max(grid - persist_ctas, 0)) != cudaSuccess)
         return -1;
     return cudaPeekAtLastError() == cudaSuccess ? 0 : -1;
 }
-
-#define SIFT_INST(TG)                                                                                              \
-    template int launch_descriptor<TG>(const TG*, const EntryTable&, const Keypoint*, OctCounters*,                \
-                                       float*, uint32_t, const RunCell*, int, int, cudaStream_t);
-SIFT_INST(float)
-SIFT_INST(__half)
-SIFT_INST(uint8_t)
-#undef SIFT_INST
 
 }  // namespace sift

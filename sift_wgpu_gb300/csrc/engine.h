@@ -90,10 +90,8 @@ int launch_orientation(const uint8_t* u8arena, const EntryTable& tab, const floa
 int launch_orient_emit(const Keypoint* refined_at, uint32_t ncap, int o, Counters* ctr, const float* ori_angle,
                        const uint32_t* ori_count, const uint32_t* ori_off, Keypoint* oriented, uint32_t cap,
                        cudaStream_t st);
-template <typename TG>
-int launch_descriptor(const TG* arena, const EntryTable& tab, const Keypoint* oriented,
-                      OctCounters* oc, float* desc, uint32_t cap, const RunCell* cell, int grid, int persist_ctas,
-                      cudaStream_t st);
+int launch_descriptor(const uint8_t* u8arena, const EntryTable& tab, const Keypoint* oriented, OctCounters* oc,
+                      float* desc, uint32_t cap, const RunCell* cell, int grid, int persist_ctas, cudaStream_t st);
 // Error reporting (engine.cu): the calling thread's sift_cuda_last_error.
 extern thread_local std::string g_last_error;
 int fail(int code, const std::string& msg);
@@ -782,7 +780,7 @@ struct Engine {
             const int grid = (int)std::max<uint32_t>(cap_c[o] / 16, 64);
             // host calls: descriptors below cap_x go straight into the mapped
             // export buffer while the stage runs, the rest to d_desc
-            if (ok(launch_descriptor<TG>(G, tab(), d_oriented.as<Keypoint>(), &ctr->oct[o], d_desc.as<float>(), cap_ori,
+            if (ok(launch_descriptor(U, tab(), d_oriented.as<Keypoint>(), &ctr->oct[o], d_desc.as<float>(), cap_ori,
                                          exp ? rc : nullptr, grid, 152 * tune.desc_ctas_per_sm, q)))
                 return cuda_fail(cudaGetLastError(), "descriptor");
             return 0;
