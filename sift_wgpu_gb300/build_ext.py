@@ -24,7 +24,7 @@ ARCH = "-gencode=arch=compute_103a,code=sm_103a"
 
 CU_SOURCES = ["scan.cu", "pyramid.cu", "detect.cu", "describe.cu", "engine.cu", "server.cu", "convert.cu", "export.cu", "noalloc.cu", "match.cu", "draw.cu", "batch.cu"]
 CPP_SOURCES = ["tables.cpp"]
-HEADERS = ["sift_internal.cuh", "tables.h", "engine.h", "tma.cuh", "level_tc.cuh"]
+HEADERS = ["sift_internal.cuh", "tables.h", "engine.h", "tma.cuh", "level_tc.cuh", "tile_scan.cuh"]
 
 
 def _nvcc() -> str:

@@ -9,12 +9,12 @@
 //                that octave of every image; each octave's levels above S run
 //                on a second stream beside the next octave
 //   extrema      one launch over the tiles of every entry
-//   candidates   one prefix scan over every entry's mask words: the mask
-//                words are image-major too, so the candidates come out in
-//                (image, octave, layer, y, x) order, each image's in the
-//                reference order
-//   refinement, orientation, oriented keypoints, descriptors: one launch
-//                each over the batch's single lists
+//   candidates   one list over every entry's mask words: they are
+//                image-major too, so the candidates come out in (image,
+//                octave, layer, y, x) order, each image's in the reference
+//                order; with their refinement
+//   orientation, oriented keypoints, descriptors: one launch each over the
+//                batch's single lists
 //   export       each image's range of the output and the octave fields
 //
 // The whole run is captured as one CUDA graph per batch geometry and replayed;
@@ -102,7 +102,7 @@ struct BatchEngine {
     bool host_reads = false;
     std::vector<unsigned long long> h_addr;
     std::vector<int> h_pitch;
-    DevMem d_words, d_cand_off, d_scan, d_cands, d_refined, d_keep, d_ori_angle, d_ori_count, d_ori_off, d_oriented,
+    DevMem d_words, d_cand_off, d_tiles, d_cands, d_refined, d_keep, d_ori_angle, d_ori_count, d_ori_off, d_oriented,
         d_desc, d_ctr;
     HostPinned h_ctr;
     // Mapped host buffer the run writes its results into: Counters | ranges
@@ -120,7 +120,7 @@ struct BatchEngine {
     cudaEvent_t ev_t0 = nullptr, ev_t1 = nullptr;
     float device_ms = 0.0f;
     uint32_t cap_cand = 0, cap_ori = 0;
-    size_t scan_words = 0, scan_b = 0;  // scan state: words scan at 0, orientation-count scan at scan_b
+    size_t n_tiles = 0, slots_at = 0;  // tile counts: of the mask words at 0, of the candidate slots at slots_at
     uint32_t n_out = 0;
     bool images_in_place = false;  // the last run read the caller's images in place
 
@@ -351,9 +351,9 @@ struct BatchEngine {
         CK(d_ori_off.ensure((size_t)cap_cand * 4), "cudaMalloc(ori_off)");
         CK(d_oriented.ensure((size_t)cap_ori * kp), "cudaMalloc(oriented)");
         CK(d_desc.ensure((size_t)cap_ori * kDescLen * 4), "cudaMalloc(desc)");
-        scan_b = scan_state_words((size_t)std::max<long long>(total_words, 1));
-        scan_words = scan_b + scan_state_words(cap_cand);
-        CK(d_scan.ensure(scan_words * sizeof(unsigned long long)), "cudaMalloc(scan state)");
+        slots_at = word_tiles(total_words);
+        n_tiles = slots_at + slot_tiles(cap_cand);
+        CK(d_tiles.ensure(std::max<size_t>(n_tiles, 1) * sizeof(uint32_t)), "cudaMalloc(tile counts)");
         return 0;
     }
 
@@ -399,7 +399,7 @@ struct BatchEngine {
             return 0;
         };
         CK(cudaMemsetAsync(d_ctr.p, 0, sizeof(Counters), st), "memset counters");
-        CK(cudaMemsetAsync(d_scan.p, 0, scan_words * sizeof(unsigned long long), st), "memset scan state");
+        CK(cudaMemsetAsync(d_tiles.p, 0, n_tiles * sizeof(uint32_t), st), "memset tile counts");
         auto level = [&](int o, int s, cudaStream_t q, uint8_t* tmp) -> int {
             const LevelBlur& b = s == 0 ? base : lv[o][s - 1];
             const OctPref& pf = opref[o];
@@ -441,34 +441,25 @@ struct BatchEngine {
         CK(cudaEventRecord(ev_side, st2), "event record");
         CK(cudaStreamWaitEvent(st, ev_side, 0), "stream wait");
         // detection over every entry
-        unsigned long long* sst = d_scan.as<unsigned long long>();
+        uint32_t *tiles = d_tiles.as<uint32_t>(), *slots = tiles + slots_at;
         if (int rc = bump(launch_extrema_mask_flat(U, lut, tb, 0, N * O, pref(ex_pref), n_ex, (int)p.image_border_width,
-                                                   d_words.as<uint32_t>(), st),
+                                                   d_words.as<uint32_t>(), tiles, st),
                           "batch extrema"))
             return rc;
-        if (scan_exclusive(d_words.as<uint32_t>(), SCAN_POPC, d_cand_off.as<uint32_t>(), (size_t)total_words, nullptr,
-                           &oc->n_cand, sst, &ctr->overflow, st))
-            return cuda_fail(cudaGetLastError(), "batch scan");
-        if (int rc = bump(launch_emit(U, lut, tb, 0, N * O, total_words, d_words.as<uint32_t>(),
-                                      d_cand_off.as<uint32_t>(), d_cands.as<Keypoint>(), cap_cand, ctr, st),
-                          "batch emit"))
-            return rc;
-        if (int rc = bump(launch_refine(U, lut, tb, p.sigma, p.contrast_threshold, p.edge_threshold,
-                                        d_cands.as<Keypoint>(), d_refined.as<Keypoint>(), d_keep.as<uint32_t>(),
-                                        cap_cand, oc, st),
-                          "batch refine"))
+        if (int rc = bump(launch_candidates(U, lut, tb, p.sigma, p.contrast_threshold, p.edge_threshold, 0, N * O,
+                                            total_words, d_words.as<uint32_t>(), tiles, d_cand_off.as<uint32_t>(),
+                                            d_cands.as<Keypoint>(), d_refined.as<Keypoint>(), d_keep.as<uint32_t>(),
+                                            cap_cand, ctr, oc, st),
+                          "batch candidates"))
             return rc;
         const int ogrid = (int)std::max<uint32_t>(cap_cand / 64, 32);
         if (int rc = bump(launch_orientation(U, tb, lut, d_bins.as<uint8_t>(), d_refined.as<Keypoint>(), d_keep.as<uint32_t>(),
                                                       cap_cand, oc, d_ori_angle.as<float>(), d_ori_count.as<uint32_t>(),
-                                                      ogrid, 152 * 4, st),
+                                                      slots, ogrid, 152 * 4, st),
                           "batch orientation"))
             return rc;
-        if (scan_exclusive(d_ori_count.as<uint32_t>(), SCAN_U32, d_ori_off.as<uint32_t>(), cap_cand, &oc->n_cand,
-                           &oc->n_ori, sst + scan_b, &ctr->overflow, st))
-            return cuda_fail(cudaGetLastError(), "batch orientation scan");
         if (int rc = bump(launch_orient_emit(d_refined.as<Keypoint>(), cap_cand, 0, ctr, d_ori_angle.as<float>(),
-                                             d_ori_count.as<uint32_t>(), d_ori_off.as<uint32_t>(),
+                                             d_ori_count.as<uint32_t>(), slots, d_ori_off.as<uint32_t>(),
                                              d_oriented.as<Keypoint>(), cap_ori, st),
                           "batch orientation emit"))
             return rc;
@@ -482,7 +473,7 @@ struct BatchEngine {
                            (const Counters*)ctr, cap_cand, d_oriented.as<Keypoint>(), cap_ori, hx_dctr, hx_dranges,
                            hx_dkps, cap_x) != cudaSuccess)
             return cuda_fail(cudaGetLastError(), "batch export");
-        launches = (uint32_t)nl + 11;  // extrema, 2 scans, emit, refine, orientation, its emit, descriptors, export
+        launches = (uint32_t)nl + 6;  // extrema, candidates, orientation, its emit, descriptors, export
         return 0;
     }
 
@@ -554,7 +545,6 @@ struct BatchEngine {
             CK(cudaStreamSynchronize(st), "batch run");
             CK(cudaEventElapsedTime(&device_ms, ev_t0, ev_t1), "event time");
             const Counters c = *hx.as<Counters>();
-            if (c.overflow & 8u) return fail(SIFT_CUDA_ERR_CUDA, "a prefix-scan wait ran out (the run was abandoned)");
             bool grow = false;
             if (c.oct[0].n_cand > cap_cand || (c.overflow & 1u)) {
                 const size_t nc = (size_t)c.oct[0].n_cand + c.oct[0].n_cand / 4 + 1024;

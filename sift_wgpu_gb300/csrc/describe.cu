@@ -11,10 +11,6 @@
 //                   columns are summed in a fixed order, then the two [1,1,1]/3
 //                   smoothing passes and the peak test run one bin per lane;
 //                   peaks come out in bin order through a ballot.
-//   k_orient_emit   candidate slot i with c_i peaks (0 if refinement rejected
-//                   it) writes its c_i oriented copies at the scanned offset,
-//                   so the output order is the reference's (keypoint, bin)
-//                   order.
 //   k_descriptor    one CTA per oriented keypoint (describe_one): the bilinear
 //                   samples of the window are computed once into a shared grid,
 //                   pairs of window samples are split over the threads and
@@ -371,7 +367,7 @@ __global__ void __launch_bounds__(32 * kOriWarps, 5) k_orientation(const uint8_t
                                                                 OctCounters* __restrict__ oc,
                                                                 float* __restrict__ ori_angle,
                                                                 uint32_t* __restrict__ ori_count,
-                                                                int persist_from) {
+                                                                uint32_t* __restrict__ tiles, int persist_from) {
     chain_wait();
     __shared__ __align__(16) float hist[kOriWarps][kOriBins][32];
     __shared__ float slut[256];
@@ -400,38 +396,10 @@ __global__ void __launch_bounds__(32 * kOriWarps, 5) k_orientation(const uint8_t
             const uint32_t i = n - 1 - (i0 + (uint32_t)__ffs(m) - 1u);
             const uint32_t cnt = orient_one(u8arena, tab, refined_at[i], &hist[wid][0][0], lane,
                                             ori_angle + (size_t)i * kOriMaxPeaks, tb);
-            if (lane == 0) ori_count[i] = cnt;
-        }
-    }
-}
-
-// Octave o's oriented keypoints go after those of octaves 0..o-1 (whose
-// counts are final: their orientation scans precede this kernel). Candidate
-// slot i holds ori_count[i] peaks (0 for a rejected candidate).
-__global__ void k_orient_emit(const Keypoint* __restrict__ refined_at, uint32_t ncap, int o,
-                              Counters* __restrict__ ctr, const float* __restrict__ ori_angle,
-                              const uint32_t* __restrict__ ori_count, const uint32_t* __restrict__ ori_off,
-                              Keypoint* __restrict__ oriented, uint32_t cap) {
-    chain_wait();
-    OctCounters* oc = &ctr->oct[o];
-    uint32_t base = 0;
-    for (int q = 0; q < o; ++q) base += ctr->oct[q].n_ori;
-    const uint32_t n = min(oc->n_cand, ncap);
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-        oc->out_base = base;
-        atomicAdd(&ctr->n_candidates, oc->n_cand);
-        atomicAdd(&ctr->n_refined, oc->n_ref);
-        atomicMax(&ctr->n_oriented, base + oc->n_ori);
-        if (base + oc->n_ori > cap) atomicOr(&ctr->overflow, 4u);
-    }
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const uint32_t c = ori_count[i], off = base + ori_off[i];
-        if (c == 0) continue;
-        Keypoint k = refined_at[i];
-        for (uint32_t j = 0; j < c; ++j) {
-            if (off + j >= cap) break;
-            k.angle = ori_angle[(size_t)i * kOriMaxPeaks + j];
-            oriented[off + j] = k;
+            if (lane == 0) {
+                ori_count[i] = cnt;
+                if (cnt) atomicAdd(&tiles[i / kSlotTile], cnt);
+            }
         }
     }
 }
@@ -1007,18 +975,10 @@ int launch_ori_bins(uint8_t* bins, cudaStream_t st) {
 
 int launch_orientation(const uint8_t* u8arena, const EntryTable& tab, const float* lut255, const uint8_t* bins,
                        const Keypoint* refined_at, const uint32_t* keep, uint32_t ncap, OctCounters* oc,
-                       float* ori_angle, uint32_t* ori_count, int grid, int persist_ctas, cudaStream_t st) {
-    if (launch_chained(k_orientation, grid, dim3(32, kOriWarps), 0, st, u8arena, tab, lut255, bins, refined_at, keep,
-                       ncap, oc, ori_angle, ori_count, std::max(grid - persist_ctas, 0)) != cudaSuccess)
-        return -1;
-    return cudaPeekAtLastError() == cudaSuccess ? 0 : -1;
-}
-
-int launch_orient_emit(const Keypoint* refined_at, uint32_t ncap, int o, Counters* ctr, const float* ori_angle,
-                       const uint32_t* ori_count, const uint32_t* ori_off, Keypoint* oriented, uint32_t cap,
+                       float* ori_angle, uint32_t* ori_count, uint32_t* tiles, int grid, int persist_ctas,
                        cudaStream_t st) {
-    if (launch_chained(k_orient_emit, 152, 256, 0, st, refined_at, ncap, o, ctr, ori_angle, ori_count, ori_off,
-                       oriented, cap) != cudaSuccess)
+    if (launch_chained(k_orientation, grid, dim3(32, kOriWarps), 0, st, u8arena, tab, lut255, bins, refined_at, keep,
+                       ncap, oc, ori_angle, ori_count, tiles, std::max(grid - persist_ctas, 0)) != cudaSuccess)
         return -1;
     return cudaPeekAtLastError() == cudaSuccess ? 0 : -1;
 }

@@ -1,20 +1,20 @@
-// detect.cu — 26-neighbour extrema, subpixel refinement, ordered compaction.
+// detect.cu — 26-neighbour extrema, ordered candidates, subpixel refinement.
 //
 // Stages (b) and (c) of the hot path: find_scale_space_extrema
 // (src/sift.rs:510-603) and refine_and_filter_extrema (src/sift.rs:299-474).
 //
-//   k_extrema_mask   one warp per 32 consecutive pixels of a row: the strict
-//                    26-neighbour test, one ballot word per warp (no atomics).
-//   scan             exclusive prefix sum of popcount(word) gives every
-//                    candidate its slot in (octave, layer, y, x) order, the
-//                    order rayon's collect produces in the reference.
-//   k_emit           one thread per word writes the word's candidates to their
-//                    slots.
-//   k_refine         one thread per candidate: the Newton refinement, contrast
-//                    and edge tests in the reference's f32 operation order;
-//                    the result stays in the candidate's slot with a keep
-//                    flag (the orientation stage reads the slots in order and
-//                    skips the rejected ones, so no compaction pass is needed).
+//   k_extrema_mask   the strict 26-neighbour test of a tile of pixels, one
+//                    ballot word per 32 pixels of a row; the candidates are
+//                    counted by tiles of words as they are found.
+//   k_candidates     a CTA per tile of words: the counts of the tiles before
+//                    it give every candidate its slot in (octave, layer, y,
+//                    x) order, the order rayon's collect produces in the
+//                    reference; then one thread per candidate, the Newton
+//                    refinement, contrast and edge tests in the reference's
+//                    f32 operation order; the result stays in the candidate's
+//                    slot with a keep flag (the orientation stage reads the
+//                    slots in order and skips the rejected ones, so no
+//                    compaction pass is needed).
 //
 // All arithmetic is f32 with separately rounded operations (no FMA), so the
 // candidates and refined keypoints are bit-identical to the CPU path; the one
@@ -22,7 +22,7 @@
 // f64 and rounded once.
 #include <algorithm>
 
-#include "sift_internal.cuh"
+#include "tile_scan.cuh"
 
 namespace sift {
 namespace {
@@ -114,7 +114,8 @@ constexpr int kExSH = kExTY + 2;
 template <int NL>
 __device__ __forceinline__ void extrema_tile(const uint8_t* __restrict__ u8arena, const float* __restrict__ lut255,
                                              const OctaveDev& od, int S, int border, uint32_t* __restrict__ words,
-                                             int x0, int y0, float* tile) {
+                                             long long word0, uint32_t* __restrict__ tiles, int x0, int y0,
+                                             float* tile) {
     const int W = od.W, H = od.H, nw = od.nw, L = NL > 0 ? NL : S + 2;
     const int tid = threadIdx.x, lane = tid & 31;
     float* lut = tile + L * kExSH * kExSW;
@@ -164,7 +165,11 @@ __device__ __forceinline__ void extrema_tile(const uint8_t* __restrict__ u8arena
                 const bool ext = yin[j] && ((v > fmaxf(fmaxf(BMp[j], BMn[j]), RMc[j])) ||
                                             (v < fminf(fminf(Bmp[j], Bmn[j]), Rmc[j])));
                 const uint32_t wv = __ballot_sync(0xffffffffu, ext);
-                if (lane == 0 && y < H && word < nw) words[od.word_base + ((long long)(s - 1) * H + y) * nw + word] = wv;
+                if (lane == 0 && y < H && word < nw) {
+                    const long long w = od.word_base + ((long long)(s - 1) * H + y) * nw + word;
+                    words[w] = wv;
+                    if (wv) atomicAdd(&tiles[(w - word0) / kWordTile], (uint32_t)__popc(wv));
+                }
             }
         }
 #pragma unroll
@@ -180,15 +185,18 @@ __device__ __forceinline__ void extrema_tile(const uint8_t* __restrict__ u8arena
     }
 }
 
-// The extrema mask of entry e (one octave of one image), a tile per CTA.
+// The extrema mask of entry e (one octave of one image), a tile per CTA; the
+// candidates are counted by tiles of kWordTile words, from word0 on.
 template <int NL>
 __global__ void __launch_bounds__(256, 4) k_extrema_mask(const uint8_t* __restrict__ u8arena,
                                                       const float* __restrict__ lut255, EntryTable tab, int e,
-                                                      int border, uint32_t* __restrict__ words) {
+                                                      int border, uint32_t* __restrict__ words, long long word0,
+                                                      uint32_t* __restrict__ tiles) {
     chain_wait();
     extern __shared__ __align__(16) float tile[];  // [layers][kExSH][kExSW], then lut[256]
     const OctaveDev od = tab.ents[e];
-    extrema_tile<NL>(u8arena, lut255, od, tab.S, border, words, blockIdx.x * kExTX, blockIdx.y * kExTY, tile);
+    extrema_tile<NL>(u8arena, lut255, od, tab.S, border, words, word0, tiles, blockIdx.x * kExTX, blockIdx.y * kExTY,
+                     tile);
 }
 
 // The extrema masks of entries e0 .. e0 + n_e - 1 in one launch: CTA b takes
@@ -198,7 +206,8 @@ template <int NL>
 __global__ void __launch_bounds__(256, 4) k_extrema_mask_flat(const uint8_t* __restrict__ u8arena,
                                                            const float* __restrict__ lut255, EntryTable tab, int e0,
                                                            int n_e, const uint32_t* __restrict__ tile_pref,
-                                                           int border, uint32_t* __restrict__ words) {
+                                                           int border, uint32_t* __restrict__ words,
+                                                           long long word0, uint32_t* __restrict__ tiles) {
     chain_wait();
     extern __shared__ __align__(16) float tile[];
     const uint32_t b = blockIdx.x;
@@ -210,7 +219,7 @@ __global__ void __launch_bounds__(256, 4) k_extrema_mask_flat(const uint8_t* __r
     const OctaveDev od = tab.ents[e0 + lo];
     const int tx = (od.W + kExTX - 1) / kExTX;
     const int t = (int)(b - tile_pref[lo]);
-    extrema_tile<NL>(u8arena, lut255, od, tab.S, border, words, (t % tx) * kExTX, (t / tx) * kExTY, tile);
+    extrema_tile<NL>(u8arena, lut255, od, tab.S, border, words, word0, tiles, (t % tx) * kExTX, (t / tx) * kExTY, tile);
 }
 
 // solve_linear_system (src/sift.rs:478-503), Cramer's rule in f32.
@@ -316,88 +325,109 @@ __device__ bool refine_one(const Dog& dog, int o, int entry, int x, int y, int s
     return false;
 }
 
-// One thread per mask word of entries e0 .. e0 + n_e - 1 (their words are
-// consecutive; w counts from the first entry's first word): the candidates of
-// the word go to their scanned slots, in x order within the word, i.e.
-// (entry, layer, y, x) order. A candidate's octave field holds its entry.
-__global__ void __launch_bounds__(256) k_emit(const uint8_t* __restrict__ u8arena, const float* __restrict__ lut255,
-                                              EntryTable tab, int e0, int n_e, long long n_words,
-                                              const uint32_t* __restrict__ words,
-                                              const uint32_t* __restrict__ cand_off,
-                                              Keypoint* __restrict__ cands, uint32_t cap,
-                                              Counters* __restrict__ ctr) {
-    chain_wait();
-    const long long w = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (w >= n_words) return;
-    uint32_t word = words[w];
-    if (word == 0u) return;
-    const long long base0 = tab.ents[e0].word_base;
-    int lo = 0, hi = n_e;  // the last entry whose first word is <= w
-    while (hi - lo > 1) {
-        const int mid = (lo + hi) >> 1;
-        if (tab.ents[e0 + mid].word_base - base0 <= w) lo = mid; else hi = mid;
-    }
-    const int e = e0 + lo;
-    const OctaveDev od = tab.ents[e];
-    const long long we = w - (od.word_base - base0);
-    const DogFromU8 dog{u8arena + od.u_off, lut255, od.plane, od.pitch, od.W, od.H};
-    const int c = (int)(we % od.nw);
-    const long long rowid = we / od.nw;
-    const int y = (int)(rowid % od.H);
-    const int s = (int)(rowid / od.H) + 1;
-    const float scale = __int_as_float((127 + od.octave) << 23);
-    uint32_t ci = cand_off[w];
-    while (word) {
-        const int b = __ffs(word) - 1;
-        word &= word - 1u;
-        const int x = c * 32 + b;
-        if (ci >= cap) {
-            atomicOr(&ctr->overflow, 1u);
-            return;
-        }
-        Keypoint k;
-        k.x = __fmul_rn(__fadd_rn((float)x, 0.5f), scale);
-        k.y = __fmul_rn(__fadd_rn((float)y, 0.5f), scale);
-        k.size = 0.0f;
-        k.angle = 0.0f;
-        k.response = dog.at(s, x, y);
-        k.octave = e;
-        k.layer = s;
-        cands[ci++] = k;
-    }
-}
-
-// One thread per candidate (persistent grid over the count); a candidate's
-// entry (its octave field) gives its octave and DoG planes. The survivors are
+// The candidates of entries e0 .. e0 + n_e - 1 (whose mask words are
+// consecutive; w counts from the first entry's first word) in (entry, layer, y,
+// x) order, and their refinement. A CTA takes a tile of words: the counts of
+// the tiles before it give its first slot, the words' bits go to a list in
+// shared memory in order, then one thread per candidate writes its slot (a
+// candidate's octave field holds its entry) and refines it. The survivors are
 // counted per warp into oc->n_ref (a count, order-free).
-__global__ void __launch_bounds__(256) k_refine(const uint8_t* __restrict__ u8arena,
-                                                const float* __restrict__ lut255, EntryTable tab,
-                                                RefineParams rp, const Keypoint* __restrict__ cands,
-                                                Keypoint* __restrict__ refined_at, uint32_t* __restrict__ keep,
-                                                uint32_t cap, OctCounters* __restrict__ oc) {
+//
+// Latency bounds it (a chain of dependent scattered reads per candidate and
+// step), so the tiles are small: 512 words, some 50 candidates of a dense
+// frame, make 380 CTAs of a 1080p octave 0. It takes 20 us there and 54 us at
+// 4096 x 4096 (cold caches); a scan of the word counts with look-back, a kernel
+// that emitted and one that refined took 12.7 + 5.9 + 20 and 30 + 17 + 60 us.
+// The stage with the mask: 123 -> 91 us at 1080p, 410 -> 351 at 4096 x 4096;
+// a 160 x 120 frame, end to end, 136 -> 122.
+constexpr int kCandThreads = 128, kCandWords = kWordTile / kCandThreads;
+constexpr uint32_t kCandList = 1024;  // candidates at a time
+static_assert(kWordTile * 32 <= 1 << 16, "a bit's index in its tile has 16 bits");
+__global__ void __launch_bounds__(kCandThreads) k_candidates(
+    const uint8_t* __restrict__ u8arena, const float* __restrict__ lut255, EntryTable tab, RefineParams rp, int e0,
+    int n_e, long long n_words, const uint32_t* __restrict__ words, const uint32_t* __restrict__ tiles,
+    uint32_t n_tiles, uint32_t* __restrict__ cand_off, Keypoint* __restrict__ cands,
+    Keypoint* __restrict__ refined_at, uint32_t* __restrict__ keep, uint32_t cap, Counters* __restrict__ ctr,
+    OctCounters* __restrict__ oc) {
     chain_wait();
     __shared__ float lut[256];
-    lut[threadIdx.x] = lut255[threadIdx.x];
-    __syncthreads();
-    const uint32_t n = min(oc->n_cand, cap);
-    const uint32_t stride = gridDim.x * blockDim.x;
-    for (uint32_t i0 = blockIdx.x * blockDim.x; i0 < n; i0 += stride) {
-        const uint32_t i = i0 + threadIdx.x;
-        bool ok = false;
-        if (i < n) {
-            const Keypoint k = cands[i];
-            const OctaveDev od = tab.ents[k.octave];
-            const DogFromU8 dog{u8arena + od.u_off, lut, od.plane, od.pitch, od.W, od.H};
-            const float scale = __int_as_float((127 + od.octave) << 23);
-            const int x = rust_as_i32(__fdiv_rn(k.x, scale)), y = rust_as_i32(__fdiv_rn(k.y, scale));
-            Keypoint r;
-            ok = refine_one(dog, od.octave, k.octave, x, y, k.layer, rp, &r);
-            if (ok) refined_at[i] = r;
-            keep[i] = ok ? 1u : 0u;
+    __shared__ uint16_t list[kCandList];
+    __shared__ uint32_t buf[kCandThreads / 32];
+    const int tid = threadIdx.x;
+    for (int v = tid; v < 256; v += kCandThreads) lut[v] = lut255[v];
+    const long long base0 = tab.ents[e0].word_base;
+    uint32_t base = 0, from = 0, kept = 0;
+    for (uint32_t t = blockIdx.x; t < n_tiles; t += gridDim.x) {
+        base += tiles_sum<kCandThreads>(tiles, from, t, buf);  // (and lut and list are free to use)
+        from = t;
+        const uint32_t count = tiles[t];
+        if (t == n_tiles - 1 && tid == 0) oc->n_cand = base + count;
+        if (count == 0 && !cand_off) continue;
+        const long long w0 = (long long)t * kWordTile, mine = w0 + tid * kCandWords;
+        uint32_t v[kCandWords], s = 0;
+#pragma unroll
+        for (int k = 0; k < kCandWords; ++k) {
+            v[k] = mine + k < n_words ? words[mine + k] : 0u;
+            s += __popc(v[k]);
         }
-        const uint32_t m = __ballot_sync(0xffffffffu, ok);
-        if ((threadIdx.x & 31) == 0 && m) atomicAdd(&oc->n_ref, (uint32_t)__popc(m));
+        const uint32_t ex = block_exclusive<kCandThreads>(s, buf);
+        if (cand_off) {
+            uint32_t at = base + ex;
+#pragma unroll
+            for (int k = 0; k < kCandWords; ++k) {
+                if (mine + k < n_words) cand_off[mine + k] = at;
+                at += __popc(v[k]);
+            }
+        }
+        for (uint32_t first = 0; first < count; first += kCandList) {
+            uint32_t at = ex - first;  // (wraps below first)
+#pragma unroll
+            for (int k = 0; k < kCandWords; ++k)
+                for (uint32_t m = v[k]; m; m &= m - 1u, ++at)
+                    if (at < kCandList) list[at] = (uint16_t)((tid * kCandWords + k) * 32 + __ffs(m) - 1);
+            __syncthreads();
+            const uint32_t n = min(count - first, kCandList);
+            for (uint32_t j = tid; j < n; j += kCandThreads) {
+                const uint32_t ci = base + first + j;
+                if (ci >= cap) {
+                    atomicOr(&ctr->overflow, 1u);
+                    break;
+                }
+                const long long w = w0 + (list[j] >> 5);
+                int lo = 0, hi = n_e;  // the last entry whose first word is <= w
+                while (hi - lo > 1) {
+                    const int mid = (lo + hi) >> 1;
+                    if (tab.ents[e0 + mid].word_base - base0 <= w) lo = mid; else hi = mid;
+                }
+                const int e = e0 + lo;
+                const OctaveDev od = tab.ents[e];
+                const DogFromU8 dog{u8arena + od.u_off, lut, od.plane, od.pitch, od.W, od.H};
+                const long long we = w - (od.word_base - base0);
+                const uint32_t row = we >> 32 ? (uint32_t)(we / od.nw) : (uint32_t)we / (uint32_t)od.nw;
+                const uint32_t layer = row / (uint32_t)od.H;
+                const int x = (int)((uint32_t)we - row * (uint32_t)od.nw) * 32 + (list[j] & 31);
+                const int y = (int)(row - layer * (uint32_t)od.H), sc = (int)layer + 1;
+                const float scale = __int_as_float((127 + od.octave) << 23);
+                Keypoint k;
+                k.x = __fmul_rn(__fadd_rn((float)x, 0.5f), scale);
+                k.y = __fmul_rn(__fadd_rn((float)y, 0.5f), scale);
+                k.size = 0.0f;
+                k.angle = 0.0f;
+                k.response = dog.at(sc, x, y);
+                k.octave = e;
+                k.layer = sc;
+                cands[ci] = k;
+                Keypoint r;
+                const bool ok = refine_one(dog, od.octave, e, x, y, sc, rp, &r);
+                if (ok) refined_at[ci] = r;
+                keep[ci] = ok ? 1u : 0u;
+                kept += ok;
+            }
+            __syncthreads();
+        }
     }
+    kept = __reduce_add_sync(0xffffffffu, kept);
+    if ((tid & 31) == 0 && kept) atomicAdd(&oc->n_ref, kept);
 }
 
 // Debug read-back of DoG layer l of octave o as a dense W x H f32 plane, each
@@ -429,17 +459,18 @@ int launch_dog_dense(const uint8_t* u8arena, const float* lut255, const PyramidD
 static size_t extrema_smem(int S) { return sizeof(float) * ((size_t)(S + 2) * kExSH * kExSW + 256); }
 
 int launch_extrema_mask(const uint8_t* u8arena, const float* lut255, const EntryTable& tab, const OctaveDev& od,
-                        int e, int border, uint32_t* words, cudaStream_t st) {
+                        int e, int border, uint32_t* words, uint32_t* tiles, cudaStream_t st) {
     if (od.W <= 0 || od.H <= 0) return 0;
     if (tab.S + 2 > kExMaxLayers) return -1;
     dim3 grid((od.W + kExTX - 1) / kExTX, (od.H + kExTY - 1) / kExTY);
     const size_t smem = extrema_smem(tab.S);
-    void (*k)(const uint8_t*, const float*, EntryTable, int, int, uint32_t*) =
+    void (*k)(const uint8_t*, const float*, EntryTable, int, int, uint32_t*, long long, uint32_t*) =
         tab.S == 3 ? k_extrema_mask<5> : (tab.S == 4 ? k_extrema_mask<6> : k_extrema_mask<0>);
     if (smem > 48 * 1024 &&
         cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
         return -1;
-    if (launch_chained(k, grid, 256, smem, st, u8arena, lut255, tab, e, border, words) != cudaSuccess)
+    if (launch_chained(k, grid, 256, smem, st, u8arena, lut255, tab, e, border, words, od.word_base, tiles) !=
+        cudaSuccess)
         return -1;
     return cudaPeekAtLastError() == cudaSuccess ? 0 : -1;
 }
@@ -450,41 +481,33 @@ int extrema_tiles(int W, int H) {
 
 int launch_extrema_mask_flat(const uint8_t* u8arena, const float* lut255, const EntryTable& tab, int e0, int n_e,
                              const uint32_t* tile_pref, uint32_t n_tiles, int border, uint32_t* words,
-                             cudaStream_t st) {
+                             uint32_t* tiles, cudaStream_t st) {
     if (n_tiles == 0) return 0;
     if (tab.S + 2 > kExMaxLayers) return -1;
     const size_t smem = extrema_smem(tab.S);
-    void (*k)(const uint8_t*, const float*, EntryTable, int, int, const uint32_t*, int, uint32_t*) =
+    void (*k)(const uint8_t*, const float*, EntryTable, int, int, const uint32_t*, int, uint32_t*, long long, uint32_t*) =
         tab.S == 3 ? k_extrema_mask_flat<5> : (tab.S == 4 ? k_extrema_mask_flat<6> : k_extrema_mask_flat<0>);
     if (smem > 48 * 1024 &&
         cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
         return -1;
-    if (launch_chained(k, n_tiles, 256, smem, st, u8arena, lut255, tab, e0, n_e, tile_pref, border, words) !=
+    if (launch_chained(k, n_tiles, 256, smem, st, u8arena, lut255, tab, e0, n_e, tile_pref, border, words, 0ll, tiles) !=
         cudaSuccess)
         return -1;
     return cudaPeekAtLastError() == cudaSuccess ? 0 : -1;
 }
 
-int launch_emit(const uint8_t* u8arena, const float* lut255, const EntryTable& tab, int e0, int n_e,
-                long long n_words, const uint32_t* words, const uint32_t* cand_off, Keypoint* cands, uint32_t cap,
-                Counters* ctr, cudaStream_t st) {
+int launch_candidates(const uint8_t* u8arena, const float* lut255, const EntryTable& tab, float sigma, float contrast,
+                      float edge, int e0, int n_e, long long n_words, const uint32_t* words, const uint32_t* tiles,
+                      uint32_t* cand_off, Keypoint* cands, Keypoint* refined_at, uint32_t* keep, uint32_t cap,
+                      Counters* ctr, OctCounters* oc, cudaStream_t st) {
     if (n_words <= 0) return 0;
-    unsigned grid = (unsigned)((n_words + 255) / 256);
-    if (launch_chained(k_emit, grid, 256, 0, st, u8arena, lut255, tab, e0, n_e, n_words, words, cand_off, cands, cap,
-                       ctr) != cudaSuccess)
-        return -1;
-    return cudaPeekAtLastError() == cudaSuccess ? 0 : -1;
-}
-
-// Refinement is a chain of dependent scattered reads per candidate: up to
-// 5 CTAs of 8 warps per SM keep enough of them in flight.
-int launch_refine(const uint8_t* u8arena, const float* lut255, const EntryTable& tab, float sigma, float contrast,
-                  float edge, const Keypoint* cands, Keypoint* refined_at, uint32_t* keep, uint32_t cap,
-                  OctCounters* oc, cudaStream_t st) {
-    RefineParams rp{sigma, contrast, edge, tab.S, tab.S + 2};
-    const unsigned grid = (unsigned)std::min<size_t>(((size_t)cap + 255) / 256, 152 * 5);
-    if (launch_chained(k_refine, grid, 256, 0, st, u8arena, lut255, tab, rp, cands, refined_at, keep, cap, oc) !=
-        cudaSuccess)
+    const RefineParams rp{sigma, contrast, edge, tab.S, tab.S + 2};
+    const size_t n_tiles = word_tiles(n_words);
+    // a CTA per tile; of a very long list several, so that the sums over the
+    // tiles before stay a small part of the reads
+    const unsigned grid = (unsigned)std::min<size_t>(n_tiles, 8192);
+    if (launch_chained(k_candidates, grid, kCandThreads, 0, st, u8arena, lut255, tab, rp, e0, n_e, n_words, words,
+                       tiles, (uint32_t)n_tiles, cand_off, cands, refined_at, keep, cap, ctr, oc) != cudaSuccess)
         return -1;
     return cudaPeekAtLastError() == cudaSuccess ? 0 : -1;
 }

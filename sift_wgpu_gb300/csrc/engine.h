@@ -6,7 +6,7 @@
 //              plane pitch x H (pitch = width rounded up to 32 elements), f32
 //              or f16 (u8-valued either way)
 //   U arena    (S+3) u8 planes per octave: every level as bytes, the input
-//              of the next level, of the resize and of the extrema scan
+//              of the next level, of the resize and of the extrema mask
 //   tmp        one u8 plane for the horizontal blur pass (largest octave)
 //   ltmp       one f32 plane for the vertical Lanczos pass
 //   mask       per octave S x H x ceil(W/32) ballot words of extrema
@@ -57,8 +57,7 @@ int launch_lanczos(const uint8_t* src, int src_pitch, int W, int H, float* tmp, 
 int lanczos_fused_span();
 int lanczos_fused_tile();
 int pixel_channels(int format);
-int launch_begin(const RunCell* hcell, RunCell* cell, Counters* ctr, unsigned long long* scan, size_t n_scan,
-                 cudaStream_t st);
+int launch_begin(const RunCell* hcell, RunCell* cell, Counters* ctr, uint32_t* tiles, size_t n_tiles, cudaStream_t st);
 int launch_fetch(const uint8_t* src, long long stride, uint8_t* img, long long pitch, int W, int H, cudaStream_t st);
 int launch_export(const Counters* ctr, const Keypoint* kps, const RunCell* cell, cudaStream_t st);
 int launch_draw_keypoints(const uint8_t* d_gray, int stride, const Keypoint* d_kps, uint32_t n, uint8_t* d_rgb,
@@ -69,27 +68,26 @@ int launch_match(const float* d_q, uint32_t nq, const float* d_t, uint32_t nt, S
 int launch_to_luma(int format, const uint8_t* px, long long stride, int W, int H, uint8_t* out, long long out_pitch,
                    cudaStream_t st);
 int launch_extrema_mask(const uint8_t* u8arena, const float* lut255, const EntryTable& tab, const OctaveDev& od,
-                        int e, int border, uint32_t* words, cudaStream_t st);
+                        int e, int border, uint32_t* words, uint32_t* tiles, cudaStream_t st);
 int extrema_tiles(int W, int H);
 int launch_extrema_mask_flat(const uint8_t* u8arena, const float* lut255, const EntryTable& tab, int e0, int n_e,
                              const uint32_t* tile_pref, uint32_t n_tiles, int border, uint32_t* words,
-                             cudaStream_t st);
+                             uint32_t* tiles, cudaStream_t st);
 int launch_dog_dense(const uint8_t* u8arena, const float* lut255, const PyramidDev& pyr, int o, int l, float* out,
                      cudaStream_t st);
-int launch_emit(const uint8_t* u8arena, const float* lut255, const EntryTable& tab, int e0, int n_e,
-                long long n_words, const uint32_t* words, const uint32_t* cand_off, Keypoint* cands, uint32_t cap,
-                Counters* ctr, cudaStream_t st);
-int launch_refine(const uint8_t* u8arena, const float* lut255, const EntryTable& tab, float sigma, float contrast,
-                  float edge, const Keypoint* cands, Keypoint* refined_at, uint32_t* keep, uint32_t cap,
-                  OctCounters* oc, cudaStream_t st);
+int launch_candidates(const uint8_t* u8arena, const float* lut255, const EntryTable& tab, float sigma, float contrast,
+                      float edge, int e0, int n_e, long long n_words, const uint32_t* words, const uint32_t* tiles,
+                      uint32_t* cand_off, Keypoint* cands, Keypoint* refined_at, uint32_t* keep, uint32_t cap,
+                      Counters* ctr, OctCounters* oc, cudaStream_t st);
 size_t ori_bins_bytes();
 int launch_ori_bins(uint8_t* bins, cudaStream_t st);
 int launch_orientation(const uint8_t* u8arena, const EntryTable& tab, const float* lut255, const uint8_t* bins,
                        const Keypoint* refined_at, const uint32_t* keep, uint32_t ncap, OctCounters* oc,
-                       float* ori_angle, uint32_t* ori_count, int grid, int persist_ctas, cudaStream_t st);
-int launch_orient_emit(const Keypoint* refined_at, uint32_t ncap, int o, Counters* ctr, const float* ori_angle,
-                       const uint32_t* ori_count, const uint32_t* ori_off, Keypoint* oriented, uint32_t cap,
+                       float* ori_angle, uint32_t* ori_count, uint32_t* tiles, int grid, int persist_ctas,
                        cudaStream_t st);
+int launch_orient_emit(const Keypoint* refined_at, uint32_t ncap, int o, Counters* ctr, const float* ori_angle,
+                       const uint32_t* ori_count, const uint32_t* tiles, uint32_t* ori_off, Keypoint* oriented,
+                       uint32_t cap, cudaStream_t st);
 int launch_descriptor(const uint8_t* u8arena, const EntryTable& tab, const Keypoint* oriented, OctCounters* oc,
                       float* desc, uint32_t cap, const RunCell* cell, int grid, int persist_ctas, cudaStream_t st);
 // Error reporting (engine.cu): the calling thread's sift_cuda_last_error.
@@ -269,11 +267,11 @@ struct Engine {
 
     // Lists. Octave o owns [cb[o], cb[o] + cap_c[o]) of the candidate-sized
     // lists (candidates, refined, keep flags, orientation scratch) and its own
-    // scan scratch; the output lists (oriented keypoints, descriptors) are
+    // tile counts; the output lists (oriented keypoints, descriptors) are
     // shared, octave after octave.
     std::vector<uint32_t> cap_c, cb;
-    std::vector<size_t> pb, tb;  // scan-state (64-bit words) and horizontal-pass buffer offsets
-    size_t scan_words = 0;       // scan state of the run, zeroed at its start
+    std::vector<size_t> pb, tb;  // tile-count and horizontal-pass buffer offsets
+    size_t n_tiles = 0;          // tile counts of the run, zeroed at its start
     uint32_t cap_cand = 0, cap_ori = 0;
 
     DevMem d_bins;  // orientation bins of byte difference pairs
@@ -282,10 +280,10 @@ struct Engine {
     HostPinned h_mo;          // its results: error word, matches from byte 256 on
     DevMem d_dg, d_dk, d_drgb;       // drawing: grey input, keypoints, RGB output
     DevMem d_img, d_G, d_U, d_tmp, d_tmpo, d_ltmp, d_wts, d_ltab, d_lw;
-    DevMem d_words, d_cand_off, d_keep, d_scan;
+    DevMem d_words, d_keep, d_tiles;
     DevMem d_ents;  // the entry table: pyr.oct[0 .. num_octaves) in device memory
     EntryTable tab() const { return EntryTable{d_ents.as<OctaveDev>(), pyr.num_octaves, pyr.S}; }
-    DevMem d_cands, d_refined_at, d_ori_angle, d_ori_count, d_ori_off, d_oriented, d_desc, d_ctr;
+    DevMem d_cands, d_refined_at, d_ori_angle, d_ori_count, d_oriented, d_desc, d_ctr;
     HostPinned h_ctr, h_kps, h_desc;
     // Host calls: the run ends with an export kernel that writes counters and
     // keypoints into this buffer (the descriptor stage its descriptors),
@@ -330,7 +328,7 @@ struct Engine {
     // One stream per octave for the level DAG and its events (see enqueue_t),
     // and the CUDA graph the whole run is replayed from.
     std::vector<cudaStream_t> st_oct;
-    std::vector<cudaEvent_t> ev_level, ev_ori, ev_done;
+    std::vector<cudaEvent_t> ev_level, ev_emit, ev_done;
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t gexec = nullptr;
     struct GraphKey {
@@ -371,7 +369,7 @@ struct Engine {
         for (auto& r : ev_runs)
             for (auto e : r) cudaEventDestroy(e);
         for (auto e : ev_free) cudaEventDestroy(e);
-        for (auto* v : {&ev_level, &ev_ori, &ev_done})
+        for (auto* v : {&ev_level, &ev_emit, &ev_done})
             for (auto e : *v)
                 if (e) cudaEventDestroy(e);
         for (auto q : st_oct)
@@ -430,8 +428,8 @@ struct Engine {
     size_t device_bytes() const {
         size_t t = 0;
         for (const DevMem* m : {&d_img, &d_G, &d_U, &d_tmp, &d_tmpo, &d_ltmp, &d_wts, &d_ltab, &d_lw, &d_words,
-                                &d_cand_off, &d_keep, &d_scan, &d_cands, &d_refined_at,
-                                &d_ori_angle, &d_ori_count, &d_ori_off, &d_oriented, &d_desc, &d_ctr})
+                                &d_keep, &d_tiles, &d_cands, &d_refined_at,
+                                &d_ori_angle, &d_ori_count, &d_oriented, &d_desc, &d_ctr})
             t += m->bytes;
         return t;
     }
@@ -459,7 +457,7 @@ struct Engine {
         for (size_t o = 0; o < st_oct.size(); ++o)
             CK(cudaStreamCreateWithPriority(&st_oct[o], cudaStreamNonBlocking, o == 0 ? base : urgent),
                "cudaStreamCreate");
-        for (auto* v : {&ev_level, &ev_ori, &ev_done}) {
+        for (auto* v : {&ev_level, &ev_emit, &ev_done}) {
             v->assign(kMaxOctaves, nullptr);
             for (auto& e : *v) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "cudaEventCreate");
         }
@@ -597,7 +595,6 @@ struct Engine {
         if (O > 0)
             CK(cudaMemcpyAsync(d_ents.p, g.oct, sizeof(OctaveDev) * (size_t)O, cudaMemcpyHostToDevice, st),
                "H2D entries");
-        CK(d_cand_off.ensure(nwb), "cudaMalloc(cand_off)");
         if (!wts.empty())
             CK(cudaMemcpyAsync(d_wts.p, wts.data(), wts.size() * sizeof(float), cudaMemcpyHostToDevice, st), "H2D wts");
         if (!itab.empty())
@@ -637,11 +634,11 @@ struct Engine {
         for (int o = 0; o < O; ++o) {
             cb[o] = (uint32_t)c;
             c += cap_c[o];
-            // two scans per octave: the candidate words, then the orientation counts
+            // the octave's tiles: of its mask words, then of its candidate slots
             pb[o] = pp;
-            pp += scan_state_words((size_t)octave_words(o)) + scan_state_words((size_t)cap_c[o]);
+            pp += word_tiles(octave_words(o)) + slot_tiles(cap_c[o]);
         }
-        scan_words = pp;
+        n_tiles = pp;
         if (c > (1u << 30)) return fail(SIFT_CUDA_ERR_CAPACITY, "keypoint lists above 2^30");
         cap_cand = (uint32_t)c;
         const size_t kp = sizeof(Keypoint);
@@ -649,11 +646,10 @@ struct Engine {
         CK(d_refined_at.ensure((size_t)cap_cand * kp), "cudaMalloc(refined_at)");
         CK(d_ori_angle.ensure((size_t)cap_cand * kOriMaxPeaks * sizeof(float)), "cudaMalloc(ori_angle)");
         CK(d_ori_count.ensure((size_t)cap_cand * sizeof(uint32_t)), "cudaMalloc(ori_count)");
-        CK(d_ori_off.ensure((size_t)cap_cand * sizeof(uint32_t)), "cudaMalloc(ori_off)");
         CK(d_keep.ensure((size_t)cap_cand * sizeof(uint32_t)), "cudaMalloc(keep)");
         CK(d_oriented.ensure((size_t)cap_ori * kp), "cudaMalloc(oriented)");
         CK(d_desc.ensure((size_t)cap_ori * kDescLen * sizeof(float)), "cudaMalloc(desc)");
-        CK(d_scan.ensure(std::max<size_t>(pp, 1) * sizeof(unsigned long long)), "cudaMalloc(scan state)");
+        CK(d_tiles.ensure(align_up(std::max<size_t>(pp, 1), 4) * sizeof(uint32_t)), "cudaMalloc(tile counts)");
         return 0;
     }
 
@@ -683,7 +679,7 @@ struct Engine {
         std::vector<cudaEvent_t> run_ev;
         mark(&run_ev);
         const RunCell* rc = d_cell.as<RunCell>();
-        if (ok(launch_begin(h_cell_dev, d_cell.as<RunCell>(), ctr, d_scan.as<unsigned long long>(), scan_words, st)))
+        if (ok(launch_begin(h_cell_dev, d_cell.as<RunCell>(), ctr, d_tiles.as<uint32_t>(), n_tiles, st)))
             return cuda_fail(cudaGetLastError(), "run start");
         int O_used = 0;
         for (int o = 0; o < O && pyr.oct[o].W > 0 && pyr.oct[o].H > 0; ++o) O_used = o + 1;
@@ -722,31 +718,23 @@ struct Engine {
             launches += nl;
             return 0;
         };
+        auto slots = [&](int o) { return d_tiles.as<uint32_t>() + pb[o] + word_tiles(octave_words(o)); };
         // (b)+(c): extrema, ordered candidates, refinement of octave o
         auto detect = [&](int o, cudaStream_t q) -> int {
             const OctaveDev& od = pyr.oct[o];
             OctCounters* oc = &ctr->oct[o];
-            unsigned long long* sstate = d_scan.as<unsigned long long>() + pb[o];
-            const long long nwo = octave_words(o);
+            uint32_t* tiles = d_tiles.as<uint32_t>() + pb[o];
             if (od.nw > 0 && ok(launch_extrema_mask(U, lut, tab(), od, o, (int)p.image_border_width,
-                                                    d_words.as<uint32_t>(), q)))
+                                                    d_words.as<uint32_t>(), tiles, q)))
                 return cuda_fail(cudaGetLastError(), "extrema mask");
-            if (scan_exclusive(d_words.as<uint32_t>() + od.word_base, SCAN_POPC,
-                               d_cand_off.as<uint32_t>() + od.word_base, (size_t)nwo, nullptr, &oc->n_cand, sstate,
-                               &ctr->overflow, q))
-                return cuda_fail(cudaGetLastError(), "scan candidates");
-            launches += nwo > 0 ? 1 : 0;
-            if (ok(launch_emit(U, lut, tab(), o, 1, nwo, d_words.as<uint32_t>() + od.word_base,
-                               d_cand_off.as<uint32_t>() + od.word_base, d_cands.as<Keypoint>() + cb[o], cap_c[o], ctr,
-                               q)))
-                return cuda_fail(cudaGetLastError(), "emit");
-            if (ok(launch_refine(U, lut, tab(), p.sigma, p.contrast_threshold, p.edge_threshold,
-                                 d_cands.as<Keypoint>() + cb[o], d_refined_at.as<Keypoint>() + cb[o],
-                                 d_keep.as<uint32_t>() + cb[o], cap_c[o], oc, q)))
-                return cuda_fail(cudaGetLastError(), "refine");
+            if (od.nw > 0 && ok(launch_candidates(U, lut, tab(), p.sigma, p.contrast_threshold, p.edge_threshold, o, 1,
+                                                  octave_words(o), d_words.as<uint32_t>() + od.word_base, tiles, nullptr,
+                                                  d_cands.as<Keypoint>() + cb[o], d_refined_at.as<Keypoint>() + cb[o],
+                                                  d_keep.as<uint32_t>() + cb[o], cap_c[o], ctr, oc, q)))
+                return cuda_fail(cudaGetLastError(), "candidates");
             return 0;
         };
-        // (d) orientation histograms of the kept candidate slots and their scan
+        // (d) orientation histograms of the kept candidate slots
         auto orient = [&](int o, cudaStream_t q) -> int {
             OctCounters* oc = &ctr->oct[o];
             // one warp-item per 8 candidate slots, 4 per warp; the last
@@ -754,22 +742,16 @@ struct Engine {
             const int grid = (int)std::max<uint32_t>(cap_c[o] / 64, 32);
             if (ok(launch_orientation(U, tab(), lut, d_bins.as<uint8_t>(), d_refined_at.as<Keypoint>() + cb[o], d_keep.as<uint32_t>() + cb[o],
                                           cap_c[o], oc, d_ori_angle.as<float>() + (size_t)cb[o] * kOriMaxPeaks,
-                                          d_ori_count.as<uint32_t>() + cb[o], grid, 152 * tune.ori_ctas_per_sm, q)))
+                                          d_ori_count.as<uint32_t>() + cb[o], slots(o), grid, 152 * tune.ori_ctas_per_sm, q)))
                 return cuda_fail(cudaGetLastError(), "orientation");
-            unsigned long long* sstate =
-                d_scan.as<unsigned long long>() + pb[o] + scan_state_words((size_t)octave_words(o));
-            if (scan_exclusive(d_ori_count.as<uint32_t>() + cb[o], SCAN_U32, d_ori_off.as<uint32_t>() + cb[o],
-                               (size_t)cap_c[o], &oc->n_cand, &oc->n_ori, sstate, &ctr->overflow, q))
-                return cuda_fail(cudaGetLastError(), "scan orientations");
-            launches += 1;
             return 0;
         };
         // output slots of octave o (after octaves 0..o-1) and its descriptors
         auto emit_out = [&](int o, cudaStream_t q) -> int {
             if (ok(launch_orient_emit(d_refined_at.as<Keypoint>() + cb[o], cap_c[o], o, ctr,
                                       d_ori_angle.as<float>() + (size_t)cb[o] * kOriMaxPeaks,
-                                      d_ori_count.as<uint32_t>() + cb[o], d_ori_off.as<uint32_t>() + cb[o],
-                                      d_oriented.as<Keypoint>(), cap_ori, q)))
+                                      d_ori_count.as<uint32_t>() + cb[o], slots(o), nullptr, d_oriented.as<Keypoint>(), cap_ori,
+                                      q)))
                 return cuda_fail(cudaGetLastError(), "orientation emit");
             return 0;
         };
@@ -815,9 +797,10 @@ struct Engine {
                     if (int rc = level(o, s, q, tmp_o)) return rc;
                 if (int rc = detect(o, q)) return rc;
                 if (int rc = orient(o, q)) return rc;
-                CK(cudaEventRecord(ev_ori[o], q), "event record");
-                for (int k = 0; k < o; ++k) CK(cudaStreamWaitEvent(q, ev_ori[k], 0), "stream wait");
+                // (which waited for those before it)
+                if (o > 0) CK(cudaStreamWaitEvent(q, ev_emit[o - 1], 0), "stream wait");
                 if (int rc = emit_out(o, q)) return rc;
+                CK(cudaEventRecord(ev_emit[o], q), "event record");
                 if (int rc = describe(o, q)) return rc;
                 CK(cudaEventRecord(ev_done[o], q), "event record");
                 if (o + 1 < O_used)
@@ -977,7 +960,6 @@ struct Engine {
     // *retry tells that the run must be repeated.
     int grow_from(const Counters& c, bool* retry) {
         *retry = false;
-        if (c.overflow & 8u) return fail(SIFT_CUDA_ERR_CUDA, "a prefix-scan wait ran out (the run was abandoned)");
         bool grow = false;
         for (int o = 0; o < pyr.num_octaves; ++o) {
             const uint32_t n = c.oct[o].n_cand;

@@ -2,7 +2,7 @@
 //
 // k_begin starts a run: it copies the run's cell (RunCell: where the image is,
 // where the results go) from mapped host memory to device memory and zeroes
-// the counters and the scan state. It takes the place of two memset nodes of
+// the counters and the tile counts. It takes the place of two memset nodes of
 // the graph (a 160 x 120 frame 176 -> 162 us); launched ahead of the graph
 // with the cell as a parameter the frame took 174 us.
 //
@@ -56,14 +56,16 @@ __device__ __forceinline__ uint4 load16(const uint8_t* p, int n) {
 // One CTA. The cell is read past the caches: the host rewrites it between runs.
 __global__ void __launch_bounds__(kBeginThreads) k_begin(const RunCell* hcell, RunCell* __restrict__ cell,
                                                          Counters* __restrict__ ctr,
-                                                         unsigned long long* __restrict__ scan, uint32_t n_scan) {
+                                                         uint32_t* __restrict__ tiles, uint32_t n_tiles) {
     chain_wait();
     const int tid = threadIdx.x;
     constexpr int kWords = sizeof(RunCell) / 4;
     uint32_t v = 0;
     if (tid < kWords) v = __ldcv(reinterpret_cast<const uint32_t*>(hcell) + tid);
     for (uint32_t i = tid; i < sizeof(Counters) / 4; i += kBeginThreads) reinterpret_cast<uint32_t*>(ctr)[i] = 0u;
-    for (uint32_t i = tid; i < n_scan; i += kBeginThreads) scan[i] = 0ull;
+    // (an allocation of whole 16-byte words)
+    for (uint32_t i = tid; i < (n_tiles + 3) / 4; i += kBeginThreads)
+        reinterpret_cast<uint4*>(tiles)[i] = make_uint4(0u, 0u, 0u, 0u);
     if (tid < kWords) reinterpret_cast<uint32_t*>(cell)[tid] = v;
 }
 
@@ -107,9 +109,8 @@ __global__ void __launch_bounds__(256) k_export(const Counters* __restrict__ ctr
 
 }  // namespace
 
-int launch_begin(const RunCell* hcell, RunCell* cell, Counters* ctr, unsigned long long* scan, size_t n_scan,
-                 cudaStream_t st) {
-    if (launch_chained(k_begin, 1, kBeginThreads, 0, st, hcell, cell, ctr, scan, (uint32_t)n_scan) != cudaSuccess)
+int launch_begin(const RunCell* hcell, RunCell* cell, Counters* ctr, uint32_t* tiles, size_t n_tiles, cudaStream_t st) {
+    if (launch_chained(k_begin, 1, kBeginThreads, 0, st, hcell, cell, ctr, tiles, (uint32_t)n_tiles) != cudaSuccess)
         return -1;
     return cudaPeekAtLastError() == cudaSuccess ? 0 : -1;
 }

@@ -42,7 +42,7 @@ struct Counters {
     uint32_t n_candidates;  // totals (filled by the last octave's chain)
     uint32_t n_refined;
     uint32_t n_oriented;    // keypoints in the output
-    uint32_t overflow;      // bit 0 candidates, 2 oriented, 8 a scan wait ran out
+    uint32_t overflow;      // bit 0 candidates, 2 oriented
     uint32_t pad[4];
     OctCounters oct[kMaxOctaves];
 };
@@ -367,14 +367,11 @@ inline cudaError_t launch_chained(void (*k)(KArgs...), dim3 grid, dim3 block, si
     return cudaLaunchKernelEx(&cfg, k, static_cast<KArgs>(args)...);
 }
 
-// Scan helpers (scan.cu).
-enum ScanInput { SCAN_U32 = 0, SCAN_POPC = 1 };
-// Exclusive scan of n values in one launch (n_dev, when not null, overrides n
-// at run time and must be <= n). total_out receives the sum. state holds
-// scan_state_words(n) 64-bit words that must be zero when the scan starts;
-// a look-back wait that runs out sets bit 8 of *err.
-size_t scan_state_words(size_t n);
-int scan_exclusive(const uint32_t* in, ScanInput mode, uint32_t* out, size_t n, const uint32_t* n_dev,
-                   uint32_t* total_out, unsigned long long* state, uint32_t* err, cudaStream_t st);
+// Tiles of the two ordered lists (tile_scan.cuh): mask words by the candidates
+// in them, candidate slots by their oriented keypoints. One 32-bit count per
+// tile, zero at a run's start, filled by the extrema mask and the orientation.
+constexpr int kWordTile = 512, kSlotTile = 256;
+inline size_t word_tiles(long long words) { return (size_t)((words + kWordTile - 1) / kWordTile); }
+inline size_t slot_tiles(uint32_t slots) { return ((size_t)slots + kSlotTile - 1) / kSlotTile; }
 
 }  // namespace sift
