@@ -442,7 +442,7 @@ struct BatchEngine {
         CK(cudaStreamWaitEvent(st, ev_side, 0), "stream wait");
         // detection over every entry
         uint32_t *tiles = d_tiles.as<uint32_t>(), *slots = tiles + slots_at;
-        if (int rc = bump(launch_extrema_mask_flat(U, lut, tb, 0, N * O, pref(ex_pref), n_ex, (int)p.image_border_width,
+        if (int rc = bump(launch_extrema_mask_flat(U, tb, 0, N * O, pref(ex_pref), n_ex, (int)p.image_border_width,
                                                    d_words.as<uint32_t>(), tiles, st),
                           "batch extrema"))
             return rc;

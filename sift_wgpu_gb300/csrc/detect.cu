@@ -20,6 +20,8 @@
 // candidates and refined keypoints are bit-identical to the CPU path; the one
 // transcendental, 2^(octave + layer/S) for the keypoint size, is evaluated in
 // f64 and rounded once.
+#include <cuda_fp16.h>
+
 #include <algorithm>
 
 #include "tile_scan.cuh"
@@ -46,131 +48,230 @@ struct DogFromU8 {
     }
 };
 
-// DoG staged from the u8 copies of the Gaussian levels of one octave:
-// D_l = lut[G_{l+1}] - lut[G_l] with lut[v] = v/255 in f32, which is the
-// reference's f32 DoG bit for bit (src/sift.rs:92-124) at a quarter of the
-// bytes.
-// Stages layers 0..L-1 of the clamped window [x0, x0+TW) x [y0, y0+TH) into
-// tile[L][TH][TW]; windows inside the plane go as aligned 4-byte words, all
-// L+1 levels of a word per thread.
-__device__ __forceinline__ void stage_dog_u8(float* tile, const float* lut, const uint8_t* base, long long plane,
-                                             int pitch, int W, int H, int L, int x0, int y0, int TW, int TH, int tid,
-                                             int nthreads) {
-    const bool inner = x0 >= 0 && y0 >= 0 && x0 + TW <= W && y0 + TH <= H && (x0 & 3) == 0 && (TW & 3) == 0 &&
-                       (pitch & 3) == 0;
-    if (inner) {
-        const int q4 = TW >> 2;
-        for (int q = tid; q < TH * q4; q += nthreads) {
-            const int yy = q / q4, xx = (q - yy * q4) * 4;
-            const uint8_t* p = base + (long long)(y0 + yy) * pitch + x0 + xx;
-            const unsigned b0 = *reinterpret_cast<const unsigned*>(p);
-            float lo0 = lut[b0 & 0xffu], lo1 = lut[(b0 >> 8) & 0xffu], lo2 = lut[(b0 >> 16) & 0xffu],
-                  lo3 = lut[b0 >> 24];
-            float* t = tile + yy * TW + xx;
-#pragma unroll 4
-            for (int l = 0; l < L; ++l) {
-                const unsigned b = *reinterpret_cast<const unsigned*>(p + (long long)(l + 1) * plane);
-                const float u0 = lut[b & 0xffu], u1 = lut[(b >> 8) & 0xffu], u2 = lut[(b >> 16) & 0xffu],
-                            u3 = lut[b >> 24];
-                *reinterpret_cast<float4*>(t + (size_t)l * TH * TW) =
-                    make_float4(__fsub_rn(u0, lo0), __fsub_rn(u1, lo1), __fsub_rn(u2, lo2), __fsub_rn(u3, lo3));
-                lo0 = u0;
-                lo1 = u1;
-                lo2 = u2;
-                lo3 = u3;
+// ---------------------------------------------------------------------------
+// Extrema of one octave, all layers s = 1..S at once:
+//   strict max  <=>  v > max(M_{s-1}, M_{s+1}, ring8max_s)
+//   strict min  <=>  v < min(m_{s-1}, m_{s+1}, ring8min_s)
+// with M, m the 3 x 3 block's max and min, which is the reference's 26 strict
+// comparisons (ties reject) of f32 DoG values.
+//
+// Only their order matters, and 16 bits hold it: two pixels go through every
+// operation, three-way minima and maxima included, in one register. With h(v)
+// the highest power of two in v (h(0) = 0), v / 255 in f32 is
+//   (v * 0x808080 + h(v)) * 2^-31,
+// (its binary digits repeat v's eight, and the bit after the 24th from the
+// first one is always 1), so the DoG value of bytes a and b is the f32 rounding
+// of (d * 0x808080 + h(a) - h(b)) * 2^-31, d = a - b. Where a <= 2 b and b <=
+// 2 a the subtraction is exact and |h(a) - h(b)| <= 64: the key
+//   128 d + h(a) - h(b) = T(a) - T(b),  T(v) = 128 v + h(v)
+// orders the values, equal keys for equal values only. Elsewhere (a dark pixel
+// beside a much brighter one in the next level) exact_key makes the key of the
+// rounded difference; with it, the order of the keys of all 65 536 pairs is
+// that of their f32 values.
+//
+// A CTA stages the keys of its 128 x 16 pixels and their neighbours for every
+// DoG layer 0..S+1 in shared memory (clamped coordinates, as get_pixel_value
+// clamps, at the image border), word i of a row the pixels x0 - 4 + i and
+// x0 + 60 + i. Each thread owns one such pair of columns and 4 rows: per layer
+// it forms the horizontal 3-max/3-min of 6 rows once and reuses them for the
+// block max/min and the ring max/min of its 8 pixels; a ballot of either half
+// is a word of the mask.
+//
+// The integer pipe bounds it (64 lanes per clock and SM for each of these
+// operations, the three-way ones too). Octave 0 takes 79 us at 4096 x 4096 and
+// 16 at 1080p; with f32 values, one pixel each, of a table in shared memory
+// (64 x 16 tiles) it took 169 and 26. The stage: 351 -> 231 us and 91 -> 79.
+// The rounded keys cost 4 us of the 79;
+// 3 CTAs per SM, which spill nothing, take 9 % more than 4.
+constexpr int kExTX = 128, kExTY = 16, kExRows = 4, kExMaxLayers = 18, kExThreads = 256;
+constexpr int kExHalf = kExTX / 2;
+constexpr int kExSW = kExHalf + 8;  // staged words of a row: pairs from x0 - 4 on
+constexpr int kExSH = kExTY + 2;
+constexpr uint32_t kExBias = 0x80008000u;
+
+// The key of level bytes a (of the layer's upper level) and b, plus 0x8000, in
+// the low 16 bits: v / 255 in units of 2^-31, its f32 difference, and what that
+// has beyond d * 0x808080 (every step but the difference is exact).
+__device__ __forceinline__ uint32_t exact_key(uint32_t a, uint32_t b) {
+    constexpr float k255 = 8421504.0f;  // 0x808080
+    const float af = (float)a, bf = (float)b;
+    const float ha = __uint_as_float(__float_as_uint(af) & 0x7F800000u), hb = __uint_as_float(__float_as_uint(bf) & 0x7F800000u);
+    const float diff = __fsub_rn(fmaf(af, k255, ha), fmaf(bf, k255, hb));
+    const float d = af - bf;
+    float e = fmaf(-d, k255, diff);
+    if (fabsf(e) == 128.0f) e = copysignf(100.0f, e);  // (others are at most 64; the next d's key starts at 128)
+    return __float_as_uint(fmaf(d, 128.0f, e) + (8388608.0f + 32768.0f));
+}
+
+// A pair of level bytes, in three forms: as f16 numbers, and their T up to a
+// constant.
+struct ExPair {
+    __half2 v;
+    uint32_t t;
+};
+// raw: the bytes below 0x64, i.e. 1024 + v as f16
+__device__ __forceinline__ ExPair ex_pair(uint32_t raw) {
+    const __half2 k1024 = __half2half2(__ushort_as_half(0x6400));
+    ExPair p;
+    p.v = __hsub2(*reinterpret_cast<const __half2*>(&raw), k1024);
+    // the exponent bits alone are h(v)
+    const uint32_t h = *reinterpret_cast<const uint32_t*>(&p.v) & 0x7C007C00u;
+    const __half2 hk = __hadd2(*reinterpret_cast<const __half2*>(&h), k1024);
+    p.t = raw * 128u + *reinterpret_cast<const uint32_t*>(&hk);
+    return p;
+}
+
+// Four bytes of a row, from x on (clamped coordinates).
+__device__ __forceinline__ uint32_t clamped_word(const uint8_t* row, int x, int W) {
+    uint32_t w = 0;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) w |= (uint32_t)row[clampi(x + k, 0, W - 1)] << (8 * k);
+    return w;
+}
+
+// Stages layers 0 .. L - 1 of the tile: an item is four words of a row, all
+// levels of it.
+template <int NL>
+__device__ __forceinline__ void stage_keys(uint32_t* tile, const uint8_t* base, long long plane, int pitch, int W,
+                                           int H, int L, int x0, int y0) {
+    constexpr int kChunks = kExSW / 4;
+    for (int q = threadIdx.x; q < kExSH * kChunks; q += kExThreads) {
+        const int yy = q / kChunks, c = q - yy * kChunks, x = x0 - 4 + 4 * c;
+        const uint8_t* row = base + (long long)clampi(y0 - 1 + yy, 0, H - 1) * pitch;
+        uint32_t* out = tile + yy * kExSW + 4 * c;
+        const bool whole = x >= 0 && x + kExHalf + 4 <= W;
+        auto word = [&](const uint8_t* r, int xx) {
+            return whole ? *reinterpret_cast<const uint32_t*>(r + xx) : clamped_word(r, xx, W);
+        };
+        ExPair prev[4];
+        uint32_t unsafe = 0;  // a bit for each layer
+        auto level = [&](int l, uint32_t lo, uint32_t hi) {
+            const uint32_t a = __byte_perm(lo, hi, 0x5140u), b = __byte_perm(lo, hi, 0x7362u);
+            const ExPair p[4] = {ex_pair(__byte_perm(a, 0x64646464u, 0x4140u)), ex_pair(__byte_perm(a, 0x64646464u, 0x4342u)),
+                                 ex_pair(__byte_perm(b, 0x64646464u, 0x4140u)), ex_pair(__byte_perm(b, 0x64646464u, 0x4342u))};
+            if (l > 0) {
+                const __half2 two = __half2half2(__ushort_as_half(0x4000));
+                uint32_t key[4], bad = 0;
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    key[k] = p[k].t + kExBias - prev[k].t;
+                    const __half2 s = __hfma2(two, p[k].v, __hneg2(prev[k].v)), t = __hfma2(two, prev[k].v, __hneg2(p[k].v));
+                    bad |= *reinterpret_cast<const uint32_t*>(&s) | *reinterpret_cast<const uint32_t*>(&t);
+                }
+                if (bad & kExBias) unsafe |= 1u << (l - 1);
+                *reinterpret_cast<uint4*>(out + (l - 1) * kExSH * kExSW) = make_uint4(key[0], key[1], key[2], key[3]);
             }
+#pragma unroll
+            for (int k = 0; k < 4; ++k) prev[k] = p[k];
+        };
+        if constexpr (NL > 0) {
+            uint32_t lo[NL + 1], hi[NL + 1];  // all reads first
+            if (whole) {
+                const uint8_t* src = row + x;
+#pragma unroll
+                for (int l = 0; l <= NL; ++l, src += plane) {
+                    lo[l] = *reinterpret_cast<const uint32_t*>(src);
+                    hi[l] = *reinterpret_cast<const uint32_t*>(src + kExHalf);
+                }
+            } else {
+                const uint8_t* src = row;
+#pragma unroll
+                for (int l = 0; l <= NL; ++l, src += plane) {
+                    lo[l] = clamped_word(src, x, W);
+                    hi[l] = clamped_word(src, x + kExHalf, W);
+                }
+            }
+#pragma unroll
+            for (int l = 0; l <= NL; ++l) level(l, lo[l], hi[l]);
+        } else {
+            const uint8_t* src = row;
+#pragma unroll 1
+            for (int l = 0; l <= L; ++l, src += plane) level(l, clamped_word(src, x, W), clamped_word(src, x + kExHalf, W));
         }
-    } else {
-        for (int q = tid; q < TH * TW; q += nthreads) {
-            const int yy = q / TW, xx = q - yy * TW;
-            const long long o = (long long)clampi(y0 + yy, 0, H - 1) * pitch + clampi(x0 + xx, 0, W - 1);
-            float lo = lut[base[o]];
-            for (int l = 0; l < L; ++l) {
-                const float up = lut[base[(long long)(l + 1) * plane + o]];
-                tile[(l * TH + yy) * TW + xx] = __fsub_rn(up, lo);
-                lo = up;
-            }
+#pragma unroll 1
+        for (; unsafe; unsafe &= unsafe - 1u) {
+            const int l = __ffs(unsafe) - 1;
+            const uint8_t *b = row + l * plane, *a = b + plane;
+            const uint32_t al = word(a, x), ah = word(a, x + kExHalf), bl = word(b, x), bh = word(b, x + kExHalf);
+            uint32_t key[4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+                key[k] = __byte_perm(exact_key(al >> (8 * k) & 255u, bl >> (8 * k) & 255u),
+                                     exact_key(ah >> (8 * k) & 255u, bh >> (8 * k) & 255u), 0x5410u);
+            *reinterpret_cast<uint4*>(out + l * kExSH * kExSW) = make_uint4(key[0], key[1], key[2], key[3]);
         }
     }
 }
 
-// ---------------------------------------------------------------------------
-// Extrema of one octave, all layers s = 1..S at once. The CTA stages the
-// neighbourhood of its 64 x 16 pixels for every DoG layer 0..S+1 in shared
-// memory, formed from the u8 levels (clamped coordinates, as get_pixel_value
-// clamps, at the image border). Each thread owns one column and 4 rows: per
-// layer it forms the horizontal 3-max/3-min of 6 rows once and reuses them for
-// the 3x3 block max/min and the 8-ring max/min of its 4 pixels:
-//   strict max  <=>  v > max(M_{s-1}, M_{s+1}, ring8max_s)
-//   strict min  <=>  v < min(m_{s-1}, m_{s+1}, ring8min_s)
-// which is the reference's 26 strict comparisons (ties reject).
-constexpr int kExTX = 64, kExTY = 16, kExRows = 4, kExMaxLayers = 18;
-constexpr int kExSW = kExTX + 8;  // staged width: x0-4 .. x0+68 (word aligned)
-constexpr int kExSH = kExTY + 2;
-
 // NL > 0: the number of DoG layers (S + 2) is compiled in and the layer loop
 // unrolls, so the sliding window renames registers instead of moving them;
-// NL == 0: any S.
+// NL == 0: any S. The candidates are counted by tiles of kWordTile words, from
+// word0 on.
 template <int NL>
-__device__ __forceinline__ void extrema_tile(const uint8_t* __restrict__ u8arena, const float* __restrict__ lut255,
-                                             const OctaveDev& od, int S, int border, uint32_t* __restrict__ words,
-                                             long long word0, uint32_t* __restrict__ tiles, int x0, int y0,
-                                             float* tile) {
+__device__ __forceinline__ void extrema_tile(const uint8_t* __restrict__ u8arena, const OctaveDev& od, int S,
+                                             int border, uint32_t* __restrict__ words, long long word0,
+                                             uint32_t* __restrict__ tiles, int x0, int y0, uint32_t* tile) {
     const int W = od.W, H = od.H, nw = od.nw, L = NL > 0 ? NL : S + 2;
     const int tid = threadIdx.x, lane = tid & 31;
-    float* lut = tile + L * kExSH * kExSW;
-    lut[tid] = lut255[tid];
+    stage_keys<NL>(tile, u8arena + od.u_off, od.plane, od.pitch, W, H, L, x0, y0);
     __syncthreads();
-    stage_dog_u8(tile, lut, u8arena + od.u_off, od.plane, od.pitch, W, H, L, x0 - 4, y0 - 1, kExSW, kExSH, tid, 256);
-    __syncthreads();
-    const int col = tid & (kExTX - 1);          // 0..63
-    const int r0 = (tid >> 6) * kExRows;       // 0, 4, 8, 12
-    const int x = x0 + col;
-    const int tx = col + 4;                     // staged column of x
-    const int word = (x0 >> 5) + ((tid >> 5) & 1);  // this warp's 32 columns
-    const bool xin = x >= border && x < W - border;
-    bool yin[kExRows];
+    const int i = tid & (kExHalf - 1);                 // columns x0 + i and x0 + 64 + i
+    const int r0 = (tid / kExHalf) * kExRows;          // 0, 4, 8, 12
+    // lanes 0 .. 7 write: row r0 + lane / 2, the low halves' word (even) or the high halves'
+    const int wrow = y0 + r0 + (lane >> 1 & 3), word = (x0 >> 5) + (i >> 5) + 2 * (lane & 1);
+    const bool writes = lane < 2 * kExRows && wrow < H && word < nw;
+    long long at = od.word_base + (long long)wrow * nw + word;
+    auto in_x = [&](int x) { return x >= border && x < W - border; };
+    const uint32_t columns = (in_x(x0 + i) ? 0x0000ffffu : 0u) | (in_x(x0 + kExHalf + i) ? 0xffff0000u : 0u);
+    uint32_t rows = 0;  // a bit for each row that may hold candidates
 #pragma unroll
-    for (int j = 0; j < kExRows; ++j) yin[j] = xin && y0 + r0 + j >= border && y0 + r0 + j < H - border;
+    for (int j = 0; j < kExRows; ++j) rows |= (y0 + r0 + j >= border && y0 + r0 + j < H - border ? 1u : 0u) << j;
     // Sliding window over the layers: p = l-2, c = l-1, n = l.
-    float BMp[kExRows], Bmp[kExRows], BMc[kExRows], Bmc[kExRows], RMc[kExRows], Rmc[kExRows], Vc[kExRows];
+    uint32_t BMp[kExRows], Bmp[kExRows], BMc[kExRows], Bmc[kExRows], RMc[kExRows], Rmc[kExRows], Vc[kExRows];
 #pragma unroll
-    for (int j = 0; j < kExRows; ++j) BMp[j] = Bmp[j] = BMc[j] = Bmc[j] = RMc[j] = Rmc[j] = Vc[j] = 0.0f;
+    for (int j = 0; j < kExRows; ++j) BMp[j] = Bmp[j] = BMc[j] = Bmc[j] = RMc[j] = Rmc[j] = Vc[j] = 0u;
 #pragma unroll
     for (int l = 0; l < (NL > 0 ? NL : L); ++l) {
-        const float* t = tile + (l * kExSH + r0) * kExSW + tx;  // staged row y0 + r0 - 1
-        float left[kExRows + 2], mid[kExRows + 2], right[kExRows + 2], hM[kExRows + 2], hm[kExRows + 2];
+        const uint32_t* t = tile + (l * kExSH + r0) * kExSW + i + 4;  // staged row y0 + r0 - 1
+        uint32_t mid[kExRows + 2], hM[kExRows + 2], hm[kExRows + 2], rM[kExRows + 2], rm[kExRows + 2];
 #pragma unroll
         for (int j = 0; j < kExRows + 2; ++j) {
-            left[j] = t[j * kExSW - 1];
+            const uint32_t left = t[j * kExSW - 1], right = t[j * kExSW + 1];
             mid[j] = t[j * kExSW];
-            right[j] = t[j * kExSW + 1];
-            hM[j] = fmaxf(fmaxf(left[j], mid[j]), right[j]);
-            hm[j] = fminf(fminf(left[j], mid[j]), right[j]);
+            hM[j] = __vimax3_u16x2(left, mid[j], right);
+            hm[j] = __vimin3_u16x2(left, mid[j], right);
+            rM[j] = __vmaxu2(left, right);
+            rm[j] = __vminu2(left, right);
         }
-        float BMn[kExRows], Bmn[kExRows], RMn[kExRows], Rmn[kExRows];
+        uint32_t BMn[kExRows], Bmn[kExRows];
 #pragma unroll
         for (int j = 0; j < kExRows; ++j) {
-            BMn[j] = fmaxf(fmaxf(hM[j], hM[j + 1]), hM[j + 2]);
-            Bmn[j] = fminf(fminf(hm[j], hm[j + 1]), hm[j + 2]);
-            RMn[j] = fmaxf(fmaxf(hM[j], hM[j + 2]), fmaxf(left[j + 1], right[j + 1]));
-            Rmn[j] = fminf(fminf(hm[j], hm[j + 2]), fminf(left[j + 1], right[j + 1]));
+            BMn[j] = __vimax3_u16x2(hM[j], hM[j + 1], hM[j + 2]);
+            Bmn[j] = __vimin3_u16x2(hm[j], hm[j + 1], hm[j + 2]);
         }
         if (l >= 2) {
-            const int s = l - 1;  // centre layer
+            // centre layer l - 1
+            uint32_t ext[kExRows], some = 0;
 #pragma unroll
             for (int j = 0; j < kExRows; ++j) {
-                const int y = y0 + r0 + j;
-                const float v = Vc[j];
-                const bool ext = yin[j] && ((v > fmaxf(fmaxf(BMp[j], BMn[j]), RMc[j])) ||
-                                            (v < fminf(fminf(Bmp[j], Bmn[j]), Rmc[j])));
-                const uint32_t wv = __ballot_sync(0xffffffffu, ext);
-                if (lane == 0 && y < H && word < nw) {
-                    const long long w = od.word_base + ((long long)(s - 1) * H + y) * nw + word;
-                    words[w] = wv;
-                    if (wv) atomicAdd(&tiles[(w - word0) / kWordTile], (uint32_t)__popc(wv));
-                }
+                const uint32_t nM = __vimax3_u16x2(BMp[j], BMn[j], RMc[j]), nm = __vimin3_u16x2(Bmp[j], Bmn[j], Rmc[j]);
+                // a half other than zero: above all or below all
+                ext[j] = (__vmaxu2(Vc[j], nM) ^ nM) | (__vminu2(Vc[j], nm) ^ nm);
+                some |= ext[j];
             }
+            uint32_t wv = 0;
+            if (__any_sync(0xffffffffu, (some & columns) != 0u)) {
+#pragma unroll
+                for (int j = 0; j < kExRows; ++j) {
+                    const uint32_t e = rows >> j & 1u ? ext[j] & columns : 0u;
+                    const uint32_t lo = __ballot_sync(0xffffffffu, (e & 0xffffu) != 0u);
+                    const uint32_t hi = __ballot_sync(0xffffffffu, e >> 16 != 0u);
+                    if (lane >> 1 == j) wv = lane & 1 ? hi : lo;
+                }
+                if (writes && wv) atomicAdd(&tiles[(at - word0) / kWordTile], (uint32_t)__popc(wv));
+            }
+            if (writes) words[at] = wv;
+            at += (long long)H * nw;
         }
 #pragma unroll
         for (int j = 0; j < kExRows; ++j) {
@@ -178,24 +279,22 @@ __device__ __forceinline__ void extrema_tile(const uint8_t* __restrict__ u8arena
             Bmp[j] = Bmc[j];
             BMc[j] = BMn[j];
             Bmc[j] = Bmn[j];
-            RMc[j] = RMn[j];
-            Rmc[j] = Rmn[j];
+            RMc[j] = __vimax3_u16x2(hM[j], hM[j + 2], rM[j + 1]);
+            Rmc[j] = __vimin3_u16x2(hm[j], hm[j + 2], rm[j + 1]);
             Vc[j] = mid[j + 1];
         }
     }
 }
 
-// The extrema mask of entry e (one octave of one image), a tile per CTA; the
-// candidates are counted by tiles of kWordTile words, from word0 on.
+// The extrema mask of entry e (one octave of one image), a tile per CTA.
 template <int NL>
-__global__ void __launch_bounds__(256, 4) k_extrema_mask(const uint8_t* __restrict__ u8arena,
-                                                      const float* __restrict__ lut255, EntryTable tab, int e,
+__global__ void __launch_bounds__(kExThreads, 4) k_extrema_mask(const uint8_t* __restrict__ u8arena, EntryTable tab, int e,
                                                       int border, uint32_t* __restrict__ words, long long word0,
                                                       uint32_t* __restrict__ tiles) {
     chain_wait();
-    extern __shared__ __align__(16) float tile[];  // [layers][kExSH][kExSW], then lut[256]
+    extern __shared__ __align__(16) uint32_t tile[];  // [layers][kExSH][kExSW]
     const OctaveDev od = tab.ents[e];
-    extrema_tile<NL>(u8arena, lut255, od, tab.S, border, words, word0, tiles, blockIdx.x * kExTX, blockIdx.y * kExTY,
+    extrema_tile<NL>(u8arena, od, tab.S, border, words, word0, tiles, blockIdx.x * kExTX, blockIdx.y * kExTY,
                      tile);
 }
 
@@ -203,13 +302,12 @@ __global__ void __launch_bounds__(256, 4) k_extrema_mask(const uint8_t* __restri
 // tile b - tile_pref[k] of entry e0 + k, tile_pref[k] <= b < tile_pref[k + 1]
 // (row-major tiles of kExTX x kExTY).
 template <int NL>
-__global__ void __launch_bounds__(256, 4) k_extrema_mask_flat(const uint8_t* __restrict__ u8arena,
-                                                           const float* __restrict__ lut255, EntryTable tab, int e0,
+__global__ void __launch_bounds__(kExThreads, 4) k_extrema_mask_flat(const uint8_t* __restrict__ u8arena, EntryTable tab, int e0,
                                                            int n_e, const uint32_t* __restrict__ tile_pref,
                                                            int border, uint32_t* __restrict__ words,
                                                            long long word0, uint32_t* __restrict__ tiles) {
     chain_wait();
-    extern __shared__ __align__(16) float tile[];
+    extern __shared__ __align__(16) uint32_t tile[];
     const uint32_t b = blockIdx.x;
     int lo = 0, hi = n_e;  // the last k with tile_pref[k] <= b
     while (hi - lo > 1) {
@@ -219,7 +317,7 @@ __global__ void __launch_bounds__(256, 4) k_extrema_mask_flat(const uint8_t* __r
     const OctaveDev od = tab.ents[e0 + lo];
     const int tx = (od.W + kExTX - 1) / kExTX;
     const int t = (int)(b - tile_pref[lo]);
-    extrema_tile<NL>(u8arena, lut255, od, tab.S, border, words, word0, tiles, (t % tx) * kExTX, (t / tx) * kExTY, tile);
+    extrema_tile<NL>(u8arena, od, tab.S, border, words, word0, tiles, (t % tx) * kExTX, (t / tx) * kExTY, tile);
 }
 
 // solve_linear_system (src/sift.rs:478-503), Cramer's rule in f32.
@@ -456,20 +554,20 @@ int launch_dog_dense(const uint8_t* u8arena, const float* lut255, const PyramidD
     return cudaPeekAtLastError() == cudaSuccess ? 0 : -1;
 }
 
-static size_t extrema_smem(int S) { return sizeof(float) * ((size_t)(S + 2) * kExSH * kExSW + 256); }
+static size_t extrema_smem(int S) { return sizeof(uint32_t) * (size_t)(S + 2) * kExSH * kExSW; }
 
-int launch_extrema_mask(const uint8_t* u8arena, const float* lut255, const EntryTable& tab, const OctaveDev& od,
+int launch_extrema_mask(const uint8_t* u8arena, const EntryTable& tab, const OctaveDev& od,
                         int e, int border, uint32_t* words, uint32_t* tiles, cudaStream_t st) {
     if (od.W <= 0 || od.H <= 0) return 0;
     if (tab.S + 2 > kExMaxLayers) return -1;
     dim3 grid((od.W + kExTX - 1) / kExTX, (od.H + kExTY - 1) / kExTY);
     const size_t smem = extrema_smem(tab.S);
-    void (*k)(const uint8_t*, const float*, EntryTable, int, int, uint32_t*, long long, uint32_t*) =
+    void (*k)(const uint8_t*, EntryTable, int, int, uint32_t*, long long, uint32_t*) =
         tab.S == 3 ? k_extrema_mask<5> : (tab.S == 4 ? k_extrema_mask<6> : k_extrema_mask<0>);
     if (smem > 48 * 1024 &&
         cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
         return -1;
-    if (launch_chained(k, grid, 256, smem, st, u8arena, lut255, tab, e, border, words, od.word_base, tiles) !=
+    if (launch_chained(k, grid, kExThreads, smem, st, u8arena, tab, e, border, words, od.word_base, tiles) !=
         cudaSuccess)
         return -1;
     return cudaPeekAtLastError() == cudaSuccess ? 0 : -1;
@@ -479,18 +577,18 @@ int extrema_tiles(int W, int H) {
     return W > 0 && H > 0 ? ((W + kExTX - 1) / kExTX) * ((H + kExTY - 1) / kExTY) : 0;
 }
 
-int launch_extrema_mask_flat(const uint8_t* u8arena, const float* lut255, const EntryTable& tab, int e0, int n_e,
+int launch_extrema_mask_flat(const uint8_t* u8arena, const EntryTable& tab, int e0, int n_e,
                              const uint32_t* tile_pref, uint32_t n_tiles, int border, uint32_t* words,
                              uint32_t* tiles, cudaStream_t st) {
     if (n_tiles == 0) return 0;
     if (tab.S + 2 > kExMaxLayers) return -1;
     const size_t smem = extrema_smem(tab.S);
-    void (*k)(const uint8_t*, const float*, EntryTable, int, int, const uint32_t*, int, uint32_t*, long long, uint32_t*) =
+    void (*k)(const uint8_t*, EntryTable, int, int, const uint32_t*, int, uint32_t*, long long, uint32_t*) =
         tab.S == 3 ? k_extrema_mask_flat<5> : (tab.S == 4 ? k_extrema_mask_flat<6> : k_extrema_mask_flat<0>);
     if (smem > 48 * 1024 &&
         cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
         return -1;
-    if (launch_chained(k, n_tiles, 256, smem, st, u8arena, lut255, tab, e0, n_e, tile_pref, border, words, 0ll, tiles) !=
+    if (launch_chained(k, n_tiles, kExThreads, smem, st, u8arena, tab, e0, n_e, tile_pref, border, words, 0ll, tiles) !=
         cudaSuccess)
         return -1;
     return cudaPeekAtLastError() == cudaSuccess ? 0 : -1;

@@ -67,10 +67,9 @@ int launch_match(const float* d_q, uint32_t nq, const float* d_t, uint32_t nt, S
                  cudaStream_t st, const float* h_q = nullptr, const float* h_t = nullptr, uint32_t* err_out = nullptr);
 int launch_to_luma(int format, const uint8_t* px, long long stride, int W, int H, uint8_t* out, long long out_pitch,
                    cudaStream_t st);
-int launch_extrema_mask(const uint8_t* u8arena, const float* lut255, const EntryTable& tab, const OctaveDev& od,
-                        int e, int border, uint32_t* words, uint32_t* tiles, cudaStream_t st);
+int launch_extrema_mask(const uint8_t* u8arena, const EntryTable& tab, const OctaveDev& od, int e, int border, uint32_t* words, uint32_t* tiles, cudaStream_t st);
 int extrema_tiles(int W, int H);
-int launch_extrema_mask_flat(const uint8_t* u8arena, const float* lut255, const EntryTable& tab, int e0, int n_e,
+int launch_extrema_mask_flat(const uint8_t* u8arena, const EntryTable& tab, int e0, int n_e,
                              const uint32_t* tile_pref, uint32_t n_tiles, int border, uint32_t* words,
                              uint32_t* tiles, cudaStream_t st);
 int launch_dog_dense(const uint8_t* u8arena, const float* lut255, const PyramidDev& pyr, int o, int l, float* out,
@@ -724,7 +723,7 @@ struct Engine {
             const OctaveDev& od = pyr.oct[o];
             OctCounters* oc = &ctr->oct[o];
             uint32_t* tiles = d_tiles.as<uint32_t>() + pb[o];
-            if (od.nw > 0 && ok(launch_extrema_mask(U, lut, tab(), od, o, (int)p.image_border_width,
+            if (od.nw > 0 && ok(launch_extrema_mask(U, tab(), od, o, (int)p.image_border_width,
                                                     d_words.as<uint32_t>(), tiles, q)))
                 return cuda_fail(cudaGetLastError(), "extrema mask");
             if (od.nw > 0 && ok(launch_candidates(U, lut, tab(), p.sigma, p.contrast_threshold, p.edge_threshold, o, 1,
