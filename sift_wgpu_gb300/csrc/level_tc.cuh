@@ -28,12 +28,18 @@
 // and the fraction are bit fields of the result.
 //
 // Bound: instruction issue and the latency around its two barriers (45 % of
-// issue slots, 20 % of the tensor cycles at 4096 x 4096). Measured against
+// issue slots, 20 % of the tensor cycles at 4096 x 4096), which a sum in the
+// reference's order lengthens: with none at all a 1080p frame's levels would
+// take 119 us instead of 139. So the error bound is kept tight (half an ulp of
+// each partial sum, tables.cpp; relative to 255 and rounded up to a power of
+// two, three times as many sums were near, 157 us with the next) and the taps
+// are in shared memory (read from the L2 cache at the first such sum, 150 us).
+// Measured against
 // the scalar kernel it replaced (one rounded multiply and add per tap):
 // a 4096 x 4096 level of radius 4, 48.1 -> 34.0 us (40 -> 18.5 M warp
 // instructions); radius 13 on 2048 x 2048 (two passes before), 36 -> 18 us;
 // radius 20 on 480 x 270, 10.3 -> 9 us; a 160 x 120 frame's pyramid,
-// 153 -> 106 us.
+// 153 -> 97 us.
 #pragma once
 
 #include "sift_internal.cuh"
@@ -53,6 +59,7 @@ namespace tc {
 
 constexpr int kTX = 64;
 constexpr int kThreads = 256;
+constexpr int kTaps = 64;  // (57 at most)
 constexpr int kHS = 72;  // row stride of the horizontal result (halves): 9 x 16 bytes, ldmatrix rows in distinct banks
 
 // P: columns staged left and right of the tile; PV: rows above and below.
@@ -61,7 +68,7 @@ struct Shape {
     static constexpr int KH = (8 + 2 * P) / 16, KV = (16 + 2 * PV) / 16;
     static constexpr int RH = TY + 2 * PV;   // rows of the horizontal pass
     static constexpr int SW = kTX + 2 * P;   // staged row (halves), an odd multiple of 8
-    static constexpr size_t smem = sizeof(uint16_t) * ((size_t)RH * SW + (size_t)RH * kHS);
+    static constexpr size_t smem = sizeof(uint16_t) * ((size_t)RH * SW + (size_t)RH * kHS) + sizeof(float) * kTaps;
     static_assert((8 + 2 * P) % 16 == 0 && (16 + 2 * PV) % 16 == 0 && RH % 16 == 0 && (SW / 8) % 2 == 1, "tile shape");
 };
 
@@ -87,7 +94,7 @@ __device__ __forceinline__ void ldsm4t(uint32_t (&r)[4], uint32_t addr) {
 
 // The reference's sum of one output over `taps` staged values `step` halves
 // apart: products and sums rounded one by one in tap order, truncated to u8.
-__device__ __noinline__ uint32_t exact_tap_sum(const uint16_t* p, int step, const float* __restrict__ wts, int taps) {
+__device__ __noinline__ uint32_t exact_tap_sum(const uint16_t* p, int step, const float* wts, int taps) {
     float s = 0.0f;
     for (int i = 0; i < taps; ++i, p += step) s = __fadd_rn(s, __fmul_rn((float)*p, wts[i]));
     return (uint32_t)clamp_u8(s);
@@ -101,23 +108,23 @@ __device__ __noinline__ uint32_t exact_tap_sum(const uint16_t* p, int step, cons
 template <bool CLAMP>
 __device__ __forceinline__ bool to_bytes(const float (&ca)[4], const float (&cb)[4], const TcParams& tp,
                                          uint32_t (&v)[4], uint32_t& m) {
-    uint32_t b[4];
-    bool near = false;
+    constexpr int kWhole = CLAMP ? 18 : 17;  // bits above the fraction
+    uint32_t b[4], frac[4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
         const float s = __fmaf_rn(cb[j], tp.scale_b, ca[j]);
         b[j] = __float_as_uint(s);
-        near = near || (b[j] & tp.near) == 0u;
+        frac[j] = b[j] << kWhole;
         // the whole part to the low mantissa bits by an addition that truncates
         v[j] = __float_as_uint(__fadd_rz(s, tp.whole));
         if (CLAMP) v[j] = min(v[j] & 0x1ffu, 255u);
     }
-    if (!__any_sync(0xffffffffu, near)) return false;
-    const uint32_t one = __float_as_uint(tp.init_a) + (1u << (CLAMP ? 14 : 15));
+    if (!__any_sync(0xffffffffu, min(min(frac[0], frac[1]), min(frac[2], frac[3])) < tp.near)) return false;
+    const uint32_t one = __float_as_uint(tp.init_a) + (1u << (32 - kWhole));
     m = 0;
 #pragma unroll
     for (int j = 0; j < 4; ++j)
-        if ((b[j] & tp.near) == 0u && b[j] >= one) m |= 1u << j;
+        if (frac[j] < tp.near && b[j] >= one) m |= 1u << j;
     return true;
 }
 
@@ -144,8 +151,10 @@ __device__ __forceinline__ void level_tile(const uint8_t* __restrict__ in, int i
     using S = Shape<P, PV, TY>;
     uint16_t* src = sm;
     uint16_t* hs = sm + S::RH * S::SW;
+    float* wts = reinterpret_cast<float*>(hs + S::RH * kHS);  // the taps
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int g = lane >> 2, t = lane & 3;
+    if (tid < 2 * tp.r + 1) wts[tid] = tp.wts[tid];
     // Stage: a row is SW / 4 words of 4 pixels, one per lane; warp w takes
     // rows w, w + 8, .. with all their loads in flight. Words outside the row
     // repeat its first or last pixel (a byte permute with the lane's
@@ -213,7 +222,7 @@ __device__ __forceinline__ void level_tile(const uint8_t* __restrict__ in, int i
                     m &= m - 1u;
                     const int dy = 8 * (j >> 1), dx = j & 1;
                     h[dy * kHS + dx] = (uint16_t)exact_tap_sum(
-                        src + (mb * 16 + g + dy) * S::SW + 8 * warp + 2 * t + dx + P - tp.r, 1, tp.wts, 2 * tp.r + 1);
+                        src + (mb * 16 + g + dy) * S::SW + 8 * warp + 2 * t + dx + P - tp.r, 1, wts, 2 * tp.r + 1);
                 }
                 __syncwarp();
             }
@@ -224,11 +233,10 @@ __device__ __forceinline__ void level_tile(const uint8_t* __restrict__ in, int i
     static_assert(NB == 2 || NB == 4, "tile height");
     const int mb = warp % kMB, c0 = 8 * NB * (warp / kMB);
     float ca[NB][4], cb[NB][4];
+    // lane l addresses row l & 15 of columns 8 (l >> 4) .. of a 16 x 16 block
+    const uint32_t b0 = (uint32_t)__cvta_generic_to_shared(hs + (mb * 16 + (lane & 15)) * kHS + c0 + 8 * (lane >> 4));
     {
         const uint4* vf = tp.frags + S::KH * 32 + 2 * lane;
-        // lane l addresses row l & 15 of columns 8 (l >> 4) .. of a 16 x 16 block
-        const uint32_t b0 =
-            (uint32_t)__cvta_generic_to_shared(hs + (mb * 16 + (lane & 15)) * kHS + c0 + 8 * (lane >> 4));
         uint4 fa = vf[0], fb = vf[1];
         __syncthreads();
 #pragma unroll
@@ -266,7 +274,7 @@ __device__ __forceinline__ void level_tile(const uint8_t* __restrict__ in, int i
                 m &= m - 1u;
                 const int dy = 8 * (j >> 1), dx = j & 1;
                 const uint32_t e = exact_tap_sum(
-                    hs + (mb * 16 + g + dy + PV - tp.r) * kHS + c0 + 8 * nb + 2 * t + dx, kHS, tp.wts, 2 * tp.r + 1);
+                    hs + (mb * 16 + g + dy + PV - tp.r) * kHS + c0 + 8 * nb + 2 * t + dx, kHS, wts, 2 * tp.r + 1);
                 p = (p & ~(0xffu << (8 * j))) | e << (8 * j);
             }
             __syncwarp();

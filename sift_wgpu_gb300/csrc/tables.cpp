@@ -126,13 +126,15 @@ TcBlur tc_blur(const std::vector<float>& w) {
     }
     for (int i = 0; i < n; ++i)
         if (a[i] > 2047) return t;
-    const double u = std::ldexp(1.0, -24);
-    double cum = 0.0, steps = 0.0;
+    // The reference's rounding error: half an ulp of each product and of each
+    // partial sum, which are largest where every pixel is 255 (half an ulp
+    // does not fall as the value rises).
+    double cum = 0.0, ref = 0.0;
+    auto half_ulp = [](double x) { return x > 0.0 ? std::ldexp(1.0, std::ilogb(x) - 24) : 0.0; };
     for (int i = 0; i < n; ++i) {
         cum += w[i];
-        steps += cum;
+        ref += half_ulp(255.0 * w[i]) + half_ulp(255.0 * cum * (1.0 + 4.0 * n * std::ldexp(1.0, -24)));
     }
-    const double ref = 255.0 * u * (steps + wsum) * (1.0 + 4.0 * n * u);
     t.clamp = 255.0 * wsum + 1.0 >= 256.0;
     const int frac = t.clamp ? 14 : 15;
     if (255.0 * wsum + 1.0 >= std::ldexp(1.0, 23 - frac) || qa + 24 - frac > 24) return t;
@@ -147,10 +149,8 @@ TcBlur tc_blur(const std::vector<float>& w) {
     t.scale_b = (float)std::ldexp(1.0, -shift);
     t.whole = (float)(std::ldexp(1.0, qa - 24 + 23) - t.init_a);
     const uint32_t thr = (uint32_t)std::ceil(2.0 * std::ldexp(be, frac - qa - shift)) + 1u;
-    uint32_t p2 = 1;
-    while (p2 < thr) p2 <<= 1;
-    if (p2 >> (frac - 2)) return t;
-    t.near = ((1u << frac) - 1u) & ~(p2 - 1u);
+    if (thr >> (frac - 2)) return t;
+    t.near = thr << (32 - frac);
     // fragments (m16n8k16): lane = 4 g + t holds k = 2t, 2t+1 (+8)
     const int P = r <= 4 ? 4 : (r + 3) / 8 * 8 + 4, PV = (r + 7) / 8 * 8;
     t.kh = (8 + 2 * P) / 16;

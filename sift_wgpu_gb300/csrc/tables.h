@@ -29,7 +29,7 @@ struct TcBlur {
     bool clamp = false;   // sums can reach 256: 9 whole bits and a clamp
     float init_a = 0, init_b = 0, scale_b = 0;  // accumulator start values, 2^-shift
     float whole = 0;      // added with truncation: the whole part to the low mantissa bits
-    uint32_t near = 0;    // fraction bits that are all 0 where the exact sum decides
+    uint32_t near = 0;    // the exact sum decides below it (the fraction in the top bits)
     std::vector<uint32_t> frags;  // kh x 32 lanes x 4, then kv x 32 lanes x 8
 };
 TcBlur tc_blur(const std::vector<float>& taps);
