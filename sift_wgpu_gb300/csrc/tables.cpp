@@ -138,7 +138,7 @@ TcBlur tc_blur(const std::vector<float>& w) {
     t.clamp = 255.0 * wsum + 1.0 >= 256.0;
     const int frac = t.clamp ? 14 : 15;
     if (255.0 * wsum + 1.0 >= std::ldexp(1.0, 23 - frac) || qa + 24 - frac > 24) return t;
-    const double e = quant + ref + std::ldexp(1.0, -frac);
+    const double e = quant + ref + std::ldexp(0.5, -frac);  // (the last: the rounding to `frac` bits)
     // s in units of 1 is 2^(qa - 24) in the accumulators (pixels enter as
     // f16 subnormals, v 2^-24); the start value puts s in the mantissa with
     // `frac` fraction bits
@@ -148,7 +148,8 @@ TcBlur tc_blur(const std::vector<float>& w) {
     t.init_b = (float)std::ldexp(be, -24);
     t.scale_b = (float)std::ldexp(1.0, -shift);
     t.whole = (float)(std::ldexp(1.0, qa - 24 + 23) - t.init_a);
-    const uint32_t thr = (uint32_t)std::ceil(2.0 * std::ldexp(be, frac - qa - shift)) + 1u;
+    // s enlarged by e: the reference's sum lies in [s - 2 e, s]
+    const uint32_t thr = (uint32_t)std::ceil(2.0 * std::ldexp(be, frac - qa - shift));
     if (thr >> (frac - 2)) return t;
     t.near = thr << (32 - frac);
     // fragments (m16n8k16): lane = 4 g + t holds k = 2t, 2t+1 (+8)
