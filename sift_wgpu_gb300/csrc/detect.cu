@@ -350,14 +350,14 @@ __device__ __forceinline__ bool solve3(const float a[3][3], const float b[3], fl
 struct RefineParams {
     float sigma;
     float contrast_threshold;
-    float edge_threshold;
+    float edge_ratio;  // (edge threshold + 1)^2 / edge threshold
     int S;
     int levels_dog;  // S + 2
 };
 
 // One candidate through refine_and_filter_extrema (src/sift.rs:299-474).
 template <class Dog>
-__device__ bool refine_one(const Dog& dog, int o, int entry, int x, int y, int s, const RefineParams& rp,
+__device__ __forceinline__ bool refine_one(const Dog& dog, int o, int entry, int x, int y, int s, const RefineParams& rp,
                            Keypoint* out) {
     int cx = x, cy = y, cl = s;
     const float scale = __int_as_float((127 + o) << 23);  // 2^o
@@ -365,28 +365,37 @@ __device__ bool refine_one(const Dog& dog, int o, int entry, int x, int y, int s
     for (int step = 0; step < 5; ++step) {
         if (cl < 1 || cl >= nl - 1) return false;
         if (cx < 1 || cx >= dog.W - 1 || cy < 1 || cy >= dog.H - 1) return false;
-        const int lp = cl - 1, lc = cl, ln = cl + 1;
-        const float c = dog.at(lc, cx, cy);
-        const float cxp = dog.at(lc, cx + 1, cy), cxm = dog.at(lc, cx - 1, cy);
-        const float cyp = dog.at(lc, cx, cy + 1), cym = dog.at(lc, cx, cy - 1);
-        const float nc = dog.at(ln, cx, cy), pc = dog.at(lp, cx, cy);
-        const float dx = __fdiv_rn(__fsub_rn(cxp, cxm), 2.0f);
-        const float dy = __fdiv_rn(__fsub_rn(cyp, cym), 2.0f);
-        const float ds = __fdiv_rn(__fsub_rn(nc, pc), 2.0f);
+        // the levels below, at and above the layer's two, rows cy - 1 .. cy + 1:
+        // all inside, so each value is one read at a constant distance
+        const uint8_t* g1 = dog.base + (long long)cl * dog.plane + (long long)cy * dog.pitch + cx;
+        const uint8_t *g0 = g1 - dog.plane, *g2 = g1 + dog.plane, *g3 = g2 + dog.plane;
+        const float* lut = dog.lut;
+        const int up = -dog.pitch, down = dog.pitch;
+        auto layer = [&](const uint8_t* lower, const uint8_t* upper, int at) {
+            return __fsub_rn(lut[upper[at]], lut[lower[at]]);
+        };
+        const float c = layer(g1, g2, 0);
+        const float cxp = layer(g1, g2, 1), cxm = layer(g1, g2, -1);
+        const float cyp = layer(g1, g2, down), cym = layer(g1, g2, up);
+        const float nc = layer(g2, g3, 0), pc = layer(g0, g1, 0);
+        // (halves and quarters are exact)
+        const float dx = __fmul_rn(__fsub_rn(cxp, cxm), 0.5f);
+        const float dy = __fmul_rn(__fsub_rn(cyp, cym), 0.5f);
+        const float ds = __fmul_rn(__fsub_rn(nc, pc), 0.5f);
         const float c2 = __fmul_rn(2.0f, c);
         const float dxx = __fsub_rn(__fadd_rn(cxp, cxm), c2);
         const float dyy = __fsub_rn(__fadd_rn(cyp, cym), c2);
         const float dss = __fsub_rn(__fadd_rn(nc, pc), c2);
-        const float dxy = __fdiv_rn(__fadd_rn(__fsub_rn(__fsub_rn(dog.at(lc, cx + 1, cy + 1), dog.at(lc, cx - 1, cy + 1)),
-                                                        dog.at(lc, cx + 1, cy - 1)),
-                                              dog.at(lc, cx - 1, cy - 1)),
-                                    4.0f);
-        const float dxs = __fdiv_rn(__fsub_rn(__fsub_rn(dog.at(ln, cx + 1, cy), dog.at(ln, cx - 1, cy)),
-                                              __fsub_rn(dog.at(lp, cx + 1, cy), dog.at(lp, cx - 1, cy))),
-                                    4.0f);
-        const float dys = __fdiv_rn(__fsub_rn(__fsub_rn(dog.at(ln, cx, cy + 1), dog.at(ln, cx, cy - 1)),
-                                              __fsub_rn(dog.at(lp, cx, cy + 1), dog.at(lp, cx, cy - 1))),
-                                    4.0f);
+        const float dxy = __fmul_rn(__fadd_rn(__fsub_rn(__fsub_rn(layer(g1, g2, down + 1), layer(g1, g2, down - 1)),
+                                                        layer(g1, g2, up + 1)),
+                                              layer(g1, g2, up - 1)),
+                                    0.25f);
+        const float dxs = __fmul_rn(__fsub_rn(__fsub_rn(layer(g2, g3, 1), layer(g2, g3, -1)),
+                                              __fsub_rn(layer(g0, g1, 1), layer(g0, g1, -1))),
+                                    0.25f);
+        const float dys = __fmul_rn(__fsub_rn(__fsub_rn(layer(g2, g3, down), layer(g2, g3, up)),
+                                              __fsub_rn(layer(g0, g1, down), layer(g0, g1, up))),
+                                    0.25f);
         const float hm[3][3] = {{dxx, dxy, dxs}, {dxy, dyy, dys}, {dxs, dys, dss}};
         const float g[3] = {-dx, -dy, -ds};
         float off[3];
@@ -400,9 +409,7 @@ __device__ bool refine_one(const Dog& dog, int o, int entry, int x, int y, int s
             const float det = __fsub_rn(__fmul_rn(dxx, dyy), __fmul_rn(dxy, dxy));
             if (det <= 0.0f) return false;
             const float ratio = __fdiv_rn(trace_sq, det);
-            const float e1 = __fadd_rn(rp.edge_threshold, 1.0f);
-            const float thr = __fdiv_rn(__fmul_rn(e1, e1), rp.edge_threshold);
-            if (ratio >= thr) return false;
+            if (ratio >= rp.edge_ratio) return false;
             const float lf = __fadd_rn((float)cl, off[2]);
             const float e = __fadd_rn((float)o, __fdiv_rn(lf, (float)rp.S));
             const float p2 = (float)exp2((double)e);
@@ -433,11 +440,13 @@ __device__ bool refine_one(const Dog& dog, int o, int entry, int x, int y, int s
 //
 // Latency bounds it (a chain of dependent scattered reads per candidate and
 // step), so the tiles are small: 512 words, some 50 candidates of a dense
-// frame, make 380 CTAs of a 1080p octave 0. It takes 20 us there and 54 us at
-// 4096 x 4096 (cold caches); a scan of the word counts with look-back, a kernel
-// that emitted and one that refined took 12.7 + 5.9 + 20 and 30 + 17 + 60 us.
-// The stage with the mask: 123 -> 91 us at 1080p, 410 -> 351 at 4096 x 4096;
-// a 160 x 120 frame, end to end, 136 -> 122.
+// frame, make 380 CTAs of a 1080p octave 0. A scan of the word counts with
+// look-back, a kernel that emitted and one that refined took 12.7 + 5.9 + 20 us
+// there and 30 + 17 + 60 us at 4096 x 4096, this one at first 20 and 54 us
+// (cold caches; the stage with the mask 123 -> 91 us at 1080p, 410 -> 351 at
+// 4096 x 4096; a 160 x 120 frame, end to end, 136 -> 122). Without the clamps of
+// its 38 reads a step, and with 28 of them, the stage went from 79 to 71 and
+// from 231 to 210 us.
 constexpr int kCandThreads = 128, kCandWords = kWordTile / kCandThreads;
 constexpr uint32_t kCandList = 1024;  // candidates at a time
 static_assert(kWordTile * 32 <= 1 << 16, "a bit's index in its tile has 16 bits");
@@ -599,7 +608,8 @@ int launch_candidates(const uint8_t* u8arena, const float* lut255, const EntryTa
                       uint32_t* cand_off, Keypoint* cands, Keypoint* refined_at, uint32_t* keep, uint32_t cap,
                       Counters* ctr, OctCounters* oc, cudaStream_t st) {
     if (n_words <= 0) return 0;
-    const RefineParams rp{sigma, contrast, edge, tab.S, tab.S + 2};
+    const float e1 = edge + 1.0f;
+    const RefineParams rp{sigma, contrast, e1 * e1 / edge, tab.S, tab.S + 2};
     const size_t n_tiles = word_tiles(n_words);
     // a CTA per tile; of a very long list several, so that the sums over the
     // tiles before stay a small part of the reads
