@@ -232,15 +232,6 @@ struct BatchEngine {
         std::vector<int> itab;
         std::vector<float> ftab;
         std::vector<uint8_t> lz(batch_lz_bytes() * (size_t)std::max(N * O, 1), 0);
-        auto max_span = [](const AxisTaps& t) {
-            const int T = lanczos_fused_tile(), n = (int)t.left.size();
-            int m = 0;
-            for (int a = 0; a < n; a += T) {
-                const int b = std::min(a + T, n) - 1;
-                m = std::max(m, t.left[b] + t.count[b] - t.left[a]);
-            }
-            return m;
-        };
         for (int i = 0; i < N; ++i)
             for (int o = 0; o + 1 < O; ++o) {
                 const OctaveDev& a = ents[(size_t)i * O + o];
@@ -248,7 +239,7 @@ struct BatchEngine {
                 if (a.W == 0 || a.H == 0 || b.W == 0 || b.H == 0) continue;
                 AxisTaps tv = lanczos_axis((uint32_t)a.H, (uint32_t)b.H);
                 AxisTaps th = lanczos_axis((uint32_t)a.W, (uint32_t)b.W);
-                if (max_span(tv) > lanczos_fused_span() || max_span(th) > lanczos_fused_span())
+                if (!lanczos_fits(tv) || !lanczos_fits(th))
                     return fail(SIFT_CUDA_ERR_UNSUPPORTED, "a batch image's resize window exceeds the fused tile");
                 const int vt = (int)itab.size();
                 itab.insert(itab.end(), tv.left.begin(), tv.left.end());

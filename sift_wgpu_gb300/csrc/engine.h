@@ -54,8 +54,7 @@ template <typename TG>
 int launch_lanczos(const uint8_t* src, int src_pitch, int W, int H, float* tmp, int tmp_pitch, TG* dst,
                    uint8_t* dst_u8, int dst_pitch, int nW, int nH, const int* vtab, const float* vw, const int* htab,
                    const float* hw, const LanczosUniform& uni, cudaStream_t st, bool fused, int* launches);
-int lanczos_fused_span();
-int lanczos_fused_tile();
+bool lanczos_fits(const AxisTaps& t);
 int pixel_channels(int format);
 int launch_begin(const RunCell* hcell, RunCell* cell, Counters* ctr, uint32_t* tiles, size_t n_tiles, cudaStream_t st);
 int launch_fetch(const uint8_t* src, long long stride, uint8_t* img, long long pitch, int W, int H, cudaStream_t st);
@@ -542,15 +541,6 @@ struct Engine {
         std::vector<int> itab;
         std::vector<float> ftab;
         ltab.assign(O, LTab{0, 0, 0, 0, false, LanczosUniform{}});
-        auto max_span = [](const AxisTaps& t) {
-            const int T = lanczos_fused_tile(), n = (int)t.left.size();
-            int m = 0;
-            for (int a = 0; a < n; a += T) {
-                const int b = std::min(a + T, n) - 1;
-                m = std::max(m, t.left[b] + t.count[b] - t.left[a]);
-            }
-            return m;
-        };
         for (int o = 0; o + 1 < O; ++o) {
             const OctaveDev& a = g.oct[o];
             const int nW = g.oct[o + 1].W, nH = g.oct[o + 1].H;
@@ -570,7 +560,7 @@ struct Engine {
             itab.insert(itab.end(), th.woff.begin(), th.woff.end());
             t.hw = ftab.size();
             ftab.insert(ftab.end(), th.w.begin(), th.w.end());
-            t.fused = max_span(tv) <= lanczos_fused_span() && max_span(th) <= lanczos_fused_span();
+            t.fused = lanczos_fits(tv) && lanczos_fits(th);
             t.uni = LanczosUniform{};
             uniform_2x(th, (uint32_t)a.W, &t.uni.x0, &t.uni.x1, t.uni.wh);
             uniform_2x(tv, (uint32_t)a.H, &t.uni.y0, &t.uni.y1, t.uni.wv);

@@ -24,6 +24,7 @@
 //   k_lanczos_fused  the 2x Lanczos3 resize between octaves, both passes.
 // The base level of a host call reads its image through an ImgRef cell (the
 // engine's device copy, or the caller's pageable buffer in place).
+#include <algorithm>
 #include <cstring>
 #include <type_traits>
 
@@ -345,7 +346,11 @@ __global__ void k_u8_to_level(const uint8_t* __restrict__ img, long long stride,
 // Tiles inside the uniform interior of a 2x resize (LanczosUniform) run both
 // passes with the 12 taps as constants: each thread sums 4 outputs from 18
 // shared loads, the tap loops unrolled; the sums are the same, in the same
-// order.
+// order. The other tiles (at the borders: all of a small plane's) stage their
+// outputs' taps in shared memory beside the window; read from device memory
+// tap by tap they took 10 us where this takes 5.5 (160 x 120; with them the
+// pyramid 97 -> 85 us, at 640 x 480 121 -> 106, at 1080p 137 -> 124).
+constexpr int kLzTaps = 14;  // of an output (a resize to half has 13 at most, of 15 pixels)
 constexpr int kLzT = 32, kLzSpan = 80, kLzMid = 81;  // odd mid stride: lanes on rows hit 32 banks
 constexpr int kLzIn = 96;  // staged row: 16-byte aligned x from x_lo & ~15, x_lo - (x_lo & ~15) + span <= 95
 
@@ -357,6 +362,8 @@ __device__ __forceinline__ void lanczos_tile(const uint8_t* __restrict__ src, in
                                              const LanczosUniform& uni, int ox0, int oy0) {
     __shared__ __align__(16) float in_rows[kLzSpan][kLzIn];
     __shared__ float mid[kLzT][kLzMid];
+    __shared__ float taps[2][kLzTaps][kLzT];       // vertical, horizontal
+    __shared__ int first[2][kLzT], count[2][kLzT];  // of the taps, from y_lo and x_lo on
     const int* vleft = vtab;
     const int* vcount = vtab + nH;
     const int* voff = vtab + 2 * nH;
@@ -368,6 +375,21 @@ __device__ __forceinline__ void lanczos_tile(const uint8_t* __restrict__ src, in
     const int x_lo = hleft[ox0], x_hi = hleft[ox1 - 1] + hcount[ox1 - 1];
     const int y_lo = vleft[oy0], y_hi = vleft[oy1 - 1] + vcount[oy1 - 1];
     const int sw = x_hi - x_lo, sh = y_hi - y_lo;
+    const bool uniform = ox0 >= uni.x0 && ox0 + kLzT <= uni.x1 && oy0 >= uni.y0 && oy0 + kLzT <= uni.y1;
+    if (!uniform) {
+        // a thread stages four taps or so of output k of an axis, and lane 0 its place
+        const int axis = warp >> 2, k = lane, i0 = warp & 3;
+        const int out = min((axis ? ox0 : oy0) + k, (axis ? ox1 : oy1) - 1);
+        const int* left = axis ? hleft : vleft;
+        const int c = (axis ? hcount : vcount)[out], o = (axis ? hoff : voff)[out];
+        const float* w = axis ? hw : vw;
+        if (i0 == 0) {
+            first[axis][k] = left[out] - (axis ? x_lo : y_lo);
+            count[axis][k] = c;
+        }
+#pragma unroll
+        for (int i = i0; i < kLzTaps; i += 4) taps[axis][i][k] = i < c ? w[o + i] : 0.0f;
+    }
     // stage: 16-byte words from xa = x_lo & ~15 (staged column c holds x =
     // xa + c; the words end at align16(x_hi) <= the row pitch, a multiple of
     // 32), each byte to a float by one byte permute and one subtraction
@@ -391,7 +413,7 @@ __device__ __forceinline__ void lanczos_tile(const uint8_t* __restrict__ src, in
     __syncthreads();
     // in[y][x]: source (y_lo + y, x_lo + x)
     auto in = [&](int y, int x) -> float { return in_rows[y][xo + x]; };
-    if (ox0 >= uni.x0 && ox0 + kLzT <= uni.x1 && oy0 >= uni.y0 && oy0 + kLzT <= uni.y1) {
+    if (uniform) {
         // vertical pass: warp w makes mid rows 4w .. 4w+3 from source rows
         // 8w .. 8w+17 (output row r reads from 2r, tap i at j = 2r + i)
         for (int xx = lane; xx < sw; xx += 32) {
@@ -429,28 +451,46 @@ __device__ __forceinline__ void lanczos_tile(const uint8_t* __restrict__ src, in
         *reinterpret_cast<unsigned*>(dst_u8 + od) = packed;
         return;
     }
-    // vertical pass: rows oy0..oy1-1 (one warp per row), columns x_lo..x_hi-1
+    // vertical pass: rows oy0..oy1-1 (one warp per row), columns x_lo..x_hi-1,
+    // three to a lane (the last ones repeat column sw - 1)
     for (int oyl = warp; oyl < oy1 - oy0; oyl += 8) {
-        const int oy = oy0 + oyl;
-        const int l = vleft[oy] - y_lo, c = vcount[oy], o = voff[oy];
-        for (int xx = lane; xx < sw; xx += 32) {
-            float t = 0.0f;
-            for (int i = 0; i < c; ++i) t = __fadd_rn(t, __fmul_rn(in(l + i, xx), vw[o + i]));
-            mid[oyl][xx] = t;
+        const int l = first[0][oyl], c = count[0][oyl];
+        const int x0 = min(lane, sw - 1), x1 = min(lane + 32, sw - 1), x2 = min(lane + 64, sw - 1);
+        float t0 = 0.0f, t1 = 0.0f, t2 = 0.0f;
+#pragma unroll
+        for (int i = 0; i < kLzTaps; ++i) {
+            if (i < c) {
+                const float w = taps[0][i][oyl];
+                t0 = __fadd_rn(t0, __fmul_rn(in(l + i, x0), w));
+                t1 = __fadd_rn(t1, __fmul_rn(in(l + i, x1), w));
+                t2 = __fadd_rn(t2, __fmul_rn(in(l + i, x2), w));
+            }
         }
+        mid[oyl][x0] = t0;
+        if (lane + 32 < sw) mid[oyl][x1] = t1;
+        if (lane + 64 < sw) mid[oyl][x2] = t2;
     }
     __syncthreads();
-    // horizontal pass
-    for (int q = tid; q < (oy1 - oy0) * kLzT; q += 256) {
-        const int oyl = q >> 5, oxl = q & 31;
-        const int ox = ox0 + oxl;
-        if (ox >= ox1) continue;
-        const int l = hleft[ox] - x_lo, c = hcount[ox], o = hoff[ox];
-        float t = 0.0f;
-        for (int i = 0; i < c; ++i) t = __fadd_rn(t, __fmul_rn(mid[oyl][l + i], hw[o + i]));
-        t = t < 0.0f ? 0.0f : (t > 255.0f ? 255.0f : t);
-        const int v = (int)roundf(t);
-        const long long od = (long long)(oy0 + oyl) * dst_pitch + ox;
+    // horizontal pass: lane = output column, warp w = rows w, w + 8, ..
+    const int ox = ox0 + lane;
+    if (ox >= ox1) return;
+    const int l = first[1][lane], c = count[1][lane];
+    float t[kLzT / 8] = {};
+#pragma unroll
+    for (int i = 0; i < kLzTaps; ++i) {
+        if (i < c) {
+            const float w = taps[1][i][lane];
+#pragma unroll
+            for (int r = 0; r < kLzT / 8; ++r) t[r] = __fadd_rn(t[r], __fmul_rn(mid[warp + 8 * r][l + i], w));
+        }
+    }
+#pragma unroll
+    for (int r = 0; r < kLzT / 8; ++r) {
+        const int oy = oy0 + warp + 8 * r;
+        if (oy >= oy1) return;
+        const float s = t[r] < 0.0f ? 0.0f : (t[r] > 255.0f ? 255.0f : t[r]);
+        const int v = (int)roundf(s);
+        const long long od = (long long)oy * dst_pitch + ox;
         store_level(dst + od, v, norm255(v));
         dst_u8[od] = (uint8_t)v;
     }
@@ -730,7 +770,15 @@ int launch_lanczos(const uint8_t* src, int src_pitch, int W, int H, float* tmp, 
     return cudaPeekAtLastError() == cudaSuccess ? 0 : -1;
 }
 
-int lanczos_fused_span() { return kLzSpan; }
+// Whether an axis' windows and taps fit the fused kernel's tiles.
+bool lanczos_fits(const AxisTaps& t) {
+    const int n = (int)t.left.size();
+    for (int a = 0; a < n; a += kLzT) {
+        const int b = std::min(a + kLzT, n) - 1;
+        if (t.left[b] + t.count[b] - t.left[a] > kLzSpan) return false;
+    }
+    return std::all_of(t.count.begin(), t.count.end(), [](int c) { return c <= kLzTaps; });
+}
 
 // ---- flattened batch launchers ------------------------------------------------
 
@@ -795,7 +843,6 @@ int launch_lanczos_flat(const BatchPyr& bp, int o, int n_img, const uint32_t* pr
         return -1;
     return cudaPeekAtLastError() == cudaSuccess ? 0 : -1;
 }
-int lanczos_fused_tile() { return kLzT; }
 
 #define SIFT_INST(TG)                                                                                              \
     template int launch_blur_level<TG>(const uint8_t*, int, uint8_t*, TG*, uint8_t*, int, int, int, int,           \
