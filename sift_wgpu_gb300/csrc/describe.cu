@@ -916,8 +916,12 @@ __device__ __forceinline__ void describe_one(const uint8_t* __restrict__ u8arena
 // rows of cells 5 apart 1261. Adding the shares of a pair's two samples at
 // once where they have the same cells and bin made 7 % more instructions and
 // no difference in time; 16 copies (2.1 wavefronts) leave room for 6 CTAs per
-// SM, and 6 took 2.5 % more than 7.
-__global__ void __launch_bounds__(kDescThreads, 7) k_descriptor(const uint8_t* __restrict__ u8arena, EntryTable tab,
+// SM, and 6 took 2.5 % more than 7, which take 1.5 % more than 8 (64 registers,
+// 1232 us at 4096 x 4096). Rows of cells mirrored where that spreads a window
+// row over more banks and 16-byte stores of the grid leave out 7 % of the
+// wavefronts, and change the time by less than 1 %: with 8 CTAs the kernel is
+// as near to the issue slots as to the shared-memory pipe.
+__global__ void __launch_bounds__(kDescThreads, 8) k_descriptor(const uint8_t* __restrict__ u8arena, EntryTable tab,
                                                               const Keypoint* __restrict__ oriented,
                                                               OctCounters* __restrict__ oc,
                                                               float* __restrict__ desc, uint32_t cap,
