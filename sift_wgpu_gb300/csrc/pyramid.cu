@@ -105,6 +105,18 @@ __device__ __forceinline__ void blur_row(const uint8_t* __restrict__ in, int in_
     }
     __syncthreads();
     uint8_t* dst = out + (long long)y * out_pitch;
+    // Short rows: a chain for each output, not four side by side in a quarter
+    // of the threads (more instructions in all: rows of 200 pixels cost the
+    // other octaves' kernels of a 1600 x 900 frame more than they save, 1 %).
+    if (W <= kRowThreads) {
+        if (threadIdx.x >= W) return;
+        const float* p = row + threadIdx.x;
+        float a = 0.0f;
+#pragma unroll 8
+        for (int i = 0; i < taps; ++i) a = __fadd_rn(a, __fmul_rn(p[i], kw[i]));
+        dst[threadIdx.x] = (uint8_t)to_u8(a);
+        return;
+    }
     for (int x0 = threadIdx.x * 4; x0 < W; x0 += blockDim.x * 4) {
         float a0 = 0.0f, a1 = 0.0f, a2 = 0.0f, a3 = 0.0f;
         const float* base = row + x0;  // x0 % 4 == 0 and wpad % 4 == 0: 16-byte aligned
@@ -166,6 +178,8 @@ __global__ void __launch_bounds__(kRowThreads) k_blur_rows(const uint8_t* __rest
 constexpr int kColTX = 32;                 // output columns per CTA
 constexpr int kColRows = 64;               // output rows per CTA
 constexpr int kColThreads = 256;           // 8 column groups of 4 x 32 row groups of 2
+constexpr int kColRowsSmall = 8;           // of a small plane: an output per thread
+constexpr int kColFew = 12;                // 64-row tiles of a small plane, at most
 
 // Vertical pass over a 32 x 64 output tile. Shared layout: weights padded
 // with zeros to a multiple of 8, lut[256] (v / 255 in f32), then
@@ -196,7 +210,7 @@ __device__ __forceinline__ void store_level4<__half>(__half* p, const int v[4], 
     *reinterpret_cast<uint2*>(p) = u;
 }
 
-template <typename TG>
+template <typename TG, int kRows>
 __device__ __forceinline__ void blur_cols_tile(const uint8_t* __restrict__ tmp, int tmp_pitch, TG* __restrict__ out,
                                                uint8_t* __restrict__ out_u8, int pitch, int W, int H, int r,
                                                const float* __restrict__ wts, const float* __restrict__ lut255,
@@ -209,7 +223,7 @@ __device__ __forceinline__ void blur_cols_tile(const uint8_t* __restrict__ tmp, 
     const int tid = threadIdx.x;
     for (int i = tid; i < tp; i += kColThreads) kw[i] = i < taps ? wts[i] : 0.0f;
     for (int i = tid; i < 256; i += kColThreads) lut[i] = lut255[i];
-    const int rows = kColRows + tp - 1;
+    const int rows = kRows + tp - 1;
     if (x0 + kColTX <= W && (tmp_pitch & 15) == 0) {
         // two 16-byte loads per row, all rows of the tile in flight
 #pragma unroll 4
@@ -231,6 +245,19 @@ __device__ __forceinline__ void blur_cols_tile(const uint8_t* __restrict__ tmp, 
         }
     }
     __syncthreads();
+    if constexpr (kRows == kColRowsSmall) {
+        const int x = x0 + (tid & (kColTX - 1)), y = y0 + tid / kColTX;
+        if (x >= W || y >= H) return;
+        const float* p = tile + tid;
+        float a = 0.0f;
+#pragma unroll 8
+        for (int i = 0; i < taps; ++i) a = __fadd_rn(a, __fmul_rn(p[i * kColTX], kw[i]));
+        const int v = to_u8(a);
+        const long long o = (long long)y * pitch + x;
+        store_level(out + o, v, lut[v]);
+        out_u8[o] = (uint8_t)v;
+        return;
+    }
     const int cg = tid & 7, rg = tid >> 3;
     const float4* col = reinterpret_cast<const float4*>(tile) + (2 * rg) * (kColTX / 4) + cg;
     float4 a0 = make_float4(0.0f, 0.0f, 0.0f, 0.0f), a1 = a0;
@@ -277,7 +304,7 @@ __device__ __forceinline__ void blur_cols_tile(const uint8_t* __restrict__ tmp, 
     }
 }
 
-template <typename TG>
+template <typename TG, int kRows>
 __global__ void __launch_bounds__(kColThreads) k_blur_cols(const uint8_t* __restrict__ tmp, int tmp_pitch,
                                                           TG* __restrict__ out, uint8_t* __restrict__ out_u8,
                                                           int pitch, int W, int H, int r,
@@ -285,8 +312,8 @@ __global__ void __launch_bounds__(kColThreads) k_blur_cols(const uint8_t* __rest
                                                           const float* __restrict__ lut255) {
     chain_wait();
     extern __shared__ __align__(16) float sm[];
-    blur_cols_tile<TG>(tmp, tmp_pitch, out, out_u8, pitch, W, H, r, wts, lut255, blockIdx.x * kColTX,
-                       blockIdx.y * kColRows, sm);
+    blur_cols_tile<TG, kRows>(tmp, tmp_pitch, out, out_u8, pitch, W, H, r, wts, lut255, blockIdx.x * kColTX,
+                              blockIdx.y * kRows, sm);
 }
 
 // Fused level kernel: both passes of one level on the tensor cores
@@ -611,7 +638,7 @@ __global__ void __launch_bounds__(kColThreads) kb_blur_cols(BatchPyr bp, const u
     const OctaveDev od = bp.ents[k * bp.O + o];
     const int t = (int)(blockIdx.x - pref[k]), tx = (od.W + kColTX - 1) / kColTX;
     uint8_t* out = bp.U + od.u_off + (long long)s * od.plane;
-    blur_cols_tile<uint8_t>(tmp + od.t_off, od.pitch, out, out, od.pitch, od.W, od.H, r, wts, lut255,
+    blur_cols_tile<uint8_t, kColRows>(tmp + od.t_off, od.pitch, out, out, od.pitch, od.W, od.H, r, wts, lut255,
                             (t % tx) * kColTX, (t / tx) * kColRows, sm);
 }
 
@@ -645,8 +672,8 @@ size_t blur_rows_smem(int W, int r) {
     int taps = 2 * r + 1;
     return sizeof(float) * ((size_t)((taps + 3) & ~3) + (size_t)W + 2 * (size_t)r + 8);
 }
-size_t blur_cols_smem(int r) {
-    return sizeof(float) * ((size_t)taps8(r) + 256 + (size_t)(kColRows + taps8(r) - 1) * kColTX);
+size_t blur_cols_smem(int r, int rows) {
+    return sizeof(float) * ((size_t)taps8(r) + 256 + (size_t)(rows + taps8(r) - 1) * kColTX);
 }
 
 // 64-row tiles from this many on (two per multiprocessor): fewer leave
@@ -713,14 +740,25 @@ int launch_blur_level(const uint8_t* in, int in_pitch, uint8_t* tmp, TG* out, ui
         *launches += 1;
         return 0;
     }
-    const size_t rs = blur_rows_smem(W, r), cs = blur_cols_smem(r);
-    if (set_smem((const void*)k_blur_rows, rs) || set_smem((const void*)k_blur_cols<TG>, cs)) return -1;
+    // Planes with few 64-row tiles take 8-row tiles: an output per thread ends
+    // sooner than eight side by side (with the rows' form, 160 x 120 107 -> 101
+    // us for the frame, 640 x 480 140 -> 137, 1280 x 720, ten tiles, 167 ->
+    // 163). They stage r rows above and below each, so with more of them they
+    // cost the other octaves' kernels more than they save (24, 1080p: 333 -> 335
+    // us; 4096 x 4096 with 128 and 32: 2123 -> 2148, and with 8 of radii 79 to
+    // 198, which stage 50 rows for one, 2120 -> 2128).
+    const int cols = (W + kColTX - 1) / kColTX;
+    const bool small = r <= kColRows && (long long)cols * ((H + kColRows - 1) / kColRows) <= kColFew;
+    const int rows = small ? kColRowsSmall : kColRows;
+    const auto k_cols = small ? k_blur_cols<TG, kColRowsSmall> : k_blur_cols<TG, kColRows>;
+    const size_t rs = blur_rows_smem(W, r), cs = blur_cols_smem(r, rows);
+    if (set_smem((const void*)k_blur_rows, rs) || set_smem((const void*)k_cols, cs)) return -1;
     if (launch_chained(k_blur_rows, H, kRowThreads, rs, st, in, in_pitch, tmp, pitch, W, r, wts, ref) !=
         cudaSuccess)
         return -1;
-    dim3 grid((W + kColTX - 1) / kColTX, (H + kColRows - 1) / kColRows);
-    if (launch_chained(k_blur_cols<TG>, grid, kColThreads, cs, st, tmp, pitch, out, out_u8, pitch, W, H, r, wts,
-                       lut255) != cudaSuccess)
+    dim3 grid(cols, (H + rows - 1) / rows);
+    if (launch_chained(k_cols, grid, kColThreads, cs, st, tmp, pitch, out, out_u8, pitch, W, H, r, wts, lut255) !=
+        cudaSuccess)
         return -1;
     *launches += 2;
     return cudaPeekAtLastError() == cudaSuccess ? 0 : -1;
@@ -821,7 +859,7 @@ int launch_blur_level_flat(const BatchPyr& bp, uint8_t* tmp, int o, int s, int r
         return cudaPeekAtLastError() == cudaSuccess ? 0 : -1;
     }
     if (n_rows == 0) return 0;
-    const size_t rs = blur_rows_smem(max_w, r), cs = blur_cols_smem(r);
+    const size_t rs = blur_rows_smem(max_w, r), cs = blur_cols_smem(r, kColRows);
     if (set_smem((const void*)kb_blur_rows, rs) || set_smem((const void*)kb_blur_cols, cs)) return -1;
     if (launch_chained(kb_blur_rows, n_rows, kRowThreads, rs, st, bp, tmp, o, s, r, n_img, rows_pref, wts) !=
         cudaSuccess)
