@@ -346,7 +346,7 @@ int sift_cuda_replay(SiftCudaServer* server, const SiftCudaParams* params, const
  * whose GPU arms take one image per call). Each stage of the hot path is one
  * launch over the flattened work of every image: the pyramid one launch per
  * (octave, level) over the tiles of that octave of all images, then
- * extrema, candidate scan, emission, refinement, orientation, oriented
+ * extrema, candidates with their refinement, orientation, oriented
  * keypoints and descriptors one launch each over all (image, octave)
  * entries; the run is captured once per batch geometry as a CUDA graph. Every
  * image's keypoints and descriptors are those of sift_cuda_detect_and_compute

@@ -6,7 +6,7 @@
 //              plane pitch x H (pitch = width rounded up to 32 elements), f32
 //              or f16 (u8-valued either way)
 //   U arena    (S+3) u8 planes per octave: every level as bytes, the input
-//              of the next level, of the resize and of the extrema mask
+//              of the next level, of the resize and of every later stage
 //   tmp        one u8 plane for the horizontal blur pass (largest octave)
 //   ltmp       one f32 plane for the vertical Lanczos pass
 //   mask       per octave S x H x ceil(W/32) ballot words of extrema
