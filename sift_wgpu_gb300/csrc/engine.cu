@@ -13,7 +13,10 @@ int fail(int code, const std::string& msg) {
     return code;
 }
 
+// The runtime keeps the error until it is read, and the launchers look there
+// (cudaPeekAtLastError): reported here, it is not the next call's.
 int cuda_fail(cudaError_t e, const char* what) {
+    cudaGetLastError();
     std::string m = std::string(what) + ": " + cudaGetErrorName(e) + " (" + cudaGetErrorString(e) + ")";
     return fail(e == cudaErrorMemoryAllocation ? SIFT_CUDA_ERR_OUT_OF_MEMORY
                                                : (e == cudaErrorNoDevice || e == cudaErrorInsufficientDriver
