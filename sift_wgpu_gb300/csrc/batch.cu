@@ -611,7 +611,10 @@ extern "C" int sift_cuda_batch_detect_and_compute(SiftCudaBatch* batch, const Si
     std::memset(out, 0, sizeof *out);
     if (n == 0) return 0;
     sift::BatchEngine& b = batch->b;
-    if (int rc = b.detect(images, n)) return rc;
+    if (int rc = b.detect(images, n)) {
+        cudaStreamSynchronize(b.st);  // kernels read the caller's images
+        return rc;
+    }
     out->n_images = n;
     out->total = b.n_out;
     out->offsets = reinterpret_cast<const uint32_t*>(b.hx.as<char>() + b.hx_ranges_off());

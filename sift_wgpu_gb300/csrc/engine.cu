@@ -287,13 +287,8 @@ int sift_cuda_match_device(const float* d_query, uint32_t n_query, const float* 
     return 0;
 }
 
-int sift_cuda_match(SiftCudaEngine* engine, const float* query, uint32_t n_query, const float* train,
-                    uint32_t n_train, SiftCudaMatch* out) {
-    sift::g_last_error.clear();
-    if (!engine) return sift::fail(SIFT_CUDA_ERR_INVALID_ARGUMENT, "engine is NULL");
-    if (n_query == 0) return 0;
-    if (!query || !out || (n_train && !train)) return sift::fail(SIFT_CUDA_ERR_INVALID_ARGUMENT, "a matching buffer is NULL");
-    Engine& e = engine->e;
+static int match_host(Engine& e, const float* query, uint32_t n_query, const float* train, uint32_t n_train,
+                      SiftCudaMatch* out) {
     if (int rc = e.set_device()) return rc;
     const size_t qb = (size_t)n_query * sift::kDescLen * sizeof(float), tb = (size_t)n_train * sift::kDescLen * sizeof(float);
     const size_t ob = (size_t)n_query * sizeof(SiftCudaMatch);
@@ -326,6 +321,17 @@ int sift_cuda_match(SiftCudaEngine* engine, const float* query, uint32_t n_query
     if (!err) std::memcpy(out, e.h_mo.as<char>() + 256, ob);
     if (err) return sift::fail(SIFT_CUDA_ERR_CUDA, "matching: a tensor-core pipeline wait ran out (no results)");
     return 0;
+}
+
+int sift_cuda_match(SiftCudaEngine* engine, const float* query, uint32_t n_query, const float* train,
+                    uint32_t n_train, SiftCudaMatch* out) {
+    sift::g_last_error.clear();
+    if (!engine) return sift::fail(SIFT_CUDA_ERR_INVALID_ARGUMENT, "engine is NULL");
+    if (n_query == 0) return 0;
+    if (!query || !out || (n_train && !train)) return sift::fail(SIFT_CUDA_ERR_INVALID_ARGUMENT, "a matching buffer is NULL");
+    const int rc = match_host(engine->e, query, n_query, train, n_train, out);
+    if (rc) cudaStreamSynchronize(engine->e.st);  // the norm kernel reads the caller's rows
+    return rc;
 }
 
 int sift_cuda_draw_keypoints(SiftCudaEngine* engine, const uint8_t* gray, uint32_t width, uint32_t height,

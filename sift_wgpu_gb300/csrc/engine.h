@@ -1027,8 +1027,18 @@ struct Engine {
         return 0;
     }
 
+    // A call that fails waits for what it has launched: kernels read the
+    // caller's image (k_fetch, the luma conversion, an in-place base level),
+    // which the caller may free as soon as the call returns.
     int detect_host(const uint8_t* img, uint32_t w, uint32_t h, uint32_t stride, bool with_desc,
                     SiftCudaResult* out, bool view = false, int format = SIFT_CUDA_PIXELS_GRAY8) {
+        const int rc = detect_image(img, w, h, stride, with_desc, out, view, format);
+        if (rc) cudaStreamSynchronize(st);
+        return rc;
+    }
+
+    int detect_image(const uint8_t* img, uint32_t w, uint32_t h, uint32_t stride, bool with_desc,
+                     SiftCudaResult* out, bool view, int format) {
         if (int rc = set_device()) return rc;
         if (int rc = ensure_geometry(w, h)) return rc;
         if (format == SIFT_CUDA_PIXELS_GRAY8) {

@@ -331,7 +331,10 @@ struct Server {
         return 0;
     }
 
+    // (What the request has launched may still read its image, which its
+    // owner may free once the request is polled: waited for.)
     void fail_request(Request* r, int rc) {
+        if (r->slot) cudaStreamSynchronize(r->slot->eng->st);
         r->status = rc ? rc : SIFT_CUDA_ERR_CUDA;
         r->t_done = now_s();
         if (r->slot && r->slot->state == Slot::Running) {

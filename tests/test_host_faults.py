@@ -90,3 +90,116 @@ def test_the_error_of_a_failed_call_is_not_the_next_ones(fake, api):
     assert fake.detect(h, img)[0] == 0
     fake.lib.sift_cuda_destroy(h)
     fake.lib.sift_cuda_destroy(fake.engine())
+
+
+READS_CALLER = ("k_fetch", "k_to_luma", "k_sq_norms", "cudaGraphLaunch")
+
+
+def waited(log):
+    """Whether a stream wait follows the last launch that may read the caller's memory; None without one."""
+    for line in reversed(log):
+        if line.startswith("cudaStreamSynchronize"):
+            return True
+        if any(k in line for k in READS_CALLER) and not line.startswith("failed"):
+            return False
+    return None
+
+
+# ---- a call that fails leaves no kernel that reads the caller's memory ------
+
+AFTER_UPLOAD = ["cudaHostAlloc", "cudaStreamBeginCapture", "cudaStreamEndCapture", "cudaGraphInstantiate",
+                "cudaGraphLaunch"]
+
+
+@pytest.mark.parametrize("api", AFTER_UPLOAD)
+@pytest.mark.parametrize("shape,start", [((1024, 1040), 0), ((40, 50), 3)])
+def test_failed_detection_has_let_go_of_the_image(fake, api, shape, start):
+    h = fake.engine()
+    fake.log()
+    fake.fail(api)
+    rc, _ = fake.detect(h, aligned(shape, start=start))
+    log = fake.log()
+    assert rc != 0 and any("k_fetch" in line for line in log)
+    assert waited(log)
+    rc, _ = fake.detect(h, aligned(shape, start=start))
+    assert rc == 0
+    fake.lib.sift_cuda_destroy(h)
+
+
+@pytest.mark.parametrize("api", AFTER_UPLOAD)
+def test_failed_colour_detection_has_let_go_of_the_pixels(fake, api):
+    px = aligned((30, 40, 4))
+    h, r = fake.engine(), _capi.Result()
+    fake.log()
+    fake.fail(api)
+    rc = fake.lib.sift_cuda_detect_and_compute_pixels(h, px.ctypes.data, 40, 30, 160, _capi.PIXELS_RGBA8, C.byref(r))
+    log = fake.log()
+    assert rc != 0 and any("k_to_luma" in line for line in log)
+    assert waited(log)
+    fake.lib.sift_cuda_destroy(h)
+
+
+def test_failed_match_has_let_go_of_the_rows(fake):
+    rows, out = aligned((5, 128), np.float32), np.zeros(5, _capi.MATCH_DTYPE)
+    h = fake.engine()
+    for api in ("encode", "cudaFuncSetAttribute"):
+        fake.log()
+        fake.fail(api)
+        rc = fake.lib.sift_cuda_match(h, rows.ctypes.data, 5, rows.ctypes.data, 5, out.ctypes.data)
+        log = fake.log()
+        assert rc != 0 and any("k_sq_norms" in line for line in log)
+        assert waited(log), api
+    fake.lib.sift_cuda_destroy(h)
+
+
+@pytest.mark.parametrize("nth", [1, 2])
+def test_failed_batch_has_let_go_of_the_images(fake, nth):
+    """A batch reads its images in place from its graph; the event after it fails (the first is before it)."""
+    p, o, h, res = _capi.Params(), _capi.Options(), C.c_void_p(), _capi.BatchResult()
+    fake.lib.sift_cuda_params_default(C.byref(p))
+    fake.lib.sift_cuda_options_default(C.byref(o))
+    assert fake.lib.sift_cuda_batch_create(C.byref(p), C.byref(o), C.byref(h)) == 0
+    img = aligned((32, 64))
+    ims = (_capi.BatchImage * 1)(_capi.BatchImage(img.ctypes.data, 64, 32, 64))
+    for _ in range(2):
+        fake.log()
+        assert fake.lib.sift_cuda_batch_detect_and_compute(h, ims, 1, C.byref(res)) == 0
+    events = sum(line == "cudaEventRecord" for line in fake.log())
+    assert events == 2
+    fake.fail("cudaEventRecord", nth)
+    assert fake.lib.sift_cuda_batch_detect_and_compute(h, ims, 1, C.byref(res)) != 0
+    assert waited(fake.log()) is not False
+    fake.lib.sift_cuda_batch_destroy(h)
+
+
+@pytest.mark.parametrize("api", ["cudaHostAlloc", "cudaGraphInstantiate", "cudaGraphLaunch", "done event"])
+@pytest.mark.parametrize("autotune", [0, 1])
+def test_failed_request_has_let_go_of_a_borrowed_image(fake, api, autotune):
+    p, o, h = _capi.Params(), _capi.ServerOptions(), C.c_void_p()
+    fake.lib.sift_cuda_params_default(C.byref(p))
+    fake.lib.sift_cuda_server_options_default(C.byref(o))
+    o.autotune = autotune
+    assert fake.lib.sift_cuda_server_create(C.byref(p), C.byref(o), C.byref(h)) == 0
+    img, ticket, served = aligned((40, 50), start=3), C.c_uint64(), _capi.Served()
+
+    def request():
+        fake.log()
+        assert fake.lib.sift_cuda_server_submit(h, img.ctypes.data, 50, 40, 50, 7, 1, C.byref(ticket)) == 0
+        assert fake.lib.sift_cuda_server_poll(h, C.byref(served), 10_000_000) == 1
+        log = fake.log()
+        assert fake.lib.sift_cuda_server_release(h, ticket) == 0
+        return served.status, log
+
+    if api == "done event":
+        status, log = request()  # a slot, tuned and captured
+        assert status == 0
+        fake.fail("cudaEventRecord")
+    elif api == "cudaHostAlloc":
+        # (the slot's own are in its creation: counters, cell)
+        fake.fail(api, 3)
+    else:
+        fake.fail(api)
+    status, log = request()
+    assert status != 0 and any("k_fetch" in line for line in log)
+    assert waited(log)
+    fake.lib.sift_cuda_server_destroy(h)
