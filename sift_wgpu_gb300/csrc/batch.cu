@@ -170,9 +170,12 @@ struct BatchEngine {
         return 0;
     }
 
-    // Arenas, tables and work-list prefixes for images of these sizes.
+    // Arenas, tables and work-list prefixes for images of these sizes. A
+    // layout holds (dims) once its last list exists; one that failed on the
+    // way is made again by the next call, whatever its sizes.
     int ensure_geometry(const std::vector<std::pair<uint32_t, uint32_t>>& d) {
         if (!ents.empty() && d == dims) return 0;
+        dims.clear();
         drop_graph();
         O = (int)p.num_octaves;
         S = (int)p.num_intervals;
@@ -321,14 +324,15 @@ struct BatchEngine {
             CK(cudaMemcpyAsync(d_lw.p, ftab.data(), sizeof(float) * ftab.size(), cudaMemcpyHostToDevice, st), "H2D");
         CK(cudaMemcpyAsync(d_lz.p, lz.data(), lz.size(), cudaMemcpyHostToDevice, st), "H2D lanczos jobs");
         CK(cudaStreamSynchronize(st), "table upload");
-        dims = d;
         // list capacities: 1/64 of the scanned positions, at least 1024 per entry
         size_t cc = 0;
         for (const auto& od : ents)
             cc += std::min<size_t>(std::max<size_t>((size_t)S * od.H * od.nw * 32 / 64, 1024), 1u << 28);
         cap_cand = (uint32_t)std::min<size_t>(cc, 1u << 30);
         cap_ori = std::max(cap_ori, cap_cand);
-        return ensure_lists();
+        if (int rc = ensure_lists()) return rc;
+        dims = d;
+        return 0;
     }
 
     int ensure_lists() {
@@ -348,9 +352,16 @@ struct BatchEngine {
         return 0;
     }
 
-    // Mapped export buffer for at least n keypoints of this batch geometry.
+    // Mapped export buffer for at least n keypoints of this batch geometry
+    // (none if a step fails).
     int ensure_export(uint32_t n, bool geometry_changed) {
         if (hx.p && n <= cap_x && !geometry_changed) return 0;
+        const int rc = make_export(n);
+        if (rc) hx.release();
+        return rc;
+    }
+
+    int make_export(uint32_t n) {
         drop_graph();
         cap_x = std::max<uint32_t>(std::max<uint32_t>(2 * n + 4096, cap_x), 4096);
         hx.release();
@@ -552,7 +563,10 @@ struct BatchEngine {
                 grow = true;
             }
             if (grow) {
-                if (int rc = ensure_lists()) return rc;
+                if (int rc = ensure_lists()) {
+                    dims.clear();
+                    return rc;
+                }
                 continue;
             }
             if (c.oct[0].n_ori > cap_x) {  // more keypoints than the export buffer holds: grow it, run again

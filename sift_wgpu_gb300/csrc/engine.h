@@ -484,8 +484,12 @@ struct Engine {
     long long octave_words(int o) const { return (long long)pyr.S * pyr.oct[o].H * pyr.oct[o].nw; }
 
     // Lays out the arena for a width x height image and builds the tables.
+    // A layout holds (have_geom) once its last list exists: a step that fails
+    // on the way leaves none, and the next call lays out again, whatever its
+    // size.
     int ensure_geometry(uint32_t w, uint32_t h) {
         if (have_geom && w == W && h == H) return 0;
+        have_geom = false;
         const int O = (int)p.num_octaves, S = (int)p.num_intervals;
         if (O > kMaxOctaves) return fail(SIFT_CUDA_ERR_UNSUPPORTED, "num_octaves above 16 is not supported");
         PyramidDev g{};
@@ -601,7 +605,6 @@ struct Engine {
         tb = tbo;
         W = w;
         H = h;
-        have_geom = true;
         // Initial list capacities: 1/64 of each octave's scanned positions
         // (measured densities on natural and synthetic images are far below
         // it), at least 1024; grown on overflow.
@@ -615,6 +618,7 @@ struct Engine {
     }
 
     int ensure_lists() {
+        have_geom = false;
         drop_graph();
         const int O = pyr.num_octaves;
         cb.assign(O, 0);
@@ -639,6 +643,7 @@ struct Engine {
         CK(d_oriented.ensure((size_t)cap_ori * kp), "cudaMalloc(oriented)");
         CK(d_desc.ensure((size_t)cap_ori * kDescLen * sizeof(float)), "cudaMalloc(desc)");
         CK(d_tiles.ensure(align_up(std::max<size_t>(pp, 1), 4) * sizeof(uint32_t)), "cudaMalloc(tile counts)");
+        have_geom = true;
         return 0;
     }
 

@@ -286,6 +286,7 @@ struct Server {
 
     int launch(Slot* s, Request* r) {
         Engine& e = *s->eng;
+        if (int rc = e.ensure_geometry(s->w, s->h)) return rc;  // again if its lists failed to grow
         if (int rc = e.upload(r->img, r->w, r->h, r->stride, cudaMemcpyHostToDevice)) return rc;
         bool tune = false;
         if (opt.autotune) {

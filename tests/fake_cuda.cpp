@@ -55,8 +55,9 @@ cudaError_t call(const char* api, const std::string& what = "") {
 void act(const Launch& l) {
     if (l.name.find("k_begin") != std::string::npos) {
         std::memcpy(l.args[1], l.args[0], 48);  // RunCell
-    } else if (l.name.find("k_export") != std::string::npos) {
-        uint32_t* ctr = *reinterpret_cast<uint32_t**>(static_cast<char*>(l.args[2]) + 16);
+    } else {  // k_export: the cell's counters; k_batch_export: its own argument's
+        uint32_t* ctr = static_cast<uint32_t*>(l.args[0]);
+        if (l.name.find("k_batch") == std::string::npos) ctr = *reinterpret_cast<uint32_t**>(static_cast<char*>(l.args[2]) + 16);
         for (auto& c : counters) ctr[c.first] = c.second;
     }
 }
@@ -69,6 +70,8 @@ cudaError_t launch(const void* func, dim3 grid, void** args) {
         return e;
     if (l.name.find("k_begin") != std::string::npos || l.name.find("k_export") != std::string::npos)
         for (int i = 0; i < 3; ++i) l.args.push_back(*static_cast<void**>(args[i]));
+    else if (l.name.find("k_batch_export") != std::string::npos)
+        l.args.push_back(*static_cast<void**>(args[10]));
     if (capturing)
         graph_of_capture->push_back(l);
     else if (!l.args.empty())

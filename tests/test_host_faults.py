@@ -43,6 +43,38 @@ class Fake:
         assert self.lib.sift_cuda_create(C.byref(params or p), C.byref(o), C.byref(h)) == 0
         return h
 
+    def batch(self):
+        p, o, h = _capi.Params(), _capi.Options(), C.c_void_p()
+        self.lib.sift_cuda_params_default(C.byref(p))
+        self.lib.sift_cuda_options_default(C.byref(o))
+        assert self.lib.sift_cuda_batch_create(C.byref(p), C.byref(o), C.byref(h)) == 0
+        return h
+
+    def detect_batch(self, h, img):
+        res = _capi.BatchResult()
+        one = (_capi.BatchImage * 1)(_capi.BatchImage(img.ctypes.data, img.shape[1], img.shape[0], img.strides[0]))
+        return self.lib.sift_cuda_batch_detect_and_compute(h, one, 1, C.byref(res))
+
+    def server(self, **options):
+        p, o, h = _capi.Params(), _capi.ServerOptions(), C.c_void_p()
+        self.lib.sift_cuda_params_default(C.byref(p))
+        self.lib.sift_cuda_server_options_default(C.byref(o))
+        for k, v in options.items():
+            setattr(o, k, v)
+        assert self.lib.sift_cuda_server_create(C.byref(p), C.byref(o), C.byref(h)) == 0
+        return h
+
+    def request(self, h, img):
+        """A borrowed image's request: its status, and the log from submit to poll."""
+        ticket, served = C.c_uint64(), _capi.Served()
+        self.log()
+        assert self.lib.sift_cuda_server_submit(h, img.ctypes.data, img.shape[1], img.shape[0], img.strides[0], 7, 1,
+                                                C.byref(ticket)) == 0
+        assert self.lib.sift_cuda_server_poll(h, C.byref(served), 10_000_000) == 1
+        log = self.log()
+        assert self.lib.sift_cuda_server_release(h, ticket) == 0
+        return served.status, log
+
     def detect(self, h, img):
         r = _capi.Result()
         rc = self.lib.sift_cuda_detect_and_compute(h, img.ctypes.data, img.shape[1], img.shape[0], img.strides[0],
@@ -155,19 +187,13 @@ def test_failed_match_has_let_go_of_the_rows(fake):
 @pytest.mark.parametrize("nth", [1, 2])
 def test_failed_batch_has_let_go_of_the_images(fake, nth):
     """A batch reads its images in place from its graph; the event after it fails (the first is before it)."""
-    p, o, h, res = _capi.Params(), _capi.Options(), C.c_void_p(), _capi.BatchResult()
-    fake.lib.sift_cuda_params_default(C.byref(p))
-    fake.lib.sift_cuda_options_default(C.byref(o))
-    assert fake.lib.sift_cuda_batch_create(C.byref(p), C.byref(o), C.byref(h)) == 0
-    img = aligned((32, 64))
-    ims = (_capi.BatchImage * 1)(_capi.BatchImage(img.ctypes.data, 64, 32, 64))
+    h, img = fake.batch(), aligned((32, 64))
     for _ in range(2):
         fake.log()
-        assert fake.lib.sift_cuda_batch_detect_and_compute(h, ims, 1, C.byref(res)) == 0
-    events = sum(line == "cudaEventRecord" for line in fake.log())
-    assert events == 2
+        assert fake.detect_batch(h, img) == 0
+    assert sum(line == "cudaEventRecord" for line in fake.log()) == 2
     fake.fail("cudaEventRecord", nth)
-    assert fake.lib.sift_cuda_batch_detect_and_compute(h, ims, 1, C.byref(res)) != 0
+    assert fake.detect_batch(h, img) != 0
     assert waited(fake.log()) is not False
     fake.lib.sift_cuda_batch_destroy(h)
 
@@ -175,31 +201,134 @@ def test_failed_batch_has_let_go_of_the_images(fake, nth):
 @pytest.mark.parametrize("api", ["cudaHostAlloc", "cudaGraphInstantiate", "cudaGraphLaunch", "done event"])
 @pytest.mark.parametrize("autotune", [0, 1])
 def test_failed_request_has_let_go_of_a_borrowed_image(fake, api, autotune):
-    p, o, h = _capi.Params(), _capi.ServerOptions(), C.c_void_p()
-    fake.lib.sift_cuda_params_default(C.byref(p))
-    fake.lib.sift_cuda_server_options_default(C.byref(o))
-    o.autotune = autotune
-    assert fake.lib.sift_cuda_server_create(C.byref(p), C.byref(o), C.byref(h)) == 0
-    img, ticket, served = aligned((40, 50), start=3), C.c_uint64(), _capi.Served()
-
-    def request():
-        fake.log()
-        assert fake.lib.sift_cuda_server_submit(h, img.ctypes.data, 50, 40, 50, 7, 1, C.byref(ticket)) == 0
-        assert fake.lib.sift_cuda_server_poll(h, C.byref(served), 10_000_000) == 1
-        log = fake.log()
-        assert fake.lib.sift_cuda_server_release(h, ticket) == 0
-        return served.status, log
-
+    h, img = fake.server(autotune=autotune), aligned((40, 50), start=3)
     if api == "done event":
-        status, log = request()  # a slot, tuned and captured
+        status, log = fake.request(h, img)  # a slot, tuned and captured
         assert status == 0
         fake.fail("cudaEventRecord")
     elif api == "cudaHostAlloc":
-        # (the slot's own are in its creation: counters, cell)
-        fake.fail(api, 3)
+        fake.fail(api, 3)  # (two are made with the slot: counters, cell)
     else:
         fake.fail(api)
-    status, log = request()
+    status, log = fake.request(h, img)
     assert status != 0 and any("k_fetch" in line for line in log)
     assert waited(log)
     fake.lib.sift_cuda_server_destroy(h)
+
+
+# ---- a layout that failed half-way is laid out again -------------------------
+
+SMALL, LARGE = (48, 64), (120, 160)
+N_CAND = 8  # the word of octave 0's candidate count in a run's counters
+
+
+def failures(api, attempt):
+    """attempt(fail) with the 1st, 2nd, .. call of the api failing, until none is left; their number."""
+    for nth in range(1, 200):
+        if not attempt(nth):
+            return nth - 1
+    raise AssertionError(api)
+
+
+@pytest.mark.parametrize("api", ["cudaMalloc", "cudaMemcpyAsync"])
+@pytest.mark.parametrize("again", [SMALL, LARGE])
+def test_engine_lays_out_again_after_a_failed_layout(fake, api, again):
+    small, large = aligned(SMALL), aligned(LARGE)
+
+    def attempt(nth):
+        h = fake.engine()
+        assert fake.detect(h, small)[0] == 0
+        buffers = fake.lib.fake_live_device()
+        fake.log()
+        fake.fail(api, nth)
+        failed = fake.detect(h, large)[0] != 0
+        fake.lib.fake_reset()
+        assert fake.detect(h, small if again == SMALL else large)[0] == 0
+        # every buffer exists, and the tables are the small size's again
+        assert fake.lib.fake_live_device() == buffers
+        assert again == LARGE or "cudaMemcpyAsync" in fake.log()
+        fake.lib.sift_cuda_destroy(h)
+        return failed
+
+    assert failures(api, attempt) >= 4
+
+
+def test_engine_lays_out_again_after_lists_failed_to_grow(fake):
+    img = aligned(SMALL)
+
+    def attempt(nth):
+        h = fake.engine()
+        assert fake.detect(h, img)[0] == 0
+        buffers = fake.lib.fake_live_device()
+        fake.lib.fake_counter(N_CAND, 100_000)
+        fake.fail("cudaMalloc", nth)
+        failed = fake.detect(h, img)[0] != 0
+        fake.lib.fake_reset()
+        assert fake.detect(h, img)[0] == 0
+        assert fake.lib.fake_live_device() == buffers
+        fake.lib.sift_cuda_destroy(h)
+        return failed
+
+    assert failures("cudaMalloc", attempt) >= 4
+
+
+def test_server_lays_out_again_after_lists_failed_to_grow(fake):
+    img = aligned(SMALL)
+
+    def attempt(nth):
+        h = fake.server()
+        assert fake.request(h, img)[0] == 0
+        buffers = fake.lib.fake_live_device()
+        fake.lib.fake_counter(N_CAND, 100_000)
+        fake.fail("cudaMalloc", nth)
+        failed = fake.request(h, img)[0] != 0
+        fake.lib.fake_reset()
+        assert fake.request(h, img)[0] == 0
+        assert fake.lib.fake_live_device() == buffers
+        fake.lib.sift_cuda_server_destroy(h)
+        return failed
+
+    assert failures("cudaMalloc", attempt) >= 4
+
+
+@pytest.mark.parametrize("api", ["cudaMalloc", "cudaMemcpyAsync", "cudaHostAlloc", "cudaHostGetDevicePointer"])
+@pytest.mark.parametrize("again", [SMALL, LARGE])
+def test_batch_lays_out_again_after_a_failed_layout(fake, api, again):
+    small, large = aligned(SMALL), aligned(LARGE)
+
+    def attempt(nth):
+        h = fake.batch()
+        assert fake.detect_batch(h, small) == 0
+        buffers = fake.lib.fake_live_device()
+        fake.fail(api, nth)
+        failed = fake.detect_batch(h, large) != 0
+        fake.lib.fake_reset()
+        assert fake.detect_batch(h, small if again == SMALL else large) == 0
+        log = fake.log()
+        assert fake.lib.fake_live_device() == buffers
+        # the result buffer is this layout's: its parts depend on it, and none is left of one that failed
+        if again == SMALL or (failed and api.startswith("cudaHost")):
+            assert "cudaHostAlloc" in log
+        fake.lib.sift_cuda_batch_destroy(h)
+        return failed
+
+    assert failures(api, attempt) >= 1
+
+
+def test_batch_lays_out_again_after_lists_failed_to_grow(fake):
+    img = aligned(SMALL)
+
+    def attempt(nth):
+        h = fake.batch()
+        assert fake.detect_batch(h, img) == 0
+        buffers = fake.lib.fake_live_device()
+        fake.lib.fake_counter(N_CAND, 100_000)
+        fake.fail("cudaMalloc", nth)
+        failed = fake.detect_batch(h, img) != 0
+        fake.lib.fake_reset()
+        assert fake.detect_batch(h, img) == 0
+        assert fake.lib.fake_live_device() == buffers
+        fake.lib.sift_cuda_batch_destroy(h)
+        return failed
+
+    assert failures("cudaMalloc", attempt) >= 4
