@@ -465,6 +465,7 @@ __device__ __forceinline__ int warp_pairs(WarpPairs* w, float ca, float sa, floa
     const float hx = (lim + 0.01f) * fabsf(ic), hy = (lim + 0.01f) * fabsf(is);
     const float rad_f = (float)rad;
     if (lane < kWarpWords) w->start[lane] = 0u;
+    __syncwarp();  // the zeroes before any lane's atomicOr (shuffles and ballots do not order memory)
     // lane l: row 4 (l % 16) + warp (the lanes above 15 repeat them)
     const int q = 4 * (lane & (kWarpRows - 1)) + warp, p = (q + 1) & 1;
     const float py = (float)q - rad_f, shift = rad_f + (float)p, end = rad_f + 1.0f;
