@@ -1014,14 +1014,14 @@ struct Engine {
         //  - anything else: copied to d_img.
         const uint8_t* src = nullptr;
         bool direct = false;
-        image_in_place = false;
         if (kind == cudaMemcpyHostToDevice && img && w && h && stride <= (1u << 30)) {
             bool pageable = false;
             const uint8_t* p = device_reads(img, &pageable);
             if (pageable) src = p;
-            image_in_place = pageable && ((uintptr_t)img & 15) == 0 && (stride & 15) == 0;
-            direct = image_in_place && base.sigma > 0.0f && (size_t)w * h < kFetchFrom;
+            direct = pageable && ((uintptr_t)img & 15) == 0 && (stride & 15) == 0 && base.sigma > 0.0f &&
+                     (size_t)w * h < kFetchFrom;
         }
+        image_in_place = direct;
         if (src && !direct) {
             if (launch_fetch(src, (long long)stride, d_img.as<uint8_t>(), (long long)img_pitch, (int)w, (int)h, st))
                 return cuda_fail(cudaGetLastError(), "fetch image");

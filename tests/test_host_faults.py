@@ -332,3 +332,25 @@ def test_batch_lays_out_again_after_lists_failed_to_grow(fake):
         return failed
 
     assert failures("cudaMalloc", attempt) >= 4
+
+
+# ---- where a run read its image ----------------------------------------------
+
+@pytest.mark.parametrize("shape,start,sigma,in_place", [
+    ((40, 64), 0, 1.6, 1), ((1023, 1024), 0, 1.6, 1),
+    ((1024, 1024), 0, 1.6, 0),  # brought in by a kernel of its own
+    ((2048, 2064), 0, 1.6, 0),
+    ((40, 64), 0, 0.5, 0),      # no base blur: the copy is read
+    ((40, 64), 1, 1.6, 0), ((40, 50), 0, 1.6, 0)])
+def test_in_place_says_where_the_run_read_the_image(fake, shape, start, sigma, in_place):
+    p = _capi.Params()
+    fake.lib.sift_cuda_params_new(C.byref(p), sigma, 1, 1, 0.5, 0.04, 10.0)
+    h = fake.engine(p)
+    assert fake.detect(h, aligned(shape, start=start))[0] == 0
+    assert any("k_fetch" in line for line in fake.log()) != bool(in_place)
+    assert fake.lib.sift_cuda_last_image_in_place(h) == in_place
+    px, r = aligned((30, 40, 4)), _capi.Result()  # colour pixels become the engine's own plane
+    assert fake.lib.sift_cuda_detect_and_compute_pixels(h, px.ctypes.data, 40, 30, 160, _capi.PIXELS_RGBA8,
+                                                        C.byref(r)) == 0
+    assert fake.lib.sift_cuda_last_image_in_place(h) == 0
+    fake.lib.sift_cuda_destroy(h)
