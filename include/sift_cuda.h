@@ -96,9 +96,9 @@ typedef enum {
 typedef struct {
     int32_t device;          /* CUDA device ordinal */
     int32_t storage;         /* SiftCudaStorage (default SIFT_CUDA_STORAGE_U8) */
-    int32_t level_tile_rows; /* rows of the fused level kernel's tiles: 0 (default) or 64: 64-row tiles on planes
-                                that fill the device with them and 32-row tiles on smaller ones; 32: 32-row
-                                tiles on every plane; the output is the same (the batched form uses 64) */
+    int32_t level_tile_rows; /* rows of the fused level kernel's tiles: 0 (default): 64-row tiles on planes that
+                                fill the device with them and 32-row tiles on smaller ones; 64 or 32: those on
+                                every plane; the output is the same (the batched form uses 64) */
     uint32_t reserved[5];
 } SiftCudaOptions;
 
@@ -309,8 +309,9 @@ int sift_cuda_server_stats(SiftCudaServer* server, SiftCudaServerStats* out);
  * orientation CTAs/SM, descriptor CTAs/SM]; returns 1 if tuned, 0 if default. */
 int sift_cuda_server_tuning(SiftCudaServer* server, uint32_t width, uint32_t height, int32_t* knobs3);
 /* The same with every knob: writes the first min(n_knobs, 4) of [fused blur
- * radius limit, fused level tile rows (64 or 32), orientation CTAs/SM,
- * descriptor CTAs/SM]; returns 1 if tuned, 0 if default. */
+ * radius limit, fused level tile rows (64: on planes that fill the device with
+ * them, 32 on smaller ones; 32: everywhere), orientation CTAs/SM, descriptor
+ * CTAs/SM]; returns 1 if tuned, 0 if default. */
 int sift_cuda_server_tuning_knobs(SiftCudaServer* server, uint32_t width, uint32_t height, int32_t* knobs,
                                   uint32_t n_knobs);
 /* Device bytes a slot for a width x height image holds (admission estimate). */

@@ -158,7 +158,7 @@ int sift_cuda_create(const SiftCudaParams* params, const SiftCudaOptions* opts, 
     if (!eng) return sift::fail(SIFT_CUDA_ERR_OUT_OF_MEMORY, "engine allocation");
     eng->e.p = *params;
     eng->e.opt = o;
-    if (o.level_tile_rows) eng->e.tune.level_tile_rows = o.level_tile_rows;
+    eng->e.tune.level_tile_rows = o.level_tile_rows;
     if (int rc = eng->e.init()) {
         delete eng;
         return rc;

@@ -43,7 +43,7 @@ template <typename TG>
 int launch_blur_level(const uint8_t* in, int in_pitch, uint8_t* tmp, TG* out, uint8_t* out_u8, int pitch, int W,
                       int H, int r, const float* wts, const TcBlur& b, const void* frags, const float* lut255,
                       cudaStream_t st, int* launches, int fused_max_radius, const ImgRef* ref = nullptr,
-                      int tile_rows = 64);
+                      int tile_rows = 0);
 template <typename TG>
 int launch_copy_level(const TG* prev, const uint8_t* prev_u8, TG* out, uint8_t* out_u8, int pitch, int W,
                       int H, cudaStream_t st);
@@ -310,13 +310,13 @@ struct Engine {
     // tuned values for single 1080p..4096 images): the largest blur radius
     // that runs as one fused kernel (8: every radius it takes), the
     // persistent grids of the orientation and descriptor kernels in CTAs per
-    // SM, and the height of the fused level kernel's tiles (64: by the
-    // plane's size; 32: always 32 rows).
+    // SM, and the height of the fused level kernel's tiles (0: by the plane's
+    // size; 64 or 32: those everywhere).
     struct Tuning {
         int fused_max_radius = 8;
         int ori_ctas_per_sm = 4;
         int desc_ctas_per_sm = 8;
-        int level_tile_rows = 64;
+        int level_tile_rows = 0;
         bool operator==(const Tuning& o) const {
             return fused_max_radius == o.fused_max_radius && ori_ctas_per_sm == o.ori_ctas_per_sm &&
                    desc_ctas_per_sm == o.desc_ctas_per_sm && level_tile_rows == o.level_tile_rows;

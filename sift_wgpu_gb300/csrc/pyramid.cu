@@ -726,10 +726,13 @@ int launch_blur_level(const uint8_t* in, int in_pitch, uint8_t* tmp, TG* out, ui
     if (level_fused(b, r, fused_max_radius)) {
         const TcParams tp{static_cast<const uint4*>(frags), wts, r, b.init_a, b.init_b, b.scale_b, b.whole, b.near};
         // planes whose 64-row tiles would leave multiprocessors idle take 32-row tiles
-        const bool tall = tile_rows != 32 && (long long)((W + 63) / 64) * ((H + 63) / 64) >= kTallTiles;
+        const bool tall = tile_rows == 64 ||
+                          (tile_rows == 0 && (long long)((W + 63) / 64) * ((H + 63) / 64) >= kTallTiles);
         const int rc = for_tc_shape(r, [&](auto p, auto pv) {
             constexpr int P = decltype(p)::value, PV = decltype(pv)::value;
             if constexpr (P == 4) {  // only narrow kernels sum to 256
+                if (b.clamp && tile_rows == 64)
+                    return launch_blur_level_tc<TG, P, PV, 64, true>(in, in_pitch, out, out_u8, pitch, W, H, tp, st, ref);
                 if (b.clamp)
                     return launch_blur_level_tc<TG, P, PV, 32, true>(in, in_pitch, out, out_u8, pitch, W, H, tp, st, ref);
             }

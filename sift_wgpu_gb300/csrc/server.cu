@@ -256,9 +256,9 @@ struct Server {
         Engine::Tuning best = e.tune;
         float best_ms = 0.0f;
         int rc = time_cfg(best, &best_ms);
-        // candidate values per knob: fused radius limit, level tile rows,
-        // orientation CTAs/SM, descriptor CTAs/SM
-        const int vals[4][3] = {{8, 4, 0}, {64, 32, 0}, {2, 4, 8}, {4, 8, 16}};
+        // candidate values per knob: fused radius limit, level tile rows (0:
+        // by the plane's size), orientation CTAs/SM, descriptor CTAs/SM
+        const int vals[4][3] = {{8, 4, 0}, {0, 32, 0}, {2, 4, 8}, {4, 8, 16}};
         const int nvals[4] = {3, 2, 3, 3};
         for (int knob = 0; knob < 4 && !rc; ++knob) {
             for (int v = 0; v < nvals[knob] && !rc; ++v) {
@@ -700,7 +700,7 @@ int sift_cuda_server_tuning_knobs(SiftCudaServer* server, uint32_t width, uint32
     auto it = S.tuned.find(sift::TuneKey{width, height});
     sift::Engine::Tuning t{};
     if (it != S.tuned.end()) t = it->second;
-    const int32_t all[4] = {t.fused_max_radius, t.level_tile_rows, t.ori_ctas_per_sm, t.desc_ctas_per_sm};
+    const int32_t all[4] = {t.fused_max_radius, t.level_tile_rows == 32 ? 32 : 64, t.ori_ctas_per_sm, t.desc_ctas_per_sm};
     for (uint32_t i = 0; i < n_knobs && i < 4; ++i) knobs[i] = all[i];
     return it != S.tuned.end() ? 1 : 0;
 }

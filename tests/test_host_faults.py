@@ -354,3 +354,21 @@ def test_in_place_says_where_the_run_read_the_image(fake, shape, start, sigma, i
                                                         C.byref(r)) == 0
     assert fake.lib.sift_cuda_last_image_in_place(h) == 0
     fake.lib.sift_cuda_destroy(h)
+
+
+# ---- rows of the level kernel's tiles ----------------------------------------
+
+@pytest.mark.parametrize("rows,small,large", [(0, 32, 64), (32, 32, 32), (64, 64, 64)])
+@pytest.mark.parametrize("sigma,assumed", [(1.6, 0.5), (0.45, 0.3)])  # (the second's taps sum above 1)
+def test_tile_rows_by_option(fake, rows, small, large, sigma, assumed):
+    p = _capi.Params()
+    fake.lib.sift_cuda_params_new(C.byref(p), sigma, 1, 3, assumed, 0.04, 10.0)
+    h = fake.engine(p, level_tile_rows=rows)
+    for shape, want in (((100, 64), small), ((1100, 1600), large)):
+        fake.log()
+        assert fake.detect(h, aligned(shape))[0] == 0
+        # (kernels of taps that sum above 1 take 32-row tiles where nothing else is asked)
+        levels = [line.split() for line in fake.log() if "k_blur_level" in line]
+        grids = {line[2] for line in levels if not (want == 64 and rows == 0 and "Lb1E" in line[1])}
+        assert grids == {f"{-(-shape[1] // 64)}x{-(-shape[0] // want)}"}
+    fake.lib.sift_cuda_destroy(h)
