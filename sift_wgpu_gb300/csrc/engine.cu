@@ -513,6 +513,7 @@ int sift_cuda_debug_stage(SiftCudaEngine* engine, int stage, void* out, uint64_t
         src = e.d_oriented.as<sift::Keypoint>();
         n = std::min<uint64_t>(c.n_oriented, e.cap_ori);
     } else if (stage == SIFT_CUDA_STAGE_DESCRIPTORS) {
+        if (int rc = e.recover_descriptors()) return rc;
         const uint64_t nd = std::min<uint64_t>(c.n_oriented, e.cap_ori) * sift::kDescLen;
         *count = nd;
         if (out && nd) {

@@ -490,6 +490,8 @@ struct Engine {
     int ensure_geometry(uint32_t w, uint32_t h) {
         if (have_geom && w == W && h == H) return 0;
         have_geom = false;
+        desc_on_host = 0;  // (of the last run nothing is left)
+        last.reset();
         const int O = (int)p.num_octaves, S = (int)p.num_intervals;
         if (O > kMaxOctaves) return fail(SIFT_CUDA_ERR_UNSUPPORTED, "num_octaves above 16 is not supported");
         PyramidDev g{};
@@ -647,6 +649,37 @@ struct Engine {
         return 0;
     }
 
+    // The descriptors of octave o. Host calls (cell): those below the cell's
+    // capacity go straight into the mapped export buffer while the stage runs,
+    // the rest to d_desc.
+    int describe_octave(int o, const RunCell* rc, cudaStream_t q) {
+        // two keypoints per CTA for 1/8 of the candidate capacity; the last
+        // 152 x desc_ctas_per_sm CTAs drain whatever is left
+        const int grid = (int)std::max<uint32_t>(cap_c[o] / 16, 64);
+        if (launch_descriptor(d_U.as<uint8_t>(), tab(), d_oriented.as<Keypoint>(), &d_ctr.as<Counters>()->oct[o],
+                              d_desc.as<float>(), cap_ori, rc, grid, 152 * tune.desc_ctas_per_sm, q))
+            return cuda_fail(cudaGetLastError(), "descriptor");
+        return 0;
+    }
+
+    // The last run's descriptors in d_desc, for the read-back: made again by
+    // their stage where the buffer that the run wrote has been lent, whose
+    // holder may have changed it. (The stage gives the same bits every time.)
+    int recover_descriptors() {
+        if (!desc_on_host || last == hx) return 0;
+        if (int rc = set_device()) return rc;
+        Counters c;
+        CK(cudaMemcpy(&c, d_ctr.p, sizeof c, cudaMemcpyDeviceToHost), "D2H counters");
+        for (auto& oc : c.oct) oc.next_desc = 0;
+        CK(cudaMemcpyAsync(d_ctr.p, &c, sizeof c, cudaMemcpyHostToDevice, st), "H2D counters");
+        for (int o = 0; o < pyr.num_octaves && pyr.oct[o].W > 0 && pyr.oct[o].H > 0; ++o)
+            if (int rc = describe_octave(o, nullptr, st)) return rc;
+        CK(cudaStreamSynchronize(st), "descriptors");
+        desc_on_host = 0;
+        last.reset();
+        return 0;
+    }
+
     // The run as a DAG (dag) or in stage order on one stream (profiling):
     //   st        counters, base level, octave o levels 1..S, Lanczos(o) ->
     //             octave o+1 ...
@@ -751,15 +784,8 @@ struct Engine {
         };
         auto describe = [&](int o, cudaStream_t q) -> int {
             if (!with_desc) return 0;
-            // two keypoints per CTA for 1/8 of the candidate capacity; the
-            // last 152 x desc_ctas_per_sm CTAs drain whatever is left
-            const int grid = (int)std::max<uint32_t>(cap_c[o] / 16, 64);
-            // host calls: descriptors below cap_x go straight into the mapped
-            // export buffer while the stage runs, the rest to d_desc
-            if (ok(launch_descriptor(U, tab(), d_oriented.as<Keypoint>(), &ctr->oct[o], d_desc.as<float>(), cap_ori,
-                                         exp ? rc : nullptr, grid, 152 * tune.desc_ctas_per_sm, q)))
-                return cuda_fail(cudaGetLastError(), "descriptor");
-            return 0;
+            ++launches;
+            return describe_octave(o, exp ? rc : nullptr, q);
         };
 
         const OctaveDev& o0 = pyr.oct[0];

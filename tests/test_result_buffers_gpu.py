@@ -1,0 +1,29 @@
+"""Lent result buffers and what goes on around them: the read-back does not
+see what the caller writes into a result."""
+import pytest
+
+from synthetic import synth_image
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def sgb(built_lib):
+    import sift_wgpu_gb300 as sg
+    return sg
+
+
+@pytest.mark.parametrize("octaves", [1, 4])
+def test_read_back_of_a_result_that_the_caller_changed(sgb, octaves):
+    img = synth_image(901, 400, 300)
+    with sgb.Engine(sgb.Sift.new(1.6, octaves, 3, 0.5, 0.04, 10.0)) as e:
+        want = e.detect_and_compute_view(img)[1].copy()
+        for _ in range(120):
+            k, d = e.detect_and_compute(img)
+            d[:] = 7.0
+            k["x"] = -1.0
+        assert e.debug_stage(sgb.STAGE_DESCRIPTORS).tobytes() == want.tobytes()
+        assert e.debug_stage(sgb.STAGE_DESCRIPTORS).tobytes() == want.tobytes()
+        k, d = e.detect_and_compute(img)  # the run after it is its own
+        assert d.tobytes() == want.tobytes()
+        assert e.debug_stage(sgb.STAGE_KEYPOINTS).tobytes() == k.tobytes()
