@@ -156,8 +156,19 @@ struct LevelBlur {
     size_t foff;   // element offset of its fragments in the weight table
 };
 
+// While it lives, this thread may free memory although it, or another thread,
+// captures a stream in a mode that forbids that (the capture would be lost).
+struct AnyCapture {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    AnyCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    ~AnyCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    AnyCapture(const AnyCapture&) = delete;
+    AnyCapture& operator=(const AnyCapture&) = delete;
+};
+
 // A mapped pinned buffer that a run writes its results into: Counters |
-// keypoints[cap] | descriptors[cap].
+// keypoints[cap] | descriptors[cap]. A lent one is freed wherever the caller
+// frees the result (a garbage collector may), also while a stream is captured.
 struct ExportBuf {
     void* p = nullptr;
     size_t bytes = 0;
@@ -169,6 +180,7 @@ struct ExportBuf {
     ExportBuf(const ExportBuf&) = delete;
     ExportBuf& operator=(const ExportBuf&) = delete;
     ~ExportBuf() {
+        AnyCapture any;
         if (p) cudaFreeHost(p);
     }
     Counters* ctr() const { return (Counters*)p; }

@@ -230,6 +230,7 @@ cudaError_t cudaMemsetAsync(void* p, int v, size_t n, cudaStream_t) {
     return cudaSuccess;
 }
 
+cudaError_t cudaThreadExchangeStreamCaptureMode(cudaStreamCaptureMode*) { return cudaSuccess; }
 cudaError_t cudaStreamBeginCapture(cudaStream_t, cudaStreamCaptureMode) {
     Lock g(mu);
     if (cudaError_t e = call("cudaStreamBeginCapture")) return e;
