@@ -69,9 +69,9 @@ typedef struct {
  * (desc == NULL for keypoint-only detection). Free with
  * sift_cuda_result_free, from any
  * thread, also after the engine is destroyed. The arrays are the caller's
- * until then and may be written. They are the page-locked buffer that the run
- * wrote, lent while the engine has another for its next run (at most 4 of an
- * engine are out at a time), or else a copy of it. */
+ * until then and may be written. They are ordinary memory of the process: the
+ * buffer that the run wrote, lent while the engine has another for its next
+ * run (at most 4 of an engine are out at a time), or else a copy of it. */
 typedef struct {
     uint32_t n;
     SiftCudaKeypoint* kps;

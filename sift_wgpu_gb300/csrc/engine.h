@@ -20,6 +20,7 @@
 #pragma once
 
 #include <cuda_runtime.h>
+#include <sys/mman.h>
 
 #include <algorithm>
 #include <cstdio>
@@ -156,23 +157,20 @@ struct LevelBlur {
     size_t foff;   // element offset of its fragments in the weight table
 };
 
-// While it lives, this thread may free memory although it, or another thread,
-// captures a stream in a mode that forbids that (the capture would be lost).
-struct AnyCapture {
-    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
-    AnyCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
-    ~AnyCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
-    AnyCapture(const AnyCapture&) = delete;
-    AnyCapture& operator=(const AnyCapture&) = delete;
-};
-
-// A mapped pinned buffer that a run writes its results into: Counters |
-// keypoints[cap] | descriptors[cap]. A lent one is freed wherever the caller
-// frees the result (a garbage collector may), also while a stream is captured.
+// A host buffer that a run writes its results into: Counters |
+// keypoints[cap] | descriptors[cap]. Mapped and pinned, or plain: ordinary
+// memory of the process, which a device that uses the host's page tables
+// writes at the same speed (1080p calls 329 us with either, 4096 x 4096 2058).
+// Owned results are lent in plain buffers only. To CUDA those are pageable
+// memory, so that a copy to a device that the caller has enqueued holds the
+// values once the call for it returns (from pinned memory it would read them
+// later, when a next run may have the buffer), and a forked child has its own
+// (pinned memory is shared with it).
 struct ExportBuf {
     void* p = nullptr;
     size_t bytes = 0;
     uint32_t cap = 0;
+    bool plain = false;
     Counters* dctr = nullptr;  // device addresses of the three parts
     Keypoint* dkps = nullptr;
     float* ddesc = nullptr;
@@ -180,16 +178,29 @@ struct ExportBuf {
     ExportBuf(const ExportBuf&) = delete;
     ExportBuf& operator=(const ExportBuf&) = delete;
     ~ExportBuf() {
-        AnyCapture any;
-        if (p) cudaFreeHost(p);
+        if (p && plain) munmap(p, bytes);
+        else if (p) cudaFreeHost(p);
     }
     Counters* ctr() const { return (Counters*)p; }
     Keypoint* kps() const { return (Keypoint*)((char*)p + align_up(sizeof(Counters), 256)); }
     float* desc() const { return (float*)((char*)kps() + align_up((size_t)cap * sizeof(Keypoint), 256)); }
-    cudaError_t alloc(uint32_t n) {
+    cudaError_t alloc(uint32_t n, bool plain_memory) {
         cap = n;
+        plain = plain_memory;
         bytes = align_up(sizeof(Counters), 256) + align_up((size_t)n * sizeof(Keypoint), 256) +
                 (size_t)n * kDescLen * sizeof(float);
+        if (plain) {
+            // (with its pages: the device would fault on each)
+            p = mmap(nullptr, bytes, PROT_READ | PROT_WRITE, MAP_PRIVATE | MAP_ANONYMOUS | MAP_POPULATE, -1, 0);
+            if (p == MAP_FAILED) {
+                p = nullptr;
+                return cudaErrorMemoryAllocation;
+            }
+            dctr = ctr();
+            dkps = kps();
+            ddesc = desc();
+            return cudaSuccess;
+        }
         if (cudaError_t e = cudaHostAlloc(&p, bytes, cudaHostAllocMapped)) {
             p = nullptr;
             return e;
@@ -203,7 +214,8 @@ struct ExportBuf {
 // Result buffers that an engine lends to its callers: a result of
 // sift_cuda_detect_and_compute is the buffer the run wrote, given back by
 // sift_cuda_result_free (from any thread, also after the engine is gone).
-// At most kLent are out at a time; further results are copies. Without it
+// At most kLent are out at a time; further results are copies, as all are on a
+// device that does not use the host's page tables. Without it
 // half of a 4096 x 4096 call was the copy into freshly allocated pages
 // (4894 us, of which 2300), a third of a 1080p call.
 struct ExportPool {
@@ -298,7 +310,9 @@ struct Engine {
     // Host calls: the run ends with an export kernel that writes counters and
     // keypoints into this buffer (the descriptor stage its descriptors),
     // sized from the last count. An owned result lends it to the caller.
-    std::shared_ptr<ExportBuf> hx, last;  // of the next run; of the last host call
+    std::shared_ptr<ExportBuf> plain, pinned;  // for owned results; for views and the server
+    std::shared_ptr<ExportBuf> hx, last;       // of the next run (one of them); of the last host call
+    bool last_lent = false;                    // the caller has it
     std::shared_ptr<ExportPool> pool = std::make_shared<ExportPool>();
     size_t copied = 0;  // result bytes copied since the last spare buffer was made
     uint32_t last_n = 0;
@@ -314,6 +328,7 @@ struct Engine {
     DevMem d_cell;
     bool unsynced = false;  // a run that may still read the mapped copy has not been waited for
     int pageable_reads = -1;  // device attribute, read once
+    bool host_tables = false;  // the device uses the host's page tables (init)
     bool image_in_place = false;
     uint32_t launches = 0;
     bool last_desc = true;
@@ -369,6 +384,7 @@ struct Engine {
     std::vector<std::vector<cudaEvent_t>> ev_runs;  // kStages + 1 events per run
 
     ~Engine() {
+        if (st) cudaStreamSynchronize(st);  // (freeing plain result buffers does not wait)
         drop_graph();
         std::vector<std::shared_ptr<ExportBuf>> spare;
         {
@@ -453,6 +469,10 @@ struct Engine {
 
     int init() {
         if (int rc = set_device()) return rc;
+        int tables = 0;
+        if (cudaDeviceGetAttribute(&tables, cudaDevAttrPageableMemoryAccessUsesHostPageTables, opt.device) != cudaSuccess)
+            tables = 0;
+        host_tables = tables == 1;
         // Octave 0's stream runs at the engine's priority, the pyramid's main
         // stream and the smaller octaves' streams one step more urgent: while
         // octave 0's orientation and descriptors fill the device, the other
@@ -678,7 +698,7 @@ struct Engine {
     // their stage where the buffer that the run wrote has been lent, whose
     // holder may have changed it. (The stage gives the same bits every time.)
     int recover_descriptors() {
-        if (!desc_on_host || last == hx) return 0;
+        if (!desc_on_host || !last_lent) return 0;
         if (int rc = set_device()) return rc;
         Counters c;
         CK(cudaMemcpy(&c, d_ctr.p, sizeof c, cudaMemcpyDeviceToHost), "D2H counters");
@@ -903,18 +923,22 @@ struct Engine {
         return nullptr;
     }
 
-    // Result buffer for at least n keypoints (host calls). It grows with half
-    // as much headroom so that images of one size with more keypoints than
-    // the last seldom force another allocation.
-    int ensure_export(uint32_t n) {
-        if (hx && n <= hx->cap) return 0;
-        if (auto b = take_idle(n)) {
-            hx = std::move(b);
-            return 0;
+    // Result buffer for at least n keypoints (host calls), a plain one for
+    // owned results where the device can write it. It grows with half as much
+    // headroom so that images of one size with more keypoints than the last
+    // seldom force another allocation.
+    int ensure_export(uint32_t n, bool owned = false) {
+        const bool use_plain = owned && host_tables;
+        std::shared_ptr<ExportBuf>& mine = use_plain ? plain : pinned;
+        if (!mine || n > mine->cap) {
+            std::shared_ptr<ExportBuf> b = use_plain ? take_idle(n) : nullptr;
+            if (!b) {
+                b = std::make_shared<ExportBuf>();
+                CK(b->alloc(n + n / 2 + 4096, use_plain), "result buffer");
+            }
+            mine = std::move(b);
         }
-        auto b = std::make_shared<ExportBuf>();
-        CK(b->alloc(n + n / 2 + 4096), "cudaHostAlloc(export)");
-        hx = std::move(b);
+        hx = mine;
         return 0;
     }
 
@@ -928,7 +952,7 @@ struct Engine {
         if (n > hx->cap) {
             const std::shared_ptr<ExportBuf> old = hx;
             const uint32_t head = old->cap;
-            if (int rc = ensure_export(n)) return rc;
+            if (int rc = ensure_export(n, old->plain)) return rc;
             *hx->ctr() = c;
             CK(cudaMemcpy(hx->kps(), d_oriented.p, sizeof(Keypoint) * n, cudaMemcpyDeviceToHost), "D2H kps");
             if (with_desc) {
@@ -939,6 +963,7 @@ struct Engine {
             }
         }
         last = hx;
+        last_lent = false;
         last_n = n;
         desc_on_host = with_desc ? n : 0;
         return 0;
@@ -1107,7 +1132,7 @@ struct Engine {
                     return cuda_fail(cudaGetLastError(), "luma conversion");
             }
         }
-        if (int rc = ensure_export(last_n ? last_n : 4096)) return rc;
+        if (int rc = ensure_export(last_n ? last_n : 4096, !view)) return rc;
         for (int attempt = 0; attempt < 8; ++attempt) {
             if (int rc = run(with_desc, true)) return rc;
             CK(cudaStreamSynchronize(st), "run");
@@ -1123,8 +1148,8 @@ struct Engine {
         return fail(SIFT_CUDA_ERR_CAPACITY, "keypoint lists kept overflowing");
     }
 
-    // Results of a host call, already in the mapped export buffer; out points
-    // at them (valid until the next call).
+    // Results of a host call, already in the pinned buffer; out points at
+    // them (valid until the next call).
     int fetch_view(bool with_desc, SiftCudaResult* out) {
         out->n = h_ctr.as<Counters>()->n_oriented;
         out->kps = (SiftCudaKeypoint*)hx->kps();
@@ -1135,9 +1160,10 @@ struct Engine {
     // Lends the result buffer to the caller if there is another one for the
     // next run. One is made once the copies since the last have moved its
     // bytes, about the time its allocation takes (two copies of a 1080p
-    // result 0.6 ms, a 14 MB buffer 0.6 ms): an engine called once or twice
+    // result 0.8 ms, a 12 MB buffer 0.5 ms): an engine called once or twice
     // never pays for it.
     bool lend(uint32_t n, bool with_desc, SiftCudaResult* out) {
+        if (!hx->plain) return false;
         {
             std::lock_guard<std::mutex> g(pool->mu);
             if (pool->lent >= ExportPool::kLent) return false;
@@ -1146,15 +1172,13 @@ struct Engine {
         if (!next && copied >= hx->bytes) {
             copied = 0;
             next = std::make_shared<ExportBuf>();
-            if (next->alloc(hx->cap) != cudaSuccess) {
-                cudaGetLastError();
-                return false;
-            }
+            if (next->alloc(hx->cap, true) != cudaSuccess) return false;
         }
         if (!next || !lend_result(hx, pool)) return false;
         out->kps = (SiftCudaKeypoint*)hx->kps();
         out->desc = with_desc ? hx->desc() : nullptr;
-        hx = std::move(next);
+        hx = plain = std::move(next);
+        last_lent = true;
         return true;
     }
 

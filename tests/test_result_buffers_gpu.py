@@ -2,6 +2,9 @@
 see what the caller writes into a result, and a result may be freed while a
 stream is captured."""
 import gc
+import os
+import select
+import signal
 
 import numpy as np
 import pytest
@@ -69,3 +72,67 @@ def test_results_freed_during_a_capture(warmed, closed):
     if closed:
         e.close()
     captured(held.clear)
+
+
+# ---- a result is ordinary memory ---------------------------------------------
+
+def lending(sgb, img):
+    """An engine with results to lend, and one that is lent."""
+    e = sgb.Engine()
+    for _ in range(80):
+        e.detect_and_compute(img)
+    return e, e.detect_and_compute(img)
+
+
+@pytest.fixture(scope="module")
+def two(sgb):
+    imgs = [synth_image(910 + i, 400, 300) for i in range(2)]
+    with sgb.Engine() as e:
+        return imgs, [tuple(a.copy() for a in e.detect_and_compute_view(im)) for im in imgs]
+
+
+def test_a_copy_to_the_device_outlives_the_result(sgb, two):
+    """An enqueued copy of a result whose stream is busy (for some 25 ms) while the result goes and others come."""
+    import torch
+    imgs, want = two
+    e, (k, d) = lending(sgb, imgs[0])
+    stream = torch.cuda.Stream()
+    with torch.cuda.stream(stream):
+        torch.cuda._sleep(50_000_000)
+        on_device = torch.from_numpy(d).to("cuda", non_blocking=True)
+    del k, d
+    for _ in range(8):
+        e.detect_and_compute(imgs[1])
+    torch.cuda.synchronize()
+    e.close()
+    assert on_device.cpu().numpy().tobytes() == want[0][1].tobytes()
+
+
+@pytest.mark.filterwarnings("ignore:This process .* is multi-threaded:DeprecationWarning")
+def test_a_forked_child_keeps_its_results(sgb, two):
+    """A child that looks at a result, and writes to it, after the parent has dropped it and gone on."""
+    imgs, want = two
+    e, r = lending(sgb, imgs[0])
+    go, answer = os.pipe(), os.pipe()
+    pid = os.fork()
+    if pid == 0:
+        os.read(go[0], 1)
+        ok = r[0].tobytes() == want[0][0].tobytes() and r[1].tobytes() == want[0][1].tobytes()
+        r[1][:] = 7.0
+        os.write(answer[1], b"1" if ok else b"0")
+        os._exit(0)
+    held = e.detect_and_compute(imgs[1])
+    del r
+    for _ in range(8):
+        k, d = e.detect_and_compute(imgs[1])
+        assert k.tobytes() == want[1][0].tobytes() and d.tobytes() == want[1][1].tobytes()
+    os.write(go[1], b"x")
+    answered = select.select([answer[0]], [], [], 60)[0]
+    if not answered:
+        os.kill(pid, signal.SIGKILL)
+    os.waitpid(pid, 0)
+    assert answered and os.read(answer[0], 1) == b"1"
+    for fd in go + answer:
+        os.close(fd)
+    assert held[1].tobytes() == want[1][1].tobytes() and d.tobytes() == want[1][1].tobytes()
+    e.close()
