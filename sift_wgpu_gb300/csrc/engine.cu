@@ -1,5 +1,7 @@
 // engine.cu — error state, lent result buffers and the C ABI of the per-image
 // engine (engine.h).
+#include <pthread.h>
+
 #include <unordered_map>
 
 #include "engine.h"
@@ -37,41 +39,40 @@ struct Lent {
     std::shared_ptr<ExportBuf> buf;
     std::shared_ptr<ExportPool> pool;
 };
-struct LentTable {
-    std::mutex mu;
-    std::unordered_map<const void*, Lent> by_kps;
-};
-LentTable& lent_table() {
-    static LentTable* t = new LentTable;
+std::unordered_map<const void*, Lent>& lent_by_kps() {
+    static auto* t = new std::unordered_map<const void*, Lent>;
     return *t;
 }
 }  // namespace
 
+std::mutex& lend_mutex() {
+    static std::mutex* mu = [] {
+        pthread_atfork([] { lend_mutex().lock(); }, [] { lend_mutex().unlock(); }, [] { lend_mutex().unlock(); });
+        return new std::mutex;
+    }();
+    return *mu;
+}
+
 bool lend_result(const std::shared_ptr<ExportBuf>& buf, const std::shared_ptr<ExportPool>& pool) {
+    std::lock_guard<std::mutex> g(lend_mutex());
     try {
-        LentTable& t = lent_table();
-        std::lock_guard<std::mutex> g(t.mu);
-        t.by_kps.emplace(buf->kps(), Lent{buf, pool});
+        lent_by_kps().emplace(buf->kps(), Lent{buf, pool});
     } catch (const std::bad_alloc&) {
         return false;
     }
-    std::lock_guard<std::mutex> g(pool->mu);
     ++pool->lent;
     return true;
 }
 
 // Takes a lent buffer back; false if kps is not one's.
 static bool return_result(const void* kps) {
-    Lent l;
-    {
-        LentTable& t = lent_table();
-        std::lock_guard<std::mutex> g(t.mu);
-        auto it = t.by_kps.find(kps);
-        if (it == t.by_kps.end()) return false;
-        l = std::move(it->second);
-        t.by_kps.erase(it);
-    }
-    std::lock_guard<std::mutex> g(l.pool->mu);
+    Lent l;  // (freed after the lock)
+    std::lock_guard<std::mutex> g(lend_mutex());
+    auto& t = lent_by_kps();
+    auto it = t.find(kps);
+    if (it == t.end()) return false;
+    l = std::move(it->second);
+    t.erase(it);
     --l.pool->lent;
     if (!l.pool->closed && l.pool->idle.size() < ExportPool::kIdle) l.pool->idle.push_back(l.buf);
     return true;

@@ -220,12 +220,14 @@ struct ExportBuf {
 // (4894 us, of which 2300), a third of a 1080p call.
 struct ExportPool {
     static constexpr uint32_t kLent = 4, kIdle = 3;
-    std::mutex mu;
     std::vector<std::shared_ptr<ExportBuf>> idle;
     uint32_t lent = 0;
     bool closed = false;
     ExportPool() { idle.reserve(kIdle); }  // giving back never allocates
 };
+// Guards every pool and the table of lent buffers. A fork waits for it, so that
+// the child, where results are freed too, does not find it taken.
+std::mutex& lend_mutex();
 // Registers buf as lent (engine.cu); false, and nothing lent, if the host is out of memory.
 bool lend_result(const std::shared_ptr<ExportBuf>& buf, const std::shared_ptr<ExportPool>& pool);
 
@@ -388,7 +390,7 @@ struct Engine {
         drop_graph();
         std::vector<std::shared_ptr<ExportBuf>> spare;
         {
-            std::lock_guard<std::mutex> g(pool->mu);
+            std::lock_guard<std::mutex> g(lend_mutex());
             pool->closed = true;
             spare.swap(pool->idle);
         }
@@ -913,7 +915,7 @@ struct Engine {
     // The pool's buffer for at least n keypoints, if it has one; smaller ones go.
     std::shared_ptr<ExportBuf> take_idle(uint32_t n) {
         std::vector<std::shared_ptr<ExportBuf>> small;  // freed after the lock
-        std::lock_guard<std::mutex> g(pool->mu);
+        std::lock_guard<std::mutex> g(lend_mutex());
         while (!pool->idle.empty()) {
             std::shared_ptr<ExportBuf> b = std::move(pool->idle.back());
             pool->idle.pop_back();
@@ -1165,7 +1167,7 @@ struct Engine {
     bool lend(uint32_t n, bool with_desc, SiftCudaResult* out) {
         if (!hx->plain) return false;
         {
-            std::lock_guard<std::mutex> g(pool->mu);
+            std::lock_guard<std::mutex> g(lend_mutex());
             if (pool->lent >= ExportPool::kLent) return false;
         }
         std::shared_ptr<ExportBuf> next = take_idle(n);

@@ -7,11 +7,13 @@
 #include <cuda.h>
 #include <cuda_runtime_api.h>
 
+#include <atomic>
 #include <cstdlib>
 #include <cstring>
 #include <map>
 #include <mutex>
 #include <string>
+#include <thread>
 #include <vector>
 
 namespace {
@@ -22,6 +24,7 @@ std::map<void*, size_t> device, pinned;
 std::map<std::string, std::pair<int, int>> failures;  // call: how many from now, the error
 std::vector<std::pair<uint32_t, uint32_t>> counters;  // words of a run's counters
 bool capturing = false;
+int host_tables = 0;  // whether the device uses the host's page tables
 thread_local cudaError_t last = cudaSuccess;
 
 struct Launch {
@@ -125,6 +128,23 @@ size_t fake_log(char* out, size_t cap) {
     std::memcpy(out, s.data(), n);
     out[n] = 0;
     return s.size();
+}
+void fake_host_tables(int on) { host_tables = on; }
+// threads that free results of their own (malloc'd ones) until told to stop
+void fake_free_results(void (*free_result)(void*), int threads) {
+    static std::atomic<bool> stop;
+    static std::vector<std::thread> running;
+    stop = true;
+    for (auto& t : running) t.join();
+    running.clear();
+    stop = false;
+    for (int i = 0; i < threads; ++i)
+        running.emplace_back([free_result] {
+            while (!stop) {
+                struct { uint32_t n; void *kps, *desc; } r{1, std::malloc(64), nullptr};
+                free_result(&r);
+            }
+        });
 }
 int fake_live_device() {
     Lock g(mu);
@@ -297,7 +317,9 @@ cudaError_t cudaGetDeviceCount(int* n) {
     return cudaSuccess;
 }
 cudaError_t cudaDeviceGetAttribute(int* v, cudaDeviceAttr a, int) {
-    *v = a == cudaDevAttrPageableMemoryAccess ? 1 : 0;
+    *v = a == cudaDevAttrPageableMemoryAccess                    ? 1
+         : a == cudaDevAttrPageableMemoryAccessUsesHostPageTables ? host_tables
+                                                                  : 0;
     return cudaSuccess;
 }
 cudaError_t cudaDeviceGetStreamPriorityRange(int* least, int* greatest) {

@@ -2,8 +2,11 @@
 library's objects are linked against a fake CUDA runtime (fake_cuda.cpp) that
 logs the calls and makes a chosen one return an error."""
 import ctypes as C
+import os
 import shutil
+import signal
 import subprocess
+import time
 
 import numpy as np
 import pytest
@@ -372,3 +375,53 @@ def test_tile_rows_by_option(fake, rows, small, large, sigma, assumed):
         grids = {line[2] for line in levels if not (want == 64 and rows == 0 and "Lb1E" in line[1])}
         assert grids == {f"{-(-shape[1] // 64)}x{-(-shape[0] // want)}"}
     fake.lib.sift_cuda_destroy(h)
+
+
+# ---- lent results in a forked child ------------------------------------------
+
+N_ORIENTED = 2  # the word of the keypoint count
+
+
+@pytest.fixture
+def lent(fake):
+    """A lent result, on a device that writes plain memory."""
+    fake.lib.fake_host_tables(1)
+    h, img = fake.engine(), aligned(SMALL)
+    fake.lib.fake_counter(N_ORIENTED, 1000)
+    for _ in range(10):
+        rc, r = fake.detect(h, img)
+        assert rc == 0 and r.n == 1000
+        fake.lib.sift_cuda_result_free(C.byref(r))
+    fake.log()
+    rc, r = fake.detect(h, img)
+    yield r
+    fake.lib.sift_cuda_result_free(C.byref(r))
+    fake.lib.sift_cuda_destroy(h)
+    fake.lib.fake_host_tables(0)
+
+
+def ended(pid, seconds):
+    end = time.time() + seconds
+    while time.time() < end:
+        if os.waitpid(pid, os.WNOHANG)[0]:
+            return True
+        time.sleep(0.0005)
+    os.kill(pid, signal.SIGKILL)
+    os.waitpid(pid, 0)
+    return False
+
+
+@pytest.mark.filterwarnings("ignore:This process .* is multi-threaded:DeprecationWarning")
+def test_a_forked_child_frees_a_lent_result(fake, lent):
+    """Forks while other threads free results: the child's own free comes back."""
+    free = C.cast(fake.lib.sift_cuda_result_free, C.c_void_p)
+    fake.lib.fake_free_results(free, 4)
+    try:
+        for _ in range(500):
+            pid = os.fork()
+            if pid == 0:
+                fake.lib.sift_cuda_result_free(C.byref(lent))
+                os._exit(0)
+            assert ended(pid, 20)
+    finally:
+        fake.lib.fake_free_results(free, 0)
