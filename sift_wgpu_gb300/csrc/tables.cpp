@@ -113,12 +113,13 @@ TcBlur tc_blur(const std::vector<float>& w) {
         if (shift < 4) return t;
         long long sb = 0;
         double up = 0.0, down = 0.0;
+        const double scale = std::ldexp(1.0, qa + shift), unit = std::ldexp(1.0, -(qa + shift));
         for (int i = 0; i < n; ++i) {
-            const long long W = std::llrint(std::ldexp((double)w[i], qa + shift));
+            const long long W = std::llrint((double)w[i] * scale);
             a[i] = (W + (1ll << (shift - 1))) >> shift;
             b[i] = W - a[i] * (1ll << shift);
             sb += b[i] < 0 ? -b[i] : b[i];
-            const double d = (double)w[i] - std::ldexp((double)W, -(qa + shift));
+            const double d = (double)w[i] - (double)W * unit;
             (d > 0 ? up : down) += std::fabs(d);
         }
         quant = 255.0 * std::max(up, down);
@@ -156,21 +157,29 @@ TcBlur tc_blur(const std::vector<float>& w) {
     const int P = r <= 4 ? 4 : (r + 3) / 8 * 8 + 4, PV = (r + 7) / 8 * 8;
     t.kh = (8 + 2 * P) / 16;
     t.kv = (16 + 2 * PV) / 16;
-    auto pair = [&](const std::vector<long long>& v, int i) -> uint32_t {  // taps i, i + 1
-        auto at = [&](int j) { return j >= 0 && j < n ? half_of_int((int)v[(size_t)j]) : 0u; };
-        return at(i) | at(i + 1) << 16;
+    // (each limb's halves once: a layout for a new image size makes some 18 000
+    // fragment words, 420 us of conversions tap by tap, 70 us so)
+    std::vector<uint32_t> ha(n), hb(n);
+    for (int i = 0; i < n; ++i) {
+        ha[i] = half_of_int((int)a[i]);
+        hb[i] = half_of_int((int)b[i]);
+    }
+    t.frags.resize((size_t)(t.kh * 4 + t.kv * 8) * 32);
+    uint32_t* f = t.frags.data();
+    auto pair = [n](const std::vector<uint32_t>& h, int i) -> uint32_t {  // taps i, i + 1
+        return ((unsigned)i < (unsigned)n ? h[i] : 0u) | ((unsigned)(i + 1) < (unsigned)n ? h[i + 1] << 16 : 0u);
     };
     for (int ks = 0; ks < t.kh; ++ks)
         for (int lane = 0; lane < 32; ++lane) {
             const int g = lane >> 2, k = 16 * ks + 2 * (lane & 3), i = k - g - (P - r);  // column n = g
-            for (const auto* v : {&a, &b})
-                for (int d : {0, 8}) t.frags.push_back(pair(*v, i + d));
+            for (const auto* h : {&ha, &hb})
+                for (int d : {0, 8}) *f++ = pair(*h, i + d);
         }
     for (int ks = 0; ks < t.kv; ++ks)
         for (int lane = 0; lane < 32; ++lane) {
             const int g = lane >> 2, k = 16 * ks + 2 * (lane & 3), i = k - g - (PV - r);  // row m = g, g + 8
-            for (const auto* v : {&a, &b})
-                for (int d : {0, -8, 8, 0}) t.frags.push_back(pair(*v, i + d));
+            for (const auto* h : {&ha, &hb})
+                for (int d : {0, -8, 8, 0}) *f++ = pair(*h, i + d);
         }
     t.ok = true;
     return t;
