@@ -486,6 +486,7 @@ struct BatchEngine {
             cudaGraph_t g = nullptr;
             cudaError_t e = cudaStreamEndCapture(st, &g);
             if (rc) {
+                cudaGetLastError();  // the capture's own error, after the one that rc reports
                 if (g) cudaGraphDestroy(g);
                 return rc;
             }

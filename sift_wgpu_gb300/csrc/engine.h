@@ -1000,6 +1000,7 @@ struct Engine {
             cudaGraph_t g = nullptr;
             cudaError_t e = cudaStreamEndCapture(st, &g);
             if (rc) {
+                cudaGetLastError();  // the capture's own error, after the one that rc reports
                 if (g) cudaGraphDestroy(g);
                 return rc;
             }

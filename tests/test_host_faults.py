@@ -127,6 +127,28 @@ def test_the_error_of_a_failed_call_is_not_the_next_ones(fake, api):
     fake.lib.sift_cuda_destroy(fake.engine())
 
 
+@pytest.mark.parametrize("form", ["engine", "batch"])
+def test_a_launch_that_fails_in_a_capture(fake, form):
+    """The capture's end fails too (its other streams have not come back to it), and nobody reports that."""
+    img = aligned(SMALL)
+
+    def attempt(nth):
+        fake.lib.fake_reset()
+        h = fake.engine() if form == "engine" else fake.batch()
+        run = (lambda: fake.detect(h, img)[0]) if form == "engine" else (lambda: fake.detect_batch(h, img))
+        fake.fail("launch", nth)
+        fake.fail("cudaStreamEndCapture")
+        failed = run() != 0 and "failed launch" in fake.log()
+        assert not failed or run() == 0
+        close = fake.lib.sift_cuda_destroy if form == "engine" else fake.lib.sift_cuda_batch_destroy
+        close(h)
+        if failed:
+            fake.lib.sift_cuda_destroy(fake.engine())
+        return failed
+
+    assert failures("launch", attempt) >= 20
+
+
 READS_CALLER = ("k_fetch", "k_to_luma", "k_sq_norms", "cudaGraphLaunch")
 
 
