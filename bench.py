@@ -706,15 +706,15 @@ def run_cuda(args, world, rank, local):
             "ms_per_step": statistics.mean(step_ms), "higher_is_better": True, "scaling": "weak",
             "vs_baseline": None, "dtype": "f32", "data": "synthetic",
             "config": {"workload": f"{w}x{h} u8 synthetic frame, seed {seed}, Sift::new{sargs}",
-                       "storage": args.storage, "level_tile_rows": args.level_tile_rows or 64,
+                       "storage": args.storage, "level_tile_rows": args.level_tile_rows or "by plane size",
                        "parallelism": f"replicas x{world}",
                        "l2": "256 MiB flush before every step", "keypoints": int(nk)},
             "e2e": {"value": e2e_value, "unit": "images/s", "h2d_bytes_per_step": w * h, "d2h_bytes_per_step": d2h,
                     "form": "sift_cuda_detect_and_compute_view, pinned host image, results read in place"},
             "e2e_dropin": {"value": dropin_value, "unit": "images/s", "h2d_bytes_per_step": w * h,
                            "d2h_bytes_per_step": d2h,
-                           "form": "pageable host image through sift_cuda_detect_and_compute: the library copies "
-                                   "keypoints and descriptors into arrays the caller owns (and frees)"},
+                           "form": "pageable host image through sift_cuda_detect_and_compute: keypoints and "
+                                   "descriptors in arrays the caller owns (and frees), lent by the library"},
             "keypoints_per_s": {"device": value * int(nk), "e2e": e2e_value * int(nk)},
             "roofline": roof,
             "roofline_pyramid_dog": roof_pyr,

@@ -81,10 +81,10 @@ typedef struct {
 /* Pyramid storage of the Gaussian levels in device memory. Levels of the
  * reference-compatible pyramid hold u8 integers, so every mode is exact.
  * Each level has a u8 plane, from which the detection forms DoG in f32 where
- * it reads it (no DoG plane is stored). U8 stores nothing else: orientation
- * and descriptors read v / 255 from the u8 planes through the IEEE quotient
- * table. F32 and F16 also store every level in that type (4 and 2 more bytes
- * per pixel), which orientation and descriptors then read. U8 is the default
+ * it reads it (no DoG plane is stored); orientation and descriptors read the
+ * u8 planes too, in every mode. U8 stores nothing else. F32 and F16 also store
+ * every level in that type (4 and 2 more bytes per pixel), which no stage
+ * reads but a level that copies the previous one. U8 is the default
  * (sift_cuda_options_default): the smallest footprint and, measured on a
  * GB300, the fastest of the three; all three give the same output. */
 typedef enum {

@@ -6,10 +6,11 @@
 // Squared distances are |q|^2 + |t|^2 - 2 q.t. The products q.t run on the
 // 5th-generation tensor cores (tcgen05, TF32 operands, f32 accumulators in
 // tensor memory) over TMA-staged 128-descriptor tiles; they only select
-// candidates: the 4 best per query and half of a CTA's train tiles. A second
-// kernel keeps those that TF32's error lets be among the best two and ranks
-// them by exact f32 dot products. Ties go to the lower train index, so the
-// result does not depend on how the tiles are split over the CTAs.
+// candidates: the 4 best per query and quarter of the columns of a CTA's
+// train tiles. A second kernel keeps those that TF32's error lets be among the
+// best two and ranks them by exact f32 dot products. Ties go to the lower
+// train index, so the result does not depend on how the tiles are split over
+// the CTAs.
 #include <cuda.h>
 
 #include <algorithm>
@@ -125,8 +126,8 @@ constexpr float kTf32Err = 0.0045f;
 // instruction, 16 per tile) into one of two 128-column f32 accumulators in
 // tensor memory, so the epilogue of one tile overlaps the products of the
 // next. The epilogue warps own the accumulator's lanes: a thread reads one
-// query row's products of half the tile with tcgen05.ld and keeps the row's 4
-// best columns of the segment by |t|^2 - 2 q.t.
+// query row's products of a quarter of the tile with tcgen05.ld and keeps the
+// row's 4 best columns of these quarters of the segment by |t|^2 - 2 q.t.
 //
 // The epilogue bounds the kernel. A compare and a branch per column made a
 // serial chain of 64 branches per tile in which some lane of a warp almost

@@ -12,9 +12,8 @@
 // Every level is written as its u8 plane (1 byte/pixel, what the next level,
 // the resize and every later stage read; DoG is formed from it where it is
 // read, never stored) and, in the f32 and f16 storage modes, also in that
-// type (f32 v/255 or f16 v, read by orientation and descriptors); the default
-// u8 storage writes the u8 plane alone. Nothing in the chain re-reads a
-// 4-byte plane.
+// type (f32 v/255 or f16 v, which only a copied level reads again); the
+// default u8 storage writes the u8 plane alone.
 //
 // Kernels
 //   k_blur_level   both separable passes of a level for r <= 28 on the tensor

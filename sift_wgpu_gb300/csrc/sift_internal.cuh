@@ -166,7 +166,7 @@ __device__ __forceinline__ float div255(float v) {
     return __fmaf_rn(__fmaf_rn(-q, 255.0f, v), kInv255, q);
 }
 
-// v / 3 correctly rounded, by the same scheme (fl(1/3) is the correctly
+// v / 3 correctly rounded, by the same scheme of Markstein's (fl(1/3) is the correctly
 // rounded reciprocal), for v of 0 or far from the ends of the exponent range.
 __device__ __forceinline__ float div3(float v) {
     constexpr float third = 0.3333333432674408f;  // fl(1/3)

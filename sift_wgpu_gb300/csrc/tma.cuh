@@ -1,7 +1,6 @@
-// tma.cuh — mbarrier and TMA (cp.async.bulk.tensor) helpers of the sm_103a
-// kernels (descriptor matching, the prefetching level blur), and the host's
-// tensor-map encoder (cuTensorMapEncodeTiled from the driver the runtime
-// already loaded).
+// tma.cuh — mbarrier and TMA (cp.async.bulk.tensor) helpers of descriptor
+// matching, and the host's tensor-map encoder (cuTensorMapEncodeTiled from the
+// driver the runtime already loaded).
 #pragma once
 #include <cuda.h>
 #include <cuda_runtime.h>
