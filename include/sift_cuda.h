@@ -131,8 +131,8 @@ void sift_cuda_destroy(SiftCudaEngine* engine);
 /* Sift::detect_and_compute_with_backend(img, SiftBackend::Cuda)
  * (src/sift.rs:1244-1355) for an 8-bit grayscale host image: same keypoints,
  * order and 128-float descriptors as detect_and_compute_cpu
- * (src/sift.rs:1200-1240). The image is copied to the device inside the call;
- * results are copied back into library-owned host arrays. */
+ * (src/sift.rs:1200-1240). The image is read inside the call; the results are
+ * host arrays of the library's that the caller frees (SiftCudaResult). */
 int sift_cuda_detect_and_compute(SiftCudaEngine* engine, const uint8_t* img, uint32_t width,
                                  uint32_t height, uint32_t stride, SiftCudaResult* out);
 

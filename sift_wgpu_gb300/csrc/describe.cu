@@ -950,7 +950,7 @@ __global__ void __launch_bounds__(kDescThreads, 8) k_descriptor(const uint8_t* _
     // claims the next item while the CTA works on the current one (slot
     // next[p ^ 1]), unless the CTA retires after the current one.
     __shared__ uint32_t next[2];
-    // a host call's mapped result buffer, by the run's cell
+    // a host call's result buffer, by the run's cell
     __shared__ float* hdesc;
     __shared__ uint32_t hcap;
     const bool persist = (int)blockIdx.x >= persist_from;
@@ -971,7 +971,7 @@ __global__ void __launch_bounds__(kDescThreads, 8) k_descriptor(const uint8_t* _
         // tail of the stage
         const uint32_t i = base + (n - 1 - cur);
         const Keypoint kp = oriented[i];
-        // keypoints below hcap straight into the host call's mapped buffer
+        // keypoints below hcap straight into the host call's buffer
         describe_one(u8arena, tab, kp, grid, hist, pairs_of, red_lo, red_hi,
                          [&] { return (i < hcap ? hdesc : desc) + (size_t)i * kDescLen; });
         if (tid == 0) next[p ^ 1] = claim;

@@ -684,7 +684,7 @@ struct Engine {
     }
 
     // The descriptors of octave o. Host calls (cell): those below the cell's
-    // capacity go straight into the mapped export buffer while the stage runs,
+    // capacity go straight into the host buffer while the stage runs,
     // the rest to d_desc.
     int describe_octave(int o, const RunCell* rc, cudaStream_t q) {
         // two keypoints per CTA for 1/8 of the candidate capacity; the last
@@ -974,7 +974,7 @@ struct Engine {
     // One run on the image in d_img: replayed from the CUDA graph of this
     // size (captured on first use), or launched in order with stage events
     // when profiling.
-    // exp: end the run with the export into the mapped buffer (host calls).
+    // exp: end the run with the export into the host buffer hx (host calls).
     int run(bool with_desc, bool exp = false) {
         const long long stride = (long long)img_pitch;
         desc_on_host = 0;

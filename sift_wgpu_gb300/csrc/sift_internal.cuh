@@ -74,7 +74,7 @@ struct ImgRef {
 // later kernels read it.
 struct RunCell {
     ImgRef ref;
-    Counters* ctr;       // mapped result buffer: counters, keypoints, descriptors
+    Counters* ctr;       // host result buffer: counters, keypoints, descriptors
     Keypoint* kps;
     float* desc;
     uint32_t cap;        // keypoints that the buffer holds (0: no buffer)
